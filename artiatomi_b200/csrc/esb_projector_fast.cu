@@ -401,25 +401,10 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_slicer_fused(KConst c, con
 // direction, so the major axis of the layer walk and the signs of both steps
 // are the same for all rays of a launch: they become template parameters
 // (ZMAJ, SM, SN), and the host picks the instance from the beam direction.
-// The walk is layer_sum_xz's (same sample bookkeeping, cell sums and order)
-// with cheaper loads: it keeps the near row of the current layer (3 corner
-// values, interpolated in y) and loads the far row at 4 minor positions, so
-// that after a minor crossing the next layer's near row is the far row moved
-// by one. While the 4 positions and the far row lie inside the volume, the
-// far-row corners are read through one running pointer per y plane at fixed
-// offsets (compile-time offsets for the z-major walk), without clamping or
-// index arithmetic; at the volume's faces the walk takes clamped reads.
-
-template <int VT>
-__device__ __forceinline__ float ldv(const char* p) {
-  if (VT == ESB_VOXEL_F32) return __ldg((const float*)p);
-  if (VT == ESB_VOXEL_F16) return __half2float(__ldg((const __half*)p));
-  return __bfloat162float(__ldg((const __nv_bfloat16*)p));
-}
+// The samples and their split into cells are layer_sum_xz's.
 
 // A voxel as loaded (float, or the 16 bits of a half / bfloat16), converted
-// to float where it is used: the walk's prefetched far row stays in its
-// loaded form until the next layer blends it.
+// to float where it is used.
 template <int VT>
 struct RawVoxel {
   typedef unsigned short T;
@@ -433,6 +418,14 @@ __device__ __forceinline__ typename RawVoxel<VT>::T ldraw(const char* p) {
   if constexpr (VT == ESB_VOXEL_F32) return __ldg((const float*)p);
   else return __ldg((const unsigned short*)p);
 }
+// v = the voxel at p where `on`, else v stays (a predicated load, no branch).
+template <int VT>
+__device__ __forceinline__ void ldraw_if(typename RawVoxel<VT>::T& v, const char* p, bool on) {
+  if constexpr (VT == ESB_VOXEL_F32)
+    asm("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.f32 %0, [%1];}" : "+f"(v) : "l"(p), "r"((unsigned)on));
+  else
+    asm("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u16 %0, [%1];}" : "+h"(v) : "l"(p), "r"((unsigned)on));
+}
 template <int VT>
 __device__ __forceinline__ float cvt(typename RawVoxel<VT>::T r) {
   if constexpr (VT == ESB_VOXEL_F32) return r;
@@ -440,227 +433,303 @@ __device__ __forceinline__ float cvt(typename RawVoxel<VT>::T r) {
   else return __uint_as_float((unsigned)r << 16);
 }
 
+__device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
+
+// Steps of the walk, the same for every ray of a launch whose samples lie in
+// one binade of the ray parameter (axis_step on the host; a ray with another
+// step takes ray_sum).
+struct AxisStep {
+  float step;          // of the ray parameter
+  float dM, dN;        // |step| of the major and minor coordinate, dM >= dN
+  float isM, isN;      // 1 / dM, and 1 / dN (0 for dN = 0)
+  float hM, hN;        // dM / 2, dN / 2
+  float g;             // dN dM / 12
+};
+
 // Sum of the trilinear interpolant over samples j0 .. J-1 of one ray whose y
 // interpolation coordinate lies in cell iy with weight b, walked along major
-// axis z (ZMAJ) or x with step signs SM (major) and SN (minor). Mq, Nq,
-// dM, dN: mirrored major / minor coordinate of sample 0 and |steps|
-// (dM >= dN).
-template <int VT, bool ZMAJ, int SM, int SN>
-__device__ float axis_walk(const Cell<VT>& C, float Mq, float Nq, float dM, float dN, float b, int iy, int j0,
-                           int J) {
-  constexpr long ES = VT == ESB_VOXEL_F32 ? 4 : 2;
-  const long sM = ZMAJ ? C.sz : 1, sN = ZMAJ ? 1 : C.sz;  // element strides of the major and minor axes
+// axis z (ZMAJ) or x with step signs SM (major) and SN (minor). Mq, Nq:
+// mirrored major / minor coordinate of sample 0. Off: byte offsets into the
+// volume, 32-bit below 4 GiB.
+//
+// The sum is linear in the voxels, so the walk forms the weight of every
+// voxel instead of evaluating the interpolant: the samples of a layer lie in
+// at most two cells A = (n, m) and B = (n + 1, m); a cell's M samples with
+// mean local coordinates (a, c) give its corners the weights
+//   t = M (a c + q) to the far upper one, M a - t, M c - t and
+//   M - M a - (M c - t) to the others, q = dN dM (M^2 - 1) / 12.
+// A row of voxels gets the far weights of the layer before it and the near
+// weights of the layer after it: 4 weights at the minor positions n - 1 ..
+// n + 2 of the layer's cell n, the first only after a crossing, the last
+// only before one. They are applied to the rows of both y planes with
+// separate sums, which are interpolated in y once at the end.
+//
+// What bounds it: instruction issue and the FMA pipe, with the latency of
+// the rows' loads behind them. Additions and products of cells A and B are
+// packed pairs, one issue slot for both; fused multiply-adds are not (a
+// packed one with three different operands holds the pipe for 3.2 cycles,
+// two plain ones for 2.6), the ceilings of the two crossings are a packed
+// add that rounds up (no conversion-unit instruction), the outer positions
+// are read only by the lanes whose ray needs them, the next row's loads are
+// in flight during a layer's arithmetic, and layers whose rows and window
+// lie inside the volume and wholly inside the ray take no clamps, no index
+// arithmetic and no end test.
+template <int VT, bool ZMAJ, int SM, int SN, class Off>
+__device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C, float Mq, float Nq, float b, int iy,
+                                           int j0, int J) {
+  typedef typename RawVoxel<VT>::T Raw;
+  constexpr int ES = VT == ESB_VOXEL_F32 ? 4 : 2;
+  const Off sM = ES * (ZMAJ ? (Off)C.sz : (Off)1), sN = ES * (ZMAJ ? (Off)1 : (Off)C.sz);  // strides in bytes
   const int nM = ZMAJ ? C.nz : C.nx, nN = ZMAJ ? C.nx : C.nz;
   const char* const base = (const char*)C.vol;
   const float fj0 = (float)j0;
-  const float pM = __fmaf_rn(fj0, dM, Mq), pN = __fmaf_rn(fj0, dN, Nq);
-  float fcm = floorf(pM), fcn = floorf(pN);
-  const float inf = FLT_MAX;
-  const float isM = 1.0f / dM;
-  const float isN = dN > 0.f ? 1.0f / dN : inf;
-  float nMs = ((fcm + 1.f) - pM) * isM;
-  float nNs = dN > 0.f ? ((fcn + 1.f) - pN) * isN : inf;
-  const float g = dN * dM * (1.0f / 12.0f);
-  const float jb = fj0 - 0.5f;
+  const float pM = __fmaf_rn(fj0, A.dM, Mq), pN = __fmaf_rn(fj0, A.dN, Nq);
+  const float fm = floorf(pM), fn = floorf(pN);  // mirrored cell of the first sample
+  // sample parameters of the k-th major and the kn-th minor crossing
+  const float nM0 = ((fm + 1.f) - pM) * A.isM;
+  const float nN0 = A.isN > 0.f ? ((fn + 1.f) - pN) * A.isN : FLT_MAX;
   const float Mt = (float)(J - j0);
-  const float ib = 1.0f - b;
+  // a cell's mean local coordinate is s * step / 2 + rel, s the sum of its
+  // first and past-the-last sample numbers
+  const float jb = fj0 - 0.5f;
+  float2 relN;
+  relN.x = __fmaf_rn(jb, A.dN, __fsub_rn(Nq, fn));
+  relN.y = relN.x - 1.f;
+  float relM = __fmaf_rn(jb, A.dM, __fsub_rn(Mq, fm));
   const int ny = C.ny;
-  const long y0 = (long)(iy < 0 ? 0 : (iy > ny - 1 ? ny - 1 : iy)) * C.sy;
-  const long y1 = (long)(iy + 1 < 0 ? 0 : (iy + 1 > ny - 1 ? ny - 1 : iy + 1)) * C.sy;
-  // original indices: far major row of the current layer, first minor position of the window
-  int im = SM * ((int)fcm + 1), in0 = SN * (int)fcn;
-  const char* P = base + ES * (y0 + (long)im * sM + (long)in0 * sN);  // far row, plane iy
-  const long dy = ES * (y1 - y0);
-  const long strideN = SN * ES * sN, strideM = SM * ES * sM;
-  auto ld = [&](int mi, int ni) -> float {  // clamped, interpolated in y
+  const Off yA = (Off)(ES * C.sy) * (Off)(iy < 0 ? 0 : (iy > ny - 1 ? ny - 1 : iy));
+  const Off dy = (Off)(ES * C.sy) * (Off)(iy + 1 < 0 ? 0 : (iy + 1 > ny - 1 ? ny - 1 : iy + 1)) - yA;
+  // near row of the current layer and its cell
+  int im = SM * (int)fm, in0 = SN * (int)fn;
+  const int lowN = SN > 0 ? 1 : 2, highN = SN > 0 ? nN - 3 : nN - 2;  // in0 with its window inside
+  float k = 0.f, kn = 0.f, fm0 = 0.f;
+  float g0 = 0.f, g1 = 0.f, g2 = 0.f;  // far weights of the layer before, at n - 1, n, n + 1
+  float S0 = 0.f, T0 = 0.f, S1 = 0.f, T1 = 0.f;  // sums over planes iy and iy + 1
+  // layers below kEnd end before the ray's last sample, on rows of the volume
+  const float kEnd = fminf(floorf((Mt - nM0) * A.dM), SM > 0 ? (float)(nM - 1) - fm : -fm);
+  // one layer: row values v* (plane iy) and w* (plane iy + 1) at n - 1 .. n + 2
+  auto layer = [&](bool X, float tA, float tL, Raw va, Raw vb, Raw vc, Raw vd, Raw wa, Raw wb, Raw wc, Raw wd) {
+    const float2 f = __fadd2_rn(__fadd2_ru(make_float2(tA, tL), splat(8388608.0f)), splat(-8388608.0f));  // ceil
+    // samples [fm0, f.x) lie in cell A, [f.x, f.y) in cell B
+    const float2 M = make_float2(f.x - fm0, f.y - f.x), mM = make_float2(fm0 - f.x, f.x - f.y);
+    const float sA = fm0 + f.x, sB = f.x + f.y;
+    const float2 a = make_float2(fmaf(sA, A.hN, relN.x), fmaf(sB, A.hN, relN.y));
+    const float2 c = make_float2(fmaf(sA, A.hM, relM), fmaf(sB, A.hM, relM));
+    const float2 MM = __fmul2_rn(M, M), Ma = __fmul2_rn(M, a), Mc = __fmul2_rn(M, c);
+    const float2 acq = make_float2(fmaf(a.x, c.x, fmaf(MM.x, A.g, -A.g)), fmaf(a.y, c.y, fmaf(MM.y, A.g, -A.g)));
+    const float2 mt = __fmul2_rn(mM, acq);  // - t
+    const float2 w10 = __fadd2_rn(Ma, mt), wf = __fadd2_rn(Mc, mt);
+    const float2 m00 = __fadd2_rn(__fadd2_rn(Ma, wf), mM);  // minus the near lower weights
+    const float i0 = g1 - m00.x, i1 = g2 + (w10.x - m00.y);
+    S0 = fmaf(cvt<VT>(vb), i0, S0);
+    S1 = fmaf(cvt<VT>(wb), i0, S1);
+    T0 = fmaf(cvt<VT>(vc), i1, T0);
+    T1 = fmaf(cvt<VT>(wc), i1, T1);
+    S0 = fmaf(cvt<VT>(va), g0, S0);
+    S1 = fmaf(cvt<VT>(wa), g0, S1);
+    T0 = fmaf(cvt<VT>(vd), w10.y, T0);
+    T1 = fmaf(cvt<VT>(wd), w10.y, T1);
+    const float F1 = wf.y - mt.x;
+    g0 = X ? wf.x : 0.f;
+    g1 = X ? F1 : wf.x;
+    g2 = X ? -mt.y : F1;
+    fm0 = f.y;
+    if (X) relN = __fadd2_rn(relN, splat(-1.f));
+    relM -= 1.f;
+  };
+  auto clamped = [&](int mi, int n) -> const char* {
     mi = mi < 0 ? 0 : (mi > nM - 1 ? nM - 1 : mi);
-    ni = ni < 0 ? 0 : (ni > nN - 1 ? nN - 1 : ni);
-    const char* p = base + ES * ((long)mi * sM + (long)ni * sN + y0);
-    return fmaf(b, ldv<VT>(p + dy), ib * ldv<VT>(p));
+    n = n < 0 ? 0 : (n > nN - 1 ? nN - 1 : n);
+    return base + (Off)((Off)mi * sM + (Off)n * sN + yA);
   };
-  // raw far-row values (plane iy, plane iy + 1 at minor positions 0..3)
-  // of the layer whose far row is at major index mi and window start ni
-  const bool canN = nN >= 4;
-  typename RawVoxel<VT>::T r0, r1, r2, r3, r4, r5, r6, r7;
-  auto fetch = [&](int mi, int ni, const char* q) {
-    const int lo = SN > 0 ? ni : ni - 3;
-    if (canN && (unsigned)lo <= (unsigned)(nN - 4) && (unsigned)mi < (unsigned)nM) {
-      r0 = ldraw<VT>(q);
-      r1 = ldraw<VT>(q + dy);
-      r2 = ldraw<VT>(q + strideN);
-      r3 = ldraw<VT>(q + strideN + dy);
-      r4 = ldraw<VT>(q + 2 * strideN);
-      r5 = ldraw<VT>(q + 2 * strideN + dy);
-      r6 = ldraw<VT>(q + 3 * strideN);
-      r7 = ldraw<VT>(q + 3 * strideN + dy);
-    } else {
-      mi = mi < 0 ? 0 : (mi > nM - 1 ? nM - 1 : mi);
-      const char* row = base + ES * ((long)mi * sM + y0);
-      auto at = [&](int n) {
-        n = n < 0 ? 0 : (n > nN - 1 ? nN - 1 : n);
-        return row + ES * ((long)n * sN);
-      };
-      const char* q0 = at(ni);
-      const char* q1 = at(ni + SN);
-      const char* q2 = at(ni + 2 * SN);
-      const char* q3 = at(ni + 3 * SN);
-      r0 = ldraw<VT>(q0);
-      r1 = ldraw<VT>(q0 + dy);
-      r2 = ldraw<VT>(q1);
-      r3 = ldraw<VT>(q1 + dy);
-      r4 = ldraw<VT>(q2);
-      r5 = ldraw<VT>(q2 + dy);
-      r6 = ldraw<VT>(q3);
-      r7 = ldraw<VT>(q3 + dy);
-    }
+  const long step1 = SN > 0 ? (long)sN : -(long)sN;
+  Raw va = Raw(0), vb, vc, vd = Raw(0), wa = Raw(0), wb, wc, wd = Raw(0);
+  float nMs = 0.f, nNs = 0.f;
+  bool X = false;
+  // row im with its window, clamped
+  auto fetch = [&]() {
+    const char* p = clamped(im, in0 - SN);
+    va = ldraw<VT>(p), wa = ldraw<VT>(p + dy);
+    p = clamped(im, in0);
+    vb = ldraw<VT>(p), wb = ldraw<VT>(p + dy);
+    p = clamped(im, in0 + SN);
+    vc = ldraw<VT>(p), wc = ldraw<VT>(p + dy);
+    p = clamped(im, in0 + 2 * SN);
+    vd = ldraw<VT>(p), wd = ldraw<VT>(p + dy);
+    nMs = __fmaf_rn(k, A.isM, nM0);
+    nNs = __fmaf_rn(kn, A.isN, nN0);
+    X = nNs <= nMs;
   };
-  // near row of the first layer, and its far row
-  float N0 = ld(im - SM, in0), N1 = ld(im - SM, in0 + SN), N2 = ld(im - SM, in0 + 2 * SN);
-  fetch(im, in0, P);
-  float F0 = fmaf(b, cvt<VT>(r1), ib * cvt<VT>(r0)), F1 = fmaf(b, cvt<VT>(r3), ib * cvt<VT>(r2)), F2 = fmaf(b, cvt<VT>(r5), ib * cvt<VT>(r4)), F3 = fmaf(b, cvt<VT>(r7), ib * cvt<VT>(r6));
-  float fm0 = 0.0f, acc = 0.0f;
-#pragma unroll 1
-  for (int guard = 0; guard < 1 << 20; ++guard) {
-    // samples [fm0, fmA) lie in cell (n, m), [fmA, fmL) in cell (n + 1, m)
-    const float fmL = fminf(ceilf(nMs), Mt);
-    const bool X = nNs <= nMs;
-    const float fmA = fmaxf(fminf(ceilf(fminf(nNs, nMs)), Mt), fm0);
-    // the next layer's far row, one minor position further when this layer
-    // crosses: its loads are in flight during this layer's sums
-    const char* Pn = P + strideM + (X ? strideN : 0);
-    const int imn = im + SM, in0n = in0 + (X ? SN : 0);
-    fetch(imn, in0n, Pn);
-    {  // cell (n, m): near corners N0, N1, far corners F0, F1
-      const float M = fmA - fm0;
-      const float jm = __fmaf_rn(0.5f, fm0 + fmA, jb);
-      const float a = __fmaf_rn(jm, dN, Nq) - fcn, c = __fmaf_rn(jm, dM, Mq) - fcm;
-      const float k1 = N1 - N0, k3 = F0 - N0, k5 = (F1 - F0) - k1;
-      const float f = fmaf(c, fmaf(a, k5, k3), fmaf(a, k1, N0));
-      acc = fmaf(M, fmaf(k5, fmaf(M * M, g, -g), f), acc);
-    }
-    {  // cell (n + 1, m): near corners N1, N2, far corners F1, F2
-      const float M = fmL - fmA;
-      const float jm = __fmaf_rn(0.5f, fmA + fmL, jb);
-      const float a = __fmaf_rn(jm, dN, Nq) - (fcn + 1.f), c = __fmaf_rn(jm, dM, Mq) - fcm;
-      const float k1 = N2 - N1, k3 = F1 - N1, k5 = (F2 - F1) - k1;
-      const float f = fmaf(c, fmaf(a, k5, k3), fmaf(a, k1, N1));
-      acc = fmaf(M, fmaf(k5, fmaf(M * M, g, -g), f), acc);
-    }
-    fm0 = fmL;
-    if (fm0 >= Mt) break;
-    // next layer
-    N0 = X ? F1 : F0;
-    N1 = X ? F2 : F1;
-    N2 = X ? F3 : F2;
-    F0 = fmaf(b, cvt<VT>(r1), ib * cvt<VT>(r0));
-    F1 = fmaf(b, cvt<VT>(r3), ib * cvt<VT>(r2));
-    F2 = fmaf(b, cvt<VT>(r5), ib * cvt<VT>(r4));
-    F3 = fmaf(b, cvt<VT>(r7), ib * cvt<VT>(r6));
+  // the layer of the row at hand, which may be the ray's last
+  auto edge_layer = [&]() {
+    const float tL = fminf(nMs, Mt);
+    layer(X, fminf(nNs, tL), tL, va, vb, vc, vd, wa, wb, wc, wd);
+    im += SM;
+    k += 1.f;
     if (X) {
-      fcn += 1.f;
-      nNs = ((fcn + 1.f) - pN) * isN;
+      in0 += SN;
+      kn += 1.f;
     }
-    fcm += 1.f;
-    nMs = ((fcm + 1.f) - pM) * isM;
-    im = imn;
-    in0 = in0n;
-    P = Pn;
+  };
+  // Edge layers until every ray of the warp is inside the volume or done:
+  // the rays enter the loop over inner layers together.
+  const unsigned mask = __activemask();
+  fetch();
+  for (int guard = 0; guard < 1 << 20; ++guard) {
+    const bool in = k < kEnd && (unsigned)im < (unsigned)nM && in0 >= lowN && in0 < highN;
+    if (__all_sync(mask, in || fm0 >= Mt)) break;
+    if (fm0 < Mt) {
+      edge_layer();
+      fetch();
+    }
   }
-  return acc;
+  // minor crossings until the window may leave the volume
+  const float knEnd = kn + (float)(SN > 0 ? highN - in0 : in0 - lowN);
+  if (fm0 < Mt && k < kEnd && kn < knEnd) {
+    const float k0 = k, kn0 = kn;
+    Off off = (Off)im * sM + (Off)in0 * sN + yA;
+#pragma unroll 2
+    do {
+      k += 1.f;
+      off += SM > 0 ? sM : (Off)0 - sM;
+      if (X) {
+        kn += 1.f;
+        off += SN > 0 ? sN : (Off)0 - sN;
+      }
+      const float nM1 = __fmaf_rn(k, A.isM, nM0), nN1 = __fmaf_rn(kn, A.isN, nN0);
+      const bool X1 = nN1 <= nM1;
+      // the next row, in flight during this layer's arithmetic
+      const char *u = base + off, *r = base + (Off)(off + dy);
+      Raw na = va, nd = vd, oa = wa, od = wd;
+      const Raw nb = ldraw<VT>(u), ob = ldraw<VT>(r), nc = ldraw<VT>(u + step1), oc = ldraw<VT>(r + step1);
+      ldraw_if<VT>(na, u - step1, X);
+      ldraw_if<VT>(oa, r - step1, X);
+      ldraw_if<VT>(nd, u + 2 * step1, X1);
+      ldraw_if<VT>(od, r + 2 * step1, X1);
+      layer(X, fminf(nNs, nMs), nMs, va, vb, vc, vd, wa, wb, wc, wd);
+      va = na, vb = nb, vc = nc, vd = nd, wa = oa, wb = ob, wc = oc, wd = od;
+      nMs = nM1;
+      nNs = nN1;
+      X = X1;
+    } while (k < kEnd && kn < knEnd);
+    im += SM * (int)(k - k0);
+    in0 += SN * (int)(kn - kn0);
+  }
+#pragma unroll 1
+  for (int guard = 0; guard < 1 << 20 && fm0 < Mt; ++guard) {
+    edge_layer();
+    fetch();
+  }
+  {  // the far row of the last layer
+    const char *p0 = clamped(im, in0 - SN), *p1 = clamped(im, in0), *p2 = clamped(im, in0 + SN);
+    S0 = fmaf(cvt<VT>(ldraw<VT>(p1)), g1, S0);
+    S1 = fmaf(cvt<VT>(ldraw<VT>(p1 + dy)), g1, S1);
+    T0 = fmaf(cvt<VT>(ldraw<VT>(p2)), g2, T0);
+    T1 = fmaf(cvt<VT>(ldraw<VT>(p2 + dy)), g2, T1);
+    S0 = fmaf(cvt<VT>(ldraw<VT>(p0)), g0, S0);
+    S1 = fmaf(cvt<VT>(ldraw<VT>(p0 + dy)), g0, S1);
+  }
+  return fmaf(b, S1 + T1, (1.0f - b) * (S0 + T0));
+}
+
+// ray_sum for the few rays that do not fit an axis kernel's instance; a call
+// of its own, so that its registers do not weigh on the walk.
+template <int VT>
+__device__ __noinline__ float other_ray_sum(const KConst* c, const void* vol, float3 s, float t0, float tout,
+                                            bool first_at_source) {
+  const Cell<VT> C{vol, (int)c->dim.x, (int)c->dim.y, (int)c->dim.z, (long)c->dim.x, (long)c->dim.x * (long)c->dim.y};
+  return ray_sum<VT, unsigned long long>(*c, C, s, t0, tout, first_at_source);
 }
 
 // Sum over the samples of one sub-ray from t0 to tout (ray_sum) with the
 // axis walk when the ray fits the launch's instance (its y in one cell, its
-// major axis and step signs the instance's), else ray_sum's walkers.
-template <int VT, bool ZMAJ, int SM, int SN>
-__device__ float axis_ray_sum(const KConst& c, const Cell<VT>& C, float3 s, float t0, float tout,
-                              bool first_at_source) {
+// step the launch's), else other_ray_sum. With first_at_source the first
+// sample is the one at the ray's start, whose value is `source`.
+template <int VT, bool ZMAJ, int SM, int SN, class Off>
+__device__ __forceinline__ float axis_ray_sum(const KConst& c, const AxisStep& A, const Cell<VT>& C, float3 s,
+                                              float t0, float tout, bool first_at_source, float source) {
   if (!(t0 <= tout)) return 0.0f;
   const float h = c.vs.x * 0.15f;
   float step;
   bool ok;
   const int J = progression(t0, tout, h, step, ok);
-  if (!ok) return ray_sum<VT, unsigned long long>(c, C, s, t0, tout, first_at_source);
   const float3 q0 = interp_coord(c, ray_point(c, s, t0));
-  const float3 dq = interp_step(c, step);
-  float sum = 0.0f;
-  int j0 = 0;
-  if (first_at_source) {
-    const float3 q = interp_coord(c, s);
-    sum = trilinear<VT>(C, q.x, q.y, q.z);
-    j0 = 1;
-  }
-  const float ylast = qpos(q0.y, J - 1, dq.y);
-  if (!(fabsf(dq.y) * (float)J < 1e-5f && floorf(q0.y) == floorf(ylast)))
-    return sum + cell_sum<VT>(C, q0.x, q0.y, q0.z, dq.x, dq.y, dq.z, j0, J);
+  const float dqy = __fmul_rn(__fmul_rn(__fmul_rn(step, c.n.y), c.bbRcp.y), c.dim.y);
+  const float ylast = qpos(q0.y, J - 1, dqy);
   const float fy = floorf(q0.y);
-  const float qm = ZMAJ ? q0.z : q0.x, dqm = ZMAJ ? dq.z : dq.x;
-  const float qn = ZMAJ ? q0.x : q0.z, dqn = ZMAJ ? dq.x : dq.z;
-  if ((fabsf(dq.z) >= fabsf(dq.x)) != ZMAJ || (dqm < 0.f ? -1 : 1) != SM || (dqn < 0.f ? -1 : 1) != SN)
-    return sum + cell_sum_xz<VT, unsigned long long>(C, q0.x, q0.y - fy, (int)fy, q0.z, dq.x, dq.z, j0, J);
+  if (!(ok && step == A.step && fabsf(dqy) * (float)J < 1e-5f && fy == floorf(ylast)))
+    return other_ray_sum<VT>(&c, C.vol, s, t0, tout, first_at_source);
+  const float sum = first_at_source ? source : 0.0f;
+  const int j0 = first_at_source ? 1 : 0;
   if (j0 >= J) return sum;
-  return sum + axis_walk<VT, ZMAJ, SM, SN>(C, SM > 0 ? qm : -qm, SN > 0 ? qn : -qn, fabsf(dqm), fabsf(dqn),
-                                           q0.y - fy, (int)fy, j0, J);
+  const float qm = ZMAJ ? q0.z : q0.x, qn = ZMAJ ? q0.x : q0.z;
+  return sum + axis_walk<VT, ZMAJ, SM, SN, Off>(A, C, SM > 0 ? qm : -qm, SN > 0 ? qn : -qn, q0.y - fy, (int)fy, j0, J);
 }
 
-// k_project_fast (march) for single-axis series; layout of k_project_fast.
-template <int VT, bool ZMAJ, int SM, int SN>
-__global__ void __launch_bounds__(256) k_project_axis(KConst c, const void* __restrict__ vol, float* __restrict__ proj,
-                                                      float* __restrict__ dist, size_t pitchE, int x0, int y0, int x1,
-                                                      int y1) {
-  const int lane = threadIdx.x & 31;
-  const int sub = lane & 3;
-  const int row = lane >> 2;
-  const int nw = blockDim.x >> 5;
-  const int x = x0 + (int)blockIdx.x * nw + (int)(threadIdx.x >> 5);
-  const int y = y0 + (int)blockIdx.y * 8 + row;
-  const bool active = x < x1 && y < y1;
+// Pixel of a thread in the axis kernels: the 4 sub-rays of a pixel in
+// adjacent lanes, a warp spans 8 pixels along the detector axis that crosses
+// the tilt axis (v, or u when `swap`), so that its rays lie in few y planes;
+// the warps of a block step along the other axis.
+struct AxisPixel {
+  int sub, x, y;
+  bool active;
+  __device__ __forceinline__ AxisPixel(int swap, int x0, int y0, int x1, int y1) {
+    const int lane = threadIdx.x & 31;
+    sub = lane & 3;
+    const int along = (int)blockIdx.y * 8 + (lane >> 2);
+    const int across = (int)blockIdx.x * (blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    x = x0 + (swap ? along : across);
+    y = y0 + (swap ? across : along);
+    active = x < x1 && y < y1;
+  }
+};
+
+// k_project_fast (march) for single-axis series.
+template <int VT, bool ZMAJ, int SM, int SN, class Off>
+__global__ void __launch_bounds__(256, 4) k_project_axis(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
+                                                      const void* __restrict__ vol, float* __restrict__ proj,
+                                                      float* __restrict__ dist, size_t pitchE, int swap, int x0,
+                                                      int y0, int x1, int y1) {
+  const AxisPixel P(swap, x0, y0, x1, y1);
   Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
   float sum = 0.0f, gx = 0.0f, gz = 0.0f;
-  if (active) {
-    const float osx = (sub & 2) ? 0.75f : 0.25f, osy = (sub & 1) ? 0.75f : 0.25f;
-    const float3 s = ray_src(c, (float)x + osx, (float)y + osy);
+  if (P.active) {
+    const float osx = (P.sub & 2) ? 0.75f : 0.25f, osy = (P.sub & 1) ? 0.75f : 0.25f;
+    const float3 s = ray_src(c, (float)P.x + osx, (float)P.y + osy);
     float tin, tout;
     hit(s, c.n, c.bbMin, c.bbMax, tin, tout);
     if (tout - tin > 0.0f) {
       gx = 1.0f;
       gz = tout - tin;
-      sum = axis_ray_sum<VT, ZMAJ, SM, SN>(c, C, s, tin, tout, false);
+      sum = axis_ray_sum<VT, ZMAJ, SM, SN, Off>(c, A, C, s, tin, tout, false, 0.0f);
     }
   }
   sum = quad_sum_ordered(sum);
   gx = quad_sum_ordered(gx);
   gz = quad_sum_ordered(gz);
-  if (active && sub == 0) {
-    const size_t i = (size_t)y * pitchE + x;
+  if (P.active && P.sub == 0) {
+    const size_t i = (size_t)P.y * pitchE + P.x;
     proj[i] += sum * c.vs.x * 0.15f * 0.25f;
     dist[i] = fmaxf(0.0f, gz / gx);
   }
 }
 
-// k_slicer_fused for single-axis series; layout of k_slicer_fused.
-// (16-bit volumes: at most 80 registers, 3 blocks of 256 threads per SM;
-// uncapped, those instances take about 100 and fit 2. FP32 instances take
-// 76-79 uncapped, and a cap changes their allocation for the worse.)
-template <int VT, bool ZMAJ, int SM, int SN>
-__global__ void __launch_bounds__(256, VT == ESB_VOXEL_F32 ? 0 : 3) k_slicer_axis(KConst c, const void* __restrict__ vol, float* __restrict__ imgs,
-                                                     size_t img_stride, size_t pitchE, SlabTable slabs, int x0, int y0,
-                                                     int x1, int y1) {
-  const int lane = threadIdx.x & 31;
-  const int sub = lane & 3;
-  const int row = lane >> 2;
-  const int nw = blockDim.x >> 5;
-  const int x = x0 + (int)blockIdx.x * nw + (int)(threadIdx.x >> 5);
-  const int y = y0 + (int)blockIdx.y * 8 + row;
-  const bool active = x < x1 && y < y1;
+// k_slicer_fused for single-axis series; pixels as k_project_axis. The
+// sample at the ray's start, the first of every slab, is formed once.
+template <int VT, bool ZMAJ, int SM, int SN, class Off>
+__global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
+                                                     const void* __restrict__ vol, float* __restrict__ imgs,
+                                                     size_t img_stride, size_t pitchE, SlabTable slabs, int swap,
+                                                     int x0, int y0, int x1, int y1) {
+  const AxisPixel P(swap, x0, y0, x1, y1);
   Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
   float3 s = make_float3(0.f, 0.f, 0.f);
-  float tin = 0.f, tout = -1.f;
+  float tin = 0.f, tout = -1.f, source = 0.f;
   int klo = ESB_MAX_SLABS, khi = -1;
   bool hitray = false;
-  if (active) {
-    const float osx = (sub & 2) ? 0.75f : 0.25f, osy = (sub & 1) ? 0.75f : 0.25f;
-    s = ray_src(c, (float)x + osx, (float)y + osy);
+  if (P.active) {
+    const float osx = (P.sub & 2) ? 0.75f : 0.25f, osy = (P.sub & 1) ? 0.75f : 0.25f;
+    s = ray_src(c, (float)P.x + osx, (float)P.y + osy);
     hit(s, c.n, c.bbMin, c.bbMax, tin, tout);
     hitray = tout - tin > 0.0f;
     if (hitray) {
@@ -671,6 +740,8 @@ __global__ void __launch_bounds__(256, VT == ESB_VOXEL_F32 ? 0 : 3) k_slicer_axi
           khi = max(khi, k);
         }
       }
+      const float3 q = interp_coord(c, s);
+      source = trilinear<VT>(C, q.x, q.y, q.z);
     }
   }
   for (int o = 1; o <= 2; o <<= 1) {
@@ -683,27 +754,66 @@ __global__ void __launch_bounds__(256, VT == ESB_VOXEL_F32 ? 0 : 3) k_slicer_axi
     wlo = min(wlo, __shfl_xor_sync(0xffffffffu, wlo, o));
     whi = max(whi, __shfl_xor_sync(0xffffffffu, whi, o));
   }
-  const size_t pix = (size_t)y * pitchE + x;
+  const size_t pix = (size_t)P.y * pitchE + P.x;
   for (int k = wlo; k <= whi; ++k) {
     float v = 0.0f;
     if (hitray && k >= klo && k <= khi)
-      v = axis_ray_sum<VT, ZMAJ, SM, SN>(c, C, s, fmaxf(tin, slabs.bound[k]), fminf(tout, slabs.bound[k + 1]), true);
+      v = axis_ray_sum<VT, ZMAJ, SM, SN, Off>(c, A, C, s, fmaxf(tin, slabs.bound[k]), fminf(tout, slabs.bound[k + 1]),
+                                              true, source);
     v = quad_sum_ordered(v);
-    if (active && sub == 0 && k >= klo && k <= khi) imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
+    if (P.active && P.sub == 0 && k >= klo && k <= khi)
+      imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
   }
 }
 
 // Beam directions whose rays all stay in one y plane take the axis kernels.
 bool axis_projection(const KConst& c) { return fabsf(c.n.y) <= 1e-6f; }
 
-// Instance of the axis kernels for the launch's beam direction: major axis z
-// when |dq.z| >= |dq.x| (as each ray decides it), step signs.
-void axis_orientation(const KConst& c, bool& zmaj, int& sm, int& sn) {
-  const float qx = c.n.x * c.bbRcp.x * c.dim.x, qz = c.n.z * c.bbRcp.z * c.dim.z;
+// Instance of the axis kernels for the launch's beam direction (major axis z
+// when |dq.z| >= |dq.x|, step signs) and its steps: the step of the ray
+// parameter is the one of the binade that holds the volume's centre.
+AxisStep axis_step(const KConst& c, bool& zmaj, int& sm, int& sn) {
+  const float h = c.vs.x * 0.15f;
+  double t = 0.0;
+  const double n[3] = {c.n.x, c.n.y, c.n.z}, d[3] = {c.det.x, c.det.y, c.det.z};
+  const double lo[3] = {c.bbMin.x, c.bbMin.y, c.bbMin.z}, hi[3] = {c.bbMax.x, c.bbMax.y, c.bbMax.z};
+  for (int j = 0; j < 3; ++j) t += n[j] * (0.5 * (lo[j] + hi[j]) - d[j]);
+  int e = 0;
+  frexp(t, &e);
+  volatile float t0 = (float)ldexp(0.5, e), t1 = t0 + h;  // single roundings, as the kernel's
+  AxisStep A;
+  A.step = t > 0.0 ? t1 - t0 : 0.0f;  // 0: no ray takes the walk
+  volatile float qx = A.step * c.n.x, qz = A.step * c.n.z;
+  qx = qx * c.bbRcp.x;
+  qz = qz * c.bbRcp.z;
+  qx = qx * c.dim.x;
+  qz = qz * c.dim.z;
   zmaj = fabsf(qz) >= fabsf(qx);
-  const float m = zmaj ? qz : qx, n = zmaj ? qx : qz;
+  const float m = zmaj ? qz : qx, nn = zmaj ? qx : qz;
   sm = m < 0.f ? -1 : 1;
-  sn = n < 0.f ? -1 : 1;
+  sn = nn < 0.f ? -1 : 1;
+  A.dM = fabsf(m);
+  A.dN = fabsf(nn);
+  if (!(A.dM > 0.f)) A.step = 0.0f;
+  A.isM = 1.0f / A.dM;
+  A.isN = A.dN > 0.f ? 1.0f / A.dN : 0.f;
+  A.hM = 0.5f * A.dM;
+  A.hN = 0.5f * A.dN;
+  A.g = A.dN * A.dM * (1.0f / 12.0f);
+  return A;
+}
+
+// Whether the warps of the axis kernels span detector columns (u) instead of
+// rows: when a pixel step along u moves the ray less across the volume's y
+// planes than one along v.
+int axis_swap(const KConst& c) {
+  const float uy = c.aniso[0] * c.u.y + c.aniso[3] * c.v.y, vy = c.aniso[1] * c.u.y + c.aniso[4] * c.v.y;
+  return fabsf(uy) < fabsf(vy) ? 1 : 0;
+}
+
+dim3 axis_grid(int swap, int nw, int w, int h) {
+  const int along = swap ? w : h, across = swap ? h : w;
+  return dim3((across + nw - 1) / nw, (along + 7) / 8);
 }
 
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.
@@ -714,22 +824,37 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
 // nw: warps per block (2, 4 or 8; 64-bit-offset volumes always take 4).
 
 // One launch of an axis kernel instance per beam orientation.
-#define ESB_AXIS_ORIENT(KER, VT, GRD, BLK, ST, ...)                              \
+#define ESB_AXIS_ORIENT(KER, VT, OFF, GRD, BLK, ST, ...)                         \
   do {                                                                          \
     bool zmaj_;                                                                 \
     int sm_, sn_;                                                               \
-    axis_orientation(c, zmaj_, sm_, sn_);                                       \
+    const AxisStep A_ = axis_step(c, zmaj_, sm_, sn_);                           \
     const int o_ = (zmaj_ ? 4 : 0) + (sm_ > 0 ? 2 : 0) + (sn_ > 0 ? 1 : 0);     \
     switch (o_) {                                                               \
-      case 0: KER<VT, false, -1, -1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;  \
-      case 1: KER<VT, false, -1, 1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;   \
-      case 2: KER<VT, false, 1, -1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;   \
-      case 3: KER<VT, false, 1, 1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;    \
-      case 4: KER<VT, true, -1, -1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;   \
-      case 5: KER<VT, true, -1, 1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;    \
-      case 6: KER<VT, true, 1, -1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;    \
-      default: KER<VT, true, 1, 1><<<GRD, BLK, 0, ST>>>(__VA_ARGS__); break;    \
+      case 0: KER<VT, false, -1, -1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;  \
+      case 1: KER<VT, false, -1, 1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;   \
+      case 2: KER<VT, false, 1, -1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;   \
+      case 3: KER<VT, false, 1, 1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;    \
+      case 4: KER<VT, true, -1, -1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;   \
+      case 5: KER<VT, true, -1, 1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;    \
+      case 6: KER<VT, true, 1, -1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;    \
+      default: KER<VT, true, 1, 1, OFF><<<GRD, BLK, 0, ST>>>(c, A_, __VA_ARGS__); break;    \
     }                                                                           \
+  } while (0)
+
+// Volumes below 4 GiB take 32-bit byte offsets in the axis walk.
+#define ESB_AXIS_LAUNCH(KER, GRD, BLK, ST, ...)                                                                \
+  do {                                                                                                        \
+    const double bytes_ = (double)c.dim.x * c.dim.y * c.dim.z * (vt == ESB_VOXEL_F32 ? 4.0 : 2.0);            \
+    if (bytes_ < 4294967296.0) {                                                                              \
+      if (vt == ESB_VOXEL_F32) ESB_AXIS_ORIENT(KER, ESB_VOXEL_F32, unsigned, GRD, BLK, ST, __VA_ARGS__);      \
+      else if (vt == ESB_VOXEL_F16) ESB_AXIS_ORIENT(KER, ESB_VOXEL_F16, unsigned, GRD, BLK, ST, __VA_ARGS__); \
+      else ESB_AXIS_ORIENT(KER, ESB_VOXEL_BF16, unsigned, GRD, BLK, ST, __VA_ARGS__);                         \
+    } else {                                                                                                  \
+      if (vt == ESB_VOXEL_F32) ESB_AXIS_ORIENT(KER, ESB_VOXEL_F32, size_t, GRD, BLK, ST, __VA_ARGS__);        \
+      else if (vt == ESB_VOXEL_F16) ESB_AXIS_ORIENT(KER, ESB_VOXEL_F16, size_t, GRD, BLK, ST, __VA_ARGS__);   \
+      else ESB_AXIS_ORIENT(KER, ESB_VOXEL_BF16, size_t, GRD, BLK, ST, __VA_ARGS__);                           \
+    }                                                                                                         \
   } while (0)
 
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
@@ -738,13 +863,9 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
   if (x1 <= x0 || y1 <= y0 || slabs.count <= 0) return cudaSuccess;
   if (axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
-    dim3 blk(32 * nw), grd((x1 - x0 + nw - 1) / nw, (y1 - y0 + 7) / 8);
-    if (vt == ESB_VOXEL_F32)
-      ESB_AXIS_ORIENT(k_slicer_axis, ESB_VOXEL_F32, grd, blk, st, c, vol, imgs, img_stride, pitchE, slabs, x0, y0, x1, y1);
-    else if (vt == ESB_VOXEL_F16)
-      ESB_AXIS_ORIENT(k_slicer_axis, ESB_VOXEL_F16, grd, blk, st, c, vol, imgs, img_stride, pitchE, slabs, x0, y0, x1, y1);
-    else
-      ESB_AXIS_ORIENT(k_slicer_axis, ESB_VOXEL_BF16, grd, blk, st, c, vol, imgs, img_stride, pitchE, slabs, x0, y0, x1, y1);
+    const int swap = axis_swap(c);
+    const dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
+    ESB_AXIS_LAUNCH(k_slicer_axis, grd, blk, st, vol, imgs, img_stride, pitchE, slabs, swap, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();
   }
@@ -775,13 +896,9 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
   if (mode == 0 && axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
-    dim3 blk(32 * nw), grd((x1 - x0 + nw - 1) / nw, (y1 - y0 + 7) / 8);
-    if (vt == ESB_VOXEL_F32)
-      ESB_AXIS_ORIENT(k_project_axis, ESB_VOXEL_F32, grd, blk, st, c, vol, proj, dist, pitchE, x0, y0, x1, y1);
-    else if (vt == ESB_VOXEL_F16)
-      ESB_AXIS_ORIENT(k_project_axis, ESB_VOXEL_F16, grd, blk, st, c, vol, proj, dist, pitchE, x0, y0, x1, y1);
-    else
-      ESB_AXIS_ORIENT(k_project_axis, ESB_VOXEL_BF16, grd, blk, st, c, vol, proj, dist, pitchE, x0, y0, x1, y1);
+    const int swap = axis_swap(c);
+    const dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
+    ESB_AXIS_LAUNCH(k_project_axis, grd, blk, st, vol, proj, dist, pitchE, swap, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();
   }

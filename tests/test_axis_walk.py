@@ -1,0 +1,97 @@
+"""The single-axis forward projector (k_project_axis, k_slicer_axis) where its
+layer walk has to go right: volumes thinner than the walk's window, one layer
+thick, odd sizes, beams on both sides of 45 degrees (major axis z or x, both
+step signs), in-plane rotations at which a warp spans detector rows or
+columns, FP32 and 16-bit voxels, and the walk's slabs.
+
+Against the FP64 oracle. The kernel places a ray's samples from its float
+start point, ~1e-3 voxel from the oracle's; the volume's gradient is below
+0.5 per voxel at an rms of 0.7, so a sum of samples agrees to 1e-3 * 0.5 /
+0.7 < 1e-3 of its rms, and to less where the errors of the rays differ:
+rel-L2 <= 5e-4. A ray whose length is a whole number of steps to that
+accuracy takes one sample more or less, in any 32-bit march (the oracle's
+differs from its FP64 one by up to 3.6e-3 here), so a pixel is held to
+the nearer of the oracle's two marches.
+"""
+import numpy as np
+import pytest
+
+from tests.helpers import cuda, host, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+TILTS = np.array([0.0, 20.0, -44.9, 45.2, -63.0], np.float32)
+
+
+def _case(dims, psi, W=26, H=22):
+    import artiatomi_b200 as E
+    from oracle import geometry as G
+
+    nx, ny, nz = dims
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    vol = (np.cos(0.4 * x + 0.2 * y) + 0.6 * np.sin(0.3 * z - 0.25 * x + 0.3 * y)).astype(np.float32)
+    n = len(TILTS)
+    xs, ys = np.linspace(-1.3, 1.1, n).astype(np.float32), np.linspace(0.9, -0.8, n).astype(np.float32)
+    ps = np.full(n, psi, np.float32)
+    return dict(vol=vol, W=W, H=H, vg=E.volume_geometry(dims), vo=G.volume_geometry(dims),
+                pg=E.projection_geometry(E.Markers(TILTS, xs, ys, None, ps), W, H),
+                og=G.projection_geometry(TILTS, xs, ys, None, ps, W, H))
+
+
+@pytest.mark.parametrize("dims", [(3, 5, 2), (4, 9, 1), (1, 6, 7), (33, 17, 5), (5, 8, 40), (70, 12, 9)])
+@pytest.mark.parametrize("psi", [0.0, 90.0, 37.0])
+def test_axis_projection_small_and_odd(dims, psi):
+    import torch
+
+    import artiatomi_b200 as E
+    from oracle import driver as D, geometry as G
+
+    c = _case(dims, psi)
+    W, H = c["W"], c["H"]
+    for i in range(len(TILTS)):
+        k = E.set_constant_values(c["pg"][i], c["vg"])
+        (p32, _), (p64, do) = [(np.zeros((H, W), np.float32), np.zeros((H, W), np.float32)) for _ in range(2)]
+        g = G.orc_geom(c["og"][i], c["vo"])
+        D.fp_march(g, c["vol"], 0, W, H, p32, np.zeros((H, W), np.float32), precision=0)
+        D.fp_march(g, c["vol"], 0, W, H, p64, do, precision=1)
+        for dtype in (torch.float32, torch.float16):
+            proj, dist = torch.zeros((H, W), device="cuda"), torch.zeros((H, W), device="cuda")
+            E.forward_project(k, cuda(c["vol"]).to(dtype), proj, dist, fast=True)
+            # half storage rounds each voxel by up to 2^-11 of its value
+            tol = 5e-4 if dtype == torch.float32 else 1e-3
+            p = host(proj)
+            err = np.linalg.norm(np.minimum(np.abs(p - p64), np.abs(p - p32))) / np.linalg.norm(p64)
+            assert err <= tol, (i, dtype, err)
+            # entry and exit (|t| ~ 1e4) are rounded to 2^-10 in float
+            assert np.abs(host(dist) - do).max() <= 2.5e-3
+
+
+@pytest.mark.parametrize("dims", [(33, 17, 5), (12, 9, 30)])
+@pytest.mark.parametrize("psi", [0.0, 90.0])
+def test_axis_slabs_add_up(dims, psi):
+    """The slab images of the fused slicer through a reconstructor without
+    a CTF effect: every slab's first sample is the one at the ray's start, so
+    a slab image is compared with the faithful slicer's, slab by slab, through
+    the CTF chain of both variants."""
+    import torch
+
+    import artiatomi_b200 as E
+
+    c = _case(dims, psi)
+    W, H, n = c["W"], c["H"], len(TILTS)
+    defocus = np.tile(np.array([2900.0, 3100.0, 20.0], np.float32), n)
+    kw = dict(ctf_mode=True, pixel_size_nm=0.27, ctf_slice_thickness_nm=1.9, ctf_beta_fac=(10.0, 0.0, 0.008, 0.0),
+              cut_length=(1.0, 1.0), dim_length=(2.0, 2.0))
+    got = []
+    for variant in (E.VARIANT_FAST, E.VARIANT_FAITHFUL):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=variant, **kw), c["pg"], TILTS, defocus)
+        images = []
+        for i in range(n):
+            rec.reset_projections()
+            rec.forward_projection(c["vg"], cuda(c["vol"]), i)
+            torch.cuda.synchronize()
+            images.append(host(rec.views()[0]).copy())
+        rec.close()
+        got.append(np.stack(images))
+    assert np.abs(got[1]).max() > 0
+    assert rel_l2(got[0], got[1]) <= 5e-4, rel_l2(got[0], got[1])
