@@ -25,7 +25,7 @@
 // Gauss-Newton terms) are formed, and the ray is walked a second time to
 // scatter the residual for dL/dx. Nothing is stored per ray: the second walk
 // recomputes what it needs.
-#include "esb_ray_core.cuh"
+#include "esb_axis.cuh"
 
 namespace esb {
 
@@ -265,18 +265,178 @@ struct Scatter {
 };
 
 // Thread layout of the fast projector: 4 sub-rays of a pixel in adjacent
-// lanes, a warp spans 8 detector rows, 8 warps 8 detector columns.
+// lanes, a warp spans 8 detector rows (columns with `swap`), 8 warps 8
+// detector columns (rows).
 struct PixelLanes {
   int lane, sub, x, y;
   bool active;
-  __device__ PixelLanes(int x0, int y0, int x1, int y1) {
+  __device__ PixelLanes(int x0, int y0, int x1, int y1, int swap = 0) {
     lane = threadIdx.x & 31;
     sub = lane & 3;
-    const int row = (threadIdx.x >> 2) & 7;
-    const int warp = threadIdx.x >> 5;
-    x = x0 + (int)blockIdx.x * 8 + warp;
-    y = y0 + (int)blockIdx.y * 8 + row;
+    const int along = (int)blockIdx.y * 8 + ((threadIdx.x >> 2) & 7);
+    const int across = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+    x = x0 + (swap ? along : across);
+    y = y0 + (swap ? across : along);
     active = x < x1 && y < y1;
+  }
+};
+
+// ------------------------------------------------------- single-axis rays
+// The layer walk of the forward projector's axis kernels (axis_walk in
+// esb_projector_fast.cu: the same samples, cells and weights) as a sequence
+// of rows of voxels with their weights. A row gets the far weights of the
+// layer before it and the near weights of the layer after it, at the minor
+// positions n - 1 .. n + 2 of the cell n that the ray is in: first only after
+// a crossing, last only before one.
+//
+// Compared with the walk from cell to cell (walk_xz) a row costs 4 corner
+// accesses in each y plane at most instead of 8 per cell, and the lanes of a
+// warp stay together: the loop has one step per layer for every ray.
+struct AxisWalk {
+  int sM, sN;      // step signs
+  int nM, nN;      // voxels along the major and minor axis
+  long dM, dN;     // their element strides
+};
+
+// v.row(im, in, w, wa, wc, first, last): voxel row im, cell in (indices, may
+// lie outside the volume), weights of the value and of its derivatives along
+// the mirrored minor and major axis at the 4 positions; first / last: the
+// outer positions have weights.
+template <bool GRAD, class V>
+__device__ __forceinline__ void axis_rows(const AxisStep& A, const AxisWalk& W, float Mq, float Nq, int J, V& v) {
+  const float fm = floorf(Mq), fn = floorf(Nq);
+  const float nM0 = ((fm + 1.f) - Mq) * A.isM;
+  const float nN0 = A.isN > 0.f ? ((fn + 1.f) - Nq) * A.isN : FLT_MAX;
+  const float Mt = (float)J;
+  float relN = __fmaf_rn(-0.5f, A.dN, __fsub_rn(Nq, fn)), relM = __fmaf_rn(-0.5f, A.dM, __fsub_rn(Mq, fm));
+  int im = W.sM * (int)fm, in = W.sN * (int)fn;
+  float k = 0.f, kn = 0.f, fm0 = 0.f;
+  float g0 = 0.f, g1 = 0.f, g2 = 0.f, a0 = 0.f, a1 = 0.f, a2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
+  bool Xp = false;
+#pragma unroll 1
+  for (int guard = 0; guard < 1 << 20; ++guard) {
+    const float nMs = __fmaf_rn(k, A.isM, nM0), nNs = __fmaf_rn(kn, A.isN, nN0);
+    const bool X = nNs <= nMs;
+    const float tL = fminf(nMs, Mt);
+    const float2 f = ceil2(fminf(nNs, tL), tL);
+    const float2 M = make_float2(f.x - fm0, f.y - f.x);
+    const float sA = fm0 + f.x, sB = f.x + f.y;
+    const float2 a = make_float2(fmaf(sA, A.hN, relN), fmaf(sB, A.hN, relN - 1.f));
+    const float2 c = make_float2(fmaf(sA, A.hM, relM), fmaf(sB, A.hM, relM));
+    const float2 Ma = make_float2(M.x * a.x, M.y * a.y), Mc = make_float2(M.x * c.x, M.y * c.y);
+    const float tA = M.x * fmaf(a.x, c.x, fmaf(M.x * M.x, A.g, -A.g));
+    const float tB = M.y * fmaf(a.y, c.y, fmaf(M.y * M.y, A.g, -A.g));
+    const float2 uM = make_float2(M.x - Mc.x, M.y - Mc.y), vM = make_float2(M.x - Ma.x, M.y - Ma.y);
+    // value: corners (n, m), (n + 1, m), (n, m + 1), (n + 1, m + 1) of a cell
+    // get M - Ma - Mc + t, Ma - t, Mc - t, t
+    const float w[4] = {g0, g1 + (vM.x - (Mc.x - tA)), g2 + ((Ma.x - tA) + (vM.y - (Mc.y - tB))), Ma.y - tB};
+    const float wa[4] = {a0, a1 - uM.x, a2 + (uM.x - uM.y), uM.y};
+    const float wc[4] = {c0, c1 - vM.x, c2 - (Ma.x + vM.y), -Ma.y};
+    v.row(im, in, w, wa, wc, Xp, X);
+    const float F0 = Mc.x - tA, F1 = tA + (Mc.y - tB), F2 = tB;
+    g0 = X ? F0 : 0.f;
+    g1 = X ? F1 : F0;
+    g2 = X ? F2 : F1;
+    if (GRAD) {
+      const float A0 = -Mc.x, A1 = Mc.x - Mc.y, A2 = Mc.y, C0 = vM.x, C1 = Ma.x + vM.y, C2 = Ma.y;
+      a0 = X ? A0 : 0.f;
+      a1 = X ? A1 : A0;
+      a2 = X ? A2 : A1;
+      c0 = X ? C0 : 0.f;
+      c1 = X ? C1 : C0;
+      c2 = X ? C2 : C1;
+    }
+    fm0 = f.y;
+    k += 1.f;
+    relM -= 1.f;
+    im += W.sM;
+    if (X) {
+      relN -= 1.f;
+      kn += 1.f;
+      in += W.sN;
+    }
+    Xp = X;
+    if (fm0 >= Mt) break;
+  }
+  const float w[4] = {g0, g1, g2, 0.f}, wa[4] = {a0, a1, a2, 0.f}, wc[4] = {c0, c1, c2, 0.f};
+  v.row(im, in, w, wa, wc, Xp, false);
+}
+
+// Offsets of a row's 4 positions, clamped to the volume.
+struct RowOffsets {
+  long o[4];
+  __device__ __forceinline__ RowOffsets(const AxisWalk& W, int im, int in, long y) {
+    const long row = (long)clampi(im, W.nM) * W.dM + y;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = row + (long)clampi(in + W.sN * (j - 1), W.nN) * W.dN;
+  }
+};
+
+// Value and derivative sums over planes iy (0) and iy + 1 (1).
+template <int VT>
+struct AxisForward {
+  const void* __restrict__ vol;
+  const AxisWalk& W;
+  long y0, y1;
+  float S0 = 0.f, S1 = 0.f, A0 = 0.f, A1 = 0.f, C0 = 0.f, C1 = 0.f;
+  __device__ __forceinline__ void row(int im, int in, const float* w, const float* wa, const float* wc, bool first,
+                                      bool last) {
+    const RowOffsets R(W, im, in, 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if ((j == 0 && !first) || (j == 3 && !last)) continue;
+      const float p = Voxel<VT>::load(vol, R.o[j] + y0), q = Voxel<VT>::load(vol, R.o[j] + y1);
+      S0 = fmaf(p, w[j], S0);
+      S1 = fmaf(q, w[j], S1);
+      A0 = fmaf(p, wa[j], A0);
+      A1 = fmaf(q, wa[j], A1);
+      C0 = fmaf(p, wc[j], C0);
+      C1 = fmaf(q, wc[j], C1);
+    }
+  }
+};
+
+// Adds b0 * weight to plane iy and b1 * weight to plane iy + 1.
+struct AxisScatter {
+  float* __restrict__ g;
+  const AxisWalk& W;
+  long y0, y1;
+  float b0, b1;
+  __device__ __forceinline__ void row(int im, int in, const float* w, const float*, const float*, bool first,
+                                      bool last) {
+    const RowOffsets R(W, im, in, 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if ((j == 0 && !first) || (j == 3 && !last)) continue;
+      atomicAdd(g + R.o[j] + y0, b0 * w[j]);
+      atomicAdd(g + R.o[j] + y1, b1 * w[j]);
+    }
+  }
+};
+
+// One sub-ray that fits the launch (its step the launch's, its y in one
+// cell): its start and its planes. ok = false: walk_ray takes it.
+struct AxisRay {
+  float Mq, Nq, b;
+  long y0, y1;
+  int J;
+  bool ok;
+  __device__ __forceinline__ AxisRay(const KConst& c, const AxisStep& A, const AxisWalk& W, bool zmaj, float3 s,
+                                     float t0, float tout, float3 d) {
+    float step;
+    J = progression(t0, tout, c.vs.x * 0.15f, step, ok);
+    float3 q = interp_coord(c, ray_point(c, s, t0));
+    q = make_float3(__fadd_rn(q.x, d.x), __fadd_rn(q.y, d.y), __fadd_rn(q.z, d.z));
+    const float dqy = interp_step(c, step).y;
+    const float fy = floorf(q.y);
+    ok = ok && step == A.step && fabsf(dqy) * (float)J < 1e-5f && fy == floorf(qpos(q.y, J - 1, dqy));
+    const float m = zmaj ? q.z : q.x, n = zmaj ? q.x : q.z;
+    Mq = W.sM > 0 ? m : -m;
+    Nq = W.sN > 0 ? n : -n;
+    b = q.y - fy;
+    const int ny = (int)c.dim.y, iy = (int)fy;
+    y0 = (long)clampi(iy, ny) * (long)c.dim.x;
+    y1 = (long)clampi(iy + 1, ny) * (long)c.dim.x;
   }
 };
 
@@ -302,9 +462,13 @@ __device__ __forceinline__ float3 shift_offset(const float3& tu, const float3& t
   return make_float3(su * tu.x + sv * tv.x, su * tu.y + sv * tv.y, su * tu.z + sv * tv.z);
 }
 
-__global__ void __launch_bounds__(256) k_fp_adjoint(KConst c, float* __restrict__ grad, const float* __restrict__ img,
+// AXIS: single-axis projections (W, A, zmaj; swap: pixel layout).
+template <bool AXIS>
+__global__ void __launch_bounds__(256) k_fp_adjoint(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
+                                                    const __grid_constant__ AxisWalk W, int zmaj, int swap,
+                                                    float* __restrict__ grad, const float* __restrict__ img,
                                                     size_t pitchE, float sx, float sy, int x0, int y0, int x1, int y1) {
-  const PixelLanes P(x0, y0, x1, y1);
+  const PixelLanes P(x0, y0, x1, y1, swap);
   if (!P.active) return;
   const float w = img[(size_t)P.y * pitchE + P.x] * (c.vs.x * 0.15f * 0.25f);
   if (w == 0.0f) return;
@@ -315,7 +479,16 @@ __global__ void __launch_bounds__(256) k_fp_adjoint(KConst c, float* __restrict_
   float3 tu, tv;
   shift_axes(c, tu, tv);
   Scatter S{grad, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y, w};
-  walk_ray(c, s, tin, tout, shift_offset(tu, tv, sx, sy), S);
+  const float3 d = shift_offset(tu, tv, sx, sy);
+  if (AXIS) {
+    const AxisRay R(c, A, W, zmaj != 0, s, tin, tout, d);
+    if (R.ok) {
+      AxisScatter Sc{grad, W, R.y0, R.y1, (1.0f - R.b) * w, R.b * w};
+      axis_rows<false>(A, W, R.Mq, R.Nq, R.J, Sc);
+      return;
+    }
+  }
+  walk_ray(c, s, tin, tout, d, S);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -327,12 +500,15 @@ __device__ __forceinline__ double warp_sum(double v) {
 // out: [0] loss, [1] dL/ds_u, [2] dL/ds_v, [3..5] Gauss-Newton terms
 // sum (dp/ds_u)^2, sum dp/ds_u dp/ds_v, sum (dp/ds_v)^2, and with NOUT = 8
 // [6] sum p^2, [7] sum p * b (all added to).
-template <int VT, int NOUT>
-__global__ void __launch_bounds__(256) k_loss_grad(KConst c, const void* __restrict__ vol,
+// AXIS: single-axis projections (W, A, zmaj; swap: pixel layout).
+template <int VT, int NOUT, bool AXIS>
+__global__ void __launch_bounds__(256) k_loss_grad(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
+                                                   const __grid_constant__ AxisWalk W, int zmaj, int swap,
+                                                   const void* __restrict__ vol,
                                                    const float* __restrict__ meas, size_t pitchE, float sx, float sy,
                                                    float* __restrict__ grad, float* __restrict__ proj_out,
                                                    double* __restrict__ out, int x0, int y0, int x1, int y1) {
-  const PixelLanes P(x0, y0, x1, y1);
+  const PixelLanes P(x0, y0, x1, y1, swap);
   const float kappa = c.vs.x * 0.15f * 0.25f;
   float3 s = make_float3(0.f, 0.f, 0.f);
   float tin = 0.f, tout = -1.f;
@@ -346,11 +522,28 @@ __global__ void __launch_bounds__(256) k_loss_grad(KConst c, const void* __restr
     hit(s, c.n, c.bbMin, c.bbMax, tin, tout);
     hitray = tout - tin > 0.0f;
     if (hitray) {
-      FwdGrad<VT> F{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
-      walk_ray(c, s, tin, tout, d, F);
-      sum = F.sum;
-      gx = F.ga * tu.x + F.gb * tu.y + F.gc * tu.z;
-      gy = F.ga * tv.x + F.gb * tv.y + F.gc * tv.z;
+      float3 gr;  // derivatives along x, y, z
+      bool done = false;
+      if (AXIS) {
+        const AxisRay R(c, A, W, zmaj != 0, s, tin, tout, d);
+        if (R.ok) {
+          AxisForward<VT> F{vol, W, R.y0, R.y1};
+          axis_rows<true>(A, W, R.Mq, R.Nq, R.J, F);
+          const float ib = 1.0f - R.b;
+          sum = fmaf(R.b, F.S1, ib * F.S0);
+          const float n = (float)W.sN * fmaf(R.b, F.A1, ib * F.A0), m = (float)W.sM * fmaf(R.b, F.C1, ib * F.C0);
+          gr = make_float3(zmaj ? n : m, F.S1 - F.S0, zmaj ? m : n);
+          done = true;
+        }
+      }
+      if (!done) {
+        FwdGrad<VT> F{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
+        walk_ray(c, s, tin, tout, d, F);
+        sum = F.sum;
+        gr = make_float3(F.ga, F.gb, F.gc);
+      }
+      gx = gr.x * tu.x + gr.y * tu.y + gr.z * tu.z;
+      gy = gr.x * tv.x + gr.y * tv.y + gr.z * tv.z;
     }
   }
   const float sum4 = quad_sum_ordered(sum), gx4 = quad_sum_ordered(gx), gy4 = quad_sum_ordered(gy);
@@ -393,17 +586,48 @@ __global__ void __launch_bounds__(256) k_loss_grad(KConst c, const void* __restr
   if (!grad) return;
   r = __shfl_sync(0xffffffffu, r, P.lane & ~3);
   if (!hitray || r == 0.0f) return;
+  if (AXIS) {
+    const AxisRay R(c, A, W, zmaj != 0, s, tin, tout, d);
+    if (R.ok) {
+      const float w = r * kappa;
+      AxisScatter Sc{grad, W, R.y0, R.y1, (1.0f - R.b) * w, R.b * w};
+      axis_rows<false>(A, W, R.Mq, R.Nq, R.J, Sc);
+      return;
+    }
+  }
   Scatter Sc{grad, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y, r * kappa};
   walk_ray(c, s, tin, tout, d, Sc);
 }
+
+// The axis kernels' parameters of a launch; axis = false: any geometry.
+struct AxisLaunch {
+  bool axis;
+  int zmaj, swap;
+  AxisStep A;
+  AxisWalk W;
+  explicit AxisLaunch(const KConst& c) {
+    bool z;
+    A = axis_step(c, z, W.sM, W.sN);
+    axis = axis_projection(c) && A.step > 0.0f;
+    zmaj = z ? 1 : 0;
+    swap = axis ? axis_swap(c) : 0;
+    const long sz = (long)c.dim.x * (long)c.dim.y;
+    W.nM = (int)(z ? c.dim.z : c.dim.x);
+    W.nN = (int)(z ? c.dim.x : c.dim.z);
+    W.dM = z ? sz : 1;
+    W.dN = z ? 1 : sz;
+  }
+};
 
 }  // namespace
 
 cudaError_t launch_fp_adjoint(const KConst& c, float* grad, const float* img, size_t pitchE, float sx, float sy, int w,
                               int h, cudaStream_t st) {
   if (w <= 0 || h <= 0) return cudaSuccess;
-  dim3 blk(256), grd((w + 7) / 8, (h + 7) / 8);
-  k_fp_adjoint<<<grd, blk, 0, st>>>(c, grad, img, pitchE, sx, sy, 0, 0, w, h);
+  const AxisLaunch L(c);
+  const dim3 blk(256), grd = axis_grid(L.swap, 8, w, h);
+  if (L.axis) k_fp_adjoint<true><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, grad, img, pitchE, sx, sy, 0, 0, w, h);
+  else k_fp_adjoint<false><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, grad, img, pitchE, sx, sy, 0, 0, w, h);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -416,9 +640,16 @@ cudaError_t launch_loss_grad(const KConst& c, const void* vol, int vt, const flo
   // 8 sums, with the amplitude moments)
   const int x0 = roi ? roi[0] : 0, y0 = roi ? roi[1] : 0, x1 = roi ? roi[2] : w, y1 = roi ? roi[3] : h;
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
-  dim3 blk(256), grd((x1 - x0 + 7) / 8, (y1 - y0 + 7) / 8);
-#define ESB_LG(VT, N) \
-  k_loss_grad<VT, N><<<grd, blk, 0, st>>>(c, vol, meas, pitchE, sx, sy, grad, proj_out, out, x0, y0, x1, y1)
+  const AxisLaunch L(c);
+  const dim3 blk(256), grd = axis_grid(L.swap, 8, x1 - x0, y1 - y0);
+#define ESB_LG1(VT, N, AX)                                                                                        \
+  k_loss_grad<VT, N, AX><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, meas, pitchE, sx, sy, grad, proj_out, \
+                                              out, x0, y0, x1, y1)
+#define ESB_LG(VT, N)                   \
+  do {                                  \
+    if (L.axis) ESB_LG1(VT, N, true);   \
+    else ESB_LG1(VT, N, false);         \
+  } while (0)
   if (roi) {
     if (vt == ESB_VOXEL_F32) ESB_LG(ESB_VOXEL_F32, 8);
     else if (vt == ESB_VOXEL_F16) ESB_LG(ESB_VOXEL_F16, 8);
@@ -429,6 +660,7 @@ cudaError_t launch_loss_grad(const KConst& c, const void* vol, int vt, const flo
     else ESB_LG(ESB_VOXEL_BF16, 6);
   }
 #undef ESB_LG
+#undef ESB_LG1
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }

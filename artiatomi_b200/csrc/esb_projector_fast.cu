@@ -26,7 +26,7 @@
 // are combined with warp shuffles.
 #include <float.h>
 
-#include "esb_ray_core.cuh"
+#include "esb_axis.cuh"
 
 namespace esb {
 
@@ -433,19 +433,6 @@ __device__ __forceinline__ float cvt(typename RawVoxel<VT>::T r) {
   else return __uint_as_float((unsigned)r << 16);
 }
 
-__device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
-
-// Steps of the walk, the same for every ray of a launch whose samples lie in
-// one binade of the ray parameter (axis_step on the host; a ray with another
-// step takes ray_sum).
-struct AxisStep {
-  float step;          // of the ray parameter
-  float dM, dN;        // |step| of the major and minor coordinate, dM >= dN
-  float isM, isN;      // 1 / dM, and 1 / dN (0 for dN = 0)
-  float hM, hN;        // dM / 2, dN / 2
-  float g;             // dN dM / 12
-};
-
 // Sum of the trilinear interpolant over samples j0 .. J-1 of one ray whose y
 // interpolation coordinate lies in cell iy with weight b, walked along major
 // axis z (ZMAJ) or x with step signs SM (major) and SN (minor). Mq, Nq:
@@ -509,7 +496,7 @@ __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C,
   const float kEnd = fminf(floorf((Mt - nM0) * A.dM), SM > 0 ? (float)(nM - 1) - fm : -fm);
   // one layer: row values v* (plane iy) and w* (plane iy + 1) at n - 1 .. n + 2
   auto layer = [&](bool X, float tA, float tL, Raw va, Raw vb, Raw vc, Raw vd, Raw wa, Raw wb, Raw wc, Raw wd) {
-    const float2 f = __fadd2_rn(__fadd2_ru(make_float2(tA, tL), splat(8388608.0f)), splat(-8388608.0f));  // ceil
+    const float2 f = ceil2(tA, tL);
     // samples [fm0, f.x) lie in cell A, [f.x, f.y) in cell B
     const float2 M = make_float2(f.x - fm0, f.y - f.x), mM = make_float2(fm0 - f.x, f.x - f.y);
     const float sA = fm0 + f.x, sB = f.x + f.y;
@@ -764,56 +751,6 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
     if (P.active && P.sub == 0 && k >= klo && k <= khi)
       imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
   }
-}
-
-// Beam directions whose rays all stay in one y plane take the axis kernels.
-bool axis_projection(const KConst& c) { return fabsf(c.n.y) <= 1e-6f; }
-
-// Instance of the axis kernels for the launch's beam direction (major axis z
-// when |dq.z| >= |dq.x|, step signs) and its steps: the step of the ray
-// parameter is the one of the binade that holds the volume's centre.
-AxisStep axis_step(const KConst& c, bool& zmaj, int& sm, int& sn) {
-  const float h = c.vs.x * 0.15f;
-  double t = 0.0;
-  const double n[3] = {c.n.x, c.n.y, c.n.z}, d[3] = {c.det.x, c.det.y, c.det.z};
-  const double lo[3] = {c.bbMin.x, c.bbMin.y, c.bbMin.z}, hi[3] = {c.bbMax.x, c.bbMax.y, c.bbMax.z};
-  for (int j = 0; j < 3; ++j) t += n[j] * (0.5 * (lo[j] + hi[j]) - d[j]);
-  int e = 0;
-  frexp(t, &e);
-  volatile float t0 = (float)ldexp(0.5, e), t1 = t0 + h;  // single roundings, as the kernel's
-  AxisStep A;
-  A.step = t > 0.0 ? t1 - t0 : 0.0f;  // 0: no ray takes the walk
-  volatile float qx = A.step * c.n.x, qz = A.step * c.n.z;
-  qx = qx * c.bbRcp.x;
-  qz = qz * c.bbRcp.z;
-  qx = qx * c.dim.x;
-  qz = qz * c.dim.z;
-  zmaj = fabsf(qz) >= fabsf(qx);
-  const float m = zmaj ? qz : qx, nn = zmaj ? qx : qz;
-  sm = m < 0.f ? -1 : 1;
-  sn = nn < 0.f ? -1 : 1;
-  A.dM = fabsf(m);
-  A.dN = fabsf(nn);
-  if (!(A.dM > 0.f)) A.step = 0.0f;
-  A.isM = 1.0f / A.dM;
-  A.isN = A.dN > 0.f ? 1.0f / A.dN : 0.f;
-  A.hM = 0.5f * A.dM;
-  A.hN = 0.5f * A.dN;
-  A.g = A.dN * A.dM * (1.0f / 12.0f);
-  return A;
-}
-
-// Whether the warps of the axis kernels span detector columns (u) instead of
-// rows: when a pixel step along u moves the ray less across the volume's y
-// planes than one along v.
-int axis_swap(const KConst& c) {
-  const float uy = c.aniso[0] * c.u.y + c.aniso[3] * c.v.y, vy = c.aniso[1] * c.u.y + c.aniso[4] * c.v.y;
-  return fabsf(uy) < fabsf(vy) ? 1 : 0;
-}
-
-dim3 axis_grid(int swap, int nw, int w, int h) {
-  const int along = swap ? w : h, across = swap ? h : w;
-  return dim3((across + nw - 1) / nw, (along + 7) / 8);
 }
 
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.

@@ -95,3 +95,32 @@ def test_axis_slabs_add_up(dims, psi):
         got.append(np.stack(images))
     assert np.abs(got[1]).max() > 0
     assert rel_l2(got[0], got[1]) <= 5e-4, rel_l2(got[0], got[1])
+
+
+@pytest.mark.parametrize("dims", [(3, 5, 2), (4, 9, 1), (1, 6, 7), (33, 17, 5), (5, 8, 40)])
+@pytest.mark.parametrize("psi", [0.0, 90.0, 37.0])
+def test_axis_adjoint_small_and_odd(dims, psi):
+    """The gradient kernels' walk: fp_adjoint is the transpose of the loss
+    kernel's model, and the loss kernel's volume gradient for zero measured
+    values the adjoint of its projection. Both hold to the FP32 rounding of
+    the sums (~1e-6 of the Cauchy-Schwarz bound; 1e-5 allowed)."""
+    import torch
+
+    import artiatomi_b200 as E
+
+    c = _case(dims, psi)
+    x = cuda(c["vol"])
+    rng = np.random.default_rng(4)
+    for i in range(len(TILTS)):
+        k = E.set_constant_values(c["pg"][i], c["vg"])
+        for shift in ((0.0, 0.0), (0.7, -1.2)):
+            ax = torch.zeros((c["H"], c["W"]), device="cuda")
+            grad, out = torch.zeros_like(x), torch.zeros(6, device="cuda", dtype=torch.float64)
+            E.projection_loss_grad(k, x, torch.zeros_like(ax), out, shift=shift, grad=grad, proj_out=ax)
+            y = cuda(rng.normal(size=tuple(ax.shape)).astype(np.float32))
+            aty, atax = torch.zeros_like(x), torch.zeros_like(x)
+            E.fp_adjoint(k, aty, y, shift=shift)
+            E.fp_adjoint(k, atax, ax, shift=shift)
+            lhs, rhs = float((ax.double() * y.double()).sum()), float((x.double() * aty.double()).sum())
+            assert abs(lhs - rhs) <= 1e-5 * float(ax.double().norm() * y.double().norm()), (i, shift, lhs, rhs)
+            assert rel_l2(host(grad), host(atax)) <= 1e-5, (i, shift)
