@@ -78,14 +78,13 @@ __global__ void __launch_bounds__(128) k_bp_fast(KConst k, BpGeom g, void* __res
   }
 }
 
-// k_bp_fast for single-axis tilt series (axis_sums): on pre-sampled slab
-// images (UP: one load per sample) or reading the slab images directly.
-template <int VT, bool UP>
+// k_bp_fast for single-axis tilt series (axis_sums), reading the slab images
+// directly.
+template <int VT>
 __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __restrict__ vol,
                                                  const float* __restrict__ imgs, size_t img_stride, SlabTable slabs,
                                                  int pw, int ph, size_t pitchE, float lambda, int os, float inv,
-                                                 float distMin, float distMax, int linear, int transposed,
-                                                 const float2* __restrict__ ups, size_t up_stride, int z0) {
+                                                 float distMin, float distMax, int linear, int transposed, int z0) {
   // plane z0 + blockIdx.z of the geometry, stored at plane blockIdx.z of vol
   // (z0 = 0 but for the autotuner's trial launches on a scratch slab)
   const int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -97,15 +96,11 @@ __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __r
   const int x = 4 * q;
   const float depth = macro_depth(k, x, y, z);
   const float* img = imgs;
-  const float2* up = ups;
   if (slabs.count > 0) {
     if (!(depth >= slabs.bound[0] && depth < slabs.bound[slabs.count])) return;
     int s = 0;
     while (s + 1 < slabs.count && depth >= slabs.bound[s + 1]) ++s;
-    if (UP)
-      up += (size_t)s * up_stride;
-    else
-      img += (size_t)s * img_stride;
+    img += (size_t)s * img_stride;
   } else if (!(depth >= distMin && depth < distMax)) {
     return;
   }
@@ -116,7 +111,6 @@ __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __r
   } else {
     macro_rect(g, x, y, z, pw, ph, pbx, pby, pbz, pbw);
   }
-  const int upH = ph * os;
   const float fos = (float)os;
   const float cy = k.bbMin.y + ((float)y + 0.5f) * k.vs.y, cz = k.bbMin.z + ((float)z + 0.5f) * k.vs.z;
   const float uyz = g.U.y * cy + g.U.z * cz + g.U0, vyz = g.V.y * cy + g.V.z * cz + g.V0;
@@ -126,32 +120,21 @@ __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __r
   const size_t sx = tr ? (size_t)ph : 1, sy = tr ? 1 : pitchE;
   const long base = ((long)zl * ny + y) * (long)k.dim.x + x;
   float res[4], has[4];
-  if (UP) {
-    auto read = [&](int mu, int mv) -> float2 { return __ldg(up + (size_t)mu * upH + mv); };
+  auto read = [&](int mu, int mv) -> float {
+    const float px = ((float)mu + 0.5f) * inv, py = ((float)mv + 0.5f) * inv;
+    return interior ? sample_interior(img, sx, sy, px, py, lin) : sample_image(img, pw, ph, pitchE, px, py, lin, tr);
+  };
+  const bool patch = os == 2 && lin && interior;
+  const float cx0 = k.bbMin.x + ((float)x + 0.5f) * k.vs.x;
+  const RowAnchor anchor(g, y, g.U.x * cx0 + uyz, g.V.x * cx0 + vyz, fos);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float cx = k.bbMin.x + ((float)(x + i) + 0.5f) * k.vs.x;
-      const float uc = g.U.x * cx + uyz, vc = g.V.x * cx + vyz;
-      axis_sums_rows(g, uc, vc, fos, inv, dwv, y, pbx * os, pby * os - 1, pbz * os, pbw * os - 1, read, res[i],
-                     has[i]);
-    }
-  } else {
-    auto read = [&](int mu, int mv) -> float {
-      const float px = ((float)mu + 0.5f) * inv, py = ((float)mv + 0.5f) * inv;
-      return interior ? sample_interior(img, sx, sy, px, py, lin) : sample_image(img, pw, ph, pitchE, px, py, lin, tr);
-    };
-    const bool patch = os == 2 && lin && interior;
-    const float cx0 = k.bbMin.x + ((float)x + 0.5f) * k.vs.x;
-    const RowAnchor anchor(g, y, g.U.x * cx0 + uyz, g.V.x * cx0 + vyz, fos);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float cx = k.bbMin.x + ((float)(x + i) + 0.5f) * k.vs.x;
-      const float uc = g.U.x * cx + uyz, vc = g.V.x * cx + vyz;
-      if (!(patch && axis_sums_os2(g, uc, vc, dwv, anchor, pbx * 2, pby * 2 - 1, pbz * 2, pbw * 2 - 1, img, sx, sy,
-                                   pw, ph, res[i], has[i])))
-        axis_sums(g, uc, vc, fos, inv, dwv, anchor, pbx * os, pby * os - 1, pbz * os, pbw * os - 1, read, res[i],
-                  has[i]);
-    }
+  for (int i = 0; i < 4; ++i) {
+    const float cx = k.bbMin.x + ((float)(x + i) + 0.5f) * k.vs.x;
+    const float uc = g.U.x * cx + uyz, vc = g.V.x * cx + vyz;
+    if (!(patch && axis_sums_os2(g, uc, vc, dwv, anchor, pbx * 2, pby * 2 - 1, pbz * 2, pbw * 2 - 1, img, sx, sy, pw,
+                                 ph, res[i], has[i])))
+      axis_sums(g, uc, vc, fos, inv, dwv, anchor, pbx * os, pby * os - 1, pbz * os, pbw * os - 1, read, res[i],
+                has[i]);
   }
   if (VT == ESB_VOXEL_F32 && (((uintptr_t)((float*)vol + base)) & 15) == 0) {
     float4 v = *((float4*)((float*)vol + base));
@@ -169,11 +152,43 @@ __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __r
   }
 }
 
+// Threads of a block of (quads x rows): a group of min(blockDim.x, 32)
+// threads covers 4 voxels per thread of one volume row (up_voxels).
+struct UpThread {
+  int lanes, lane, x0, y;
+  __device__ __forceinline__ UpThread() {
+    lanes = min((int)blockDim.x, 32);
+    lane = (int)threadIdx.x & (lanes - 1);
+    x0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x - lane);
+    y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  }
+};
+
+// k_bp_axis on pre-sampled slab images (k_upsample): one load per sample.
+template <int VT, int NC>
+__global__ void __launch_bounds__(128) k_bp_up(const __grid_constant__ KConst k, const __grid_constant__ AxisGeom a,
+                                               const __grid_constant__ UpGeom g, void* __restrict__ vol,
+                                               const __grid_constant__ SlabTable slabs, int pw, int ph, float lambda,
+                                               int os, float distMin, float distMax, const float2* __restrict__ ups,
+                                               size_t up_stride, int z0) {
+  // plane z0 + blockIdx.z of the geometry, stored at plane blockIdx.z of vol
+  // (z0 = 0 but for the autotuner's trial launches on a scratch slab)
+  const UpThread t;
+  const int z = z0 + (int)blockIdx.z;
+  const int ny = (int)k.dim.y;
+  const long base = ((long)blockIdx.z * ny + t.y) * (long)k.dim.x + t.x0 + t.lane;
+  up_voxels<NC>(k, a, g, slabs.bound, slabs.count, distMin, distMax, ups, up_stride, pw, ph, os, t.x0, t.lane, t.lanes,
+            t.y, z, t.y < ny && z < (int)k.dim.z, [&](int i, float acc, float dacc) {
+              const long at = base + t.lanes * i;
+              Voxel<VT>::store(vol, at, Voxel<VT>::loadrw(vol, at) + __fdividef(lambda * acc, dacc));
+            });
+}
+
 // One ordered subset back-projected in one pass over the volume (the
 // SIRTCount back-projections of EmSart.cpp:649-673): each quad is read once,
 // the updates of the subset's projections are added to it in the order of
 // the subset, as the per-projection launches add them, and it is stored once.
-// Every projection contributes exactly what k_bp_axis<VT, true> adds for it
+// Every projection contributes exactly what k_bp_up adds for it
 // (pre-sampled slab images, CTF slab chosen by the first corner's depth).
 // FP32 volumes: the result is bit for bit that of the per-projection
 // launches. FP16 / BF16 volumes: the sum is rounded to the storage type once
@@ -181,6 +196,7 @@ __global__ void __launch_bounds__(128) k_bp_axis(KConst k, AxisGeom g, void* __r
 struct BpSetItem {
   KConst k;
   AxisGeom a;
+  UpGeom g;
   const float2* up;  // pre-sampled slab images of this projection
   int nslab;         // 0: no CTF slabs
   float bound[ESB_BP_SET_MAX_SLABS + 1];
@@ -191,91 +207,52 @@ struct BpSet {
   BpSetItem p[ESB_BP_SET_MAX];
 };
 
-template <int VT>
+template <int VT, int NC>
 __global__ void __launch_bounds__(128) k_bp_axis_set(const __grid_constant__ BpSet set, void* __restrict__ vol,
-                                                     int pw, int ph, float lambda, int os, float inv) {
-  const int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+                                                     int pw, int ph, float lambda, int os) {
+  const UpThread t;
   const int z = (int)blockIdx.z;
   const KConst& k0 = set.p[0].k;
-  const int ny = (int)k0.dim.y, nz = (int)k0.dim.z;
-  if (q >= k0.dimXQuarter || y >= ny || z >= nz) return;
-  const int x = 4 * q;
-  const long base = ((long)z * ny + y) * (long)k0.dim.x + x;
-  const bool vec = VT == ESB_VOXEL_F32 && (((uintptr_t)((float*)vol + base)) & 15) == 0;
-  float v[4];
-  if (vec) {
-    const float4 t = *((const float4*)((const float*)vol + base));
-    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-  } else {
+  const int ny = (int)k0.dim.y, nx4 = 4 * k0.dimXQuarter;
+  const bool active = t.y < ny && z < (int)k0.dim.z;
+  const long base = ((long)z * ny + t.y) * (long)k0.dim.x + t.x0 + t.lane;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = Voxel<VT>::loadrw(vol, base + i);
-  }
-  const int upH = ph * os;
-  const float fos = (float)os;
-  bool touched = false;
+  for (int i = 0; i < 4; ++i)
+    if (active && t.x0 + t.lane + t.lanes * i < nx4) v[i] = Voxel<VT>::loadrw(vol, base + t.lanes * i);
+  unsigned touched = 0;
 #pragma unroll 1
   for (int j = 0; j < set.count; ++j) {
     const BpSetItem& it = set.p[j];
-    const KConst& k = it.k;
-    const AxisGeom& g = it.a;
-    const float depth = macro_depth(k, x, y, z);
-    const float2* up = it.up;
-    if (it.nslab > 0) {
-      if (!(depth >= it.bound[0] && depth < it.bound[it.nslab])) continue;
-      int s = 0;
-      while (s + 1 < it.nslab && depth >= it.bound[s + 1]) ++s;
-      up += (size_t)s * set.up_stride;
-    }
-    int pbx, pby, pbz, pbw;
-    if (g.clips) {
-      float d;
-      macro_footprint(k, x, y, z, pw, ph, d, pbx, pby, pbz, pbw);
-    } else {
-      macro_rect(g, x, y, z, pw, ph, pbx, pby, pbz, pbw);
-    }
-    const float cy = k.bbMin.y + ((float)y + 0.5f) * k.vs.y, cz = k.bbMin.z + ((float)z + 0.5f) * k.vs.z;
-    const float uyz = g.U.y * cy + g.U.z * cz + g.U0, vyz = g.V.y * cy + g.V.z * cz + g.V0;
-    const float dwv = inv * g.wv;
-    auto read = [&](int mu, int mv) -> float2 { return __ldg(up + (size_t)mu * upH + mv); };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float cx = k.bbMin.x + ((float)(x + i) + 0.5f) * k.vs.x;
-      const float uc = g.U.x * cx + uyz, vc = g.V.x * cx + vyz;
-      float res, has;
-      axis_sums_rows(g, uc, vc, fos, inv, dwv, y, pbx * os, pby * os - 1, pbz * os, pbw * os - 1, read, res, has);
-      if (has > 0.f) {
-        v[i] += __fdividef(lambda * res, has);
-        touched = true;
-      }
-    }
+    up_voxels<NC>(it.k, it.a, it.g, it.bound, it.nslab, -FLT_MAX, FLT_MAX, it.up, set.up_stride, pw, ph, os, t.x0, t.lane,
+              t.lanes, t.y, z, active, [&](int i, float acc, float dacc) {
+                v[i] += __fdividef(lambda * acc, dacc);
+                touched |= 1u << i;
+              });
   }
-  if (!touched) return;
-  if (vec) {
-    *((float4*)((float*)vol + base)) = make_float4(v[0], v[1], v[2], v[3]);
-  } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) Voxel<VT>::store(vol, base + i, v[i]);
-  }
+  for (int i = 0; i < 4; ++i)
+    if (touched >> i & 1u) Voxel<VT>::store(vol, base + t.lanes * i, v[i]);
 }
 
 // The slab images (transposed, [x][y], stride img_stride) sampled at every
 // sub-pixel grid point, with the voxel row of the grid point's ray:
-// up[s][mu][mv] = (image s at ((mu + 0.5) / os, (mv + 0.5) / os), row as int
-// bits), clamp addressing, nearest or bilinear as the back-projection reads
-// it (sample_row; meaningful for single-axis projections, which read it).
-// The row depends on the grid point and the projection only: it is formed
-// once per grid point and stored with the point's value in every slab image.
+// up[s][mu][mv] (up[s][mv][mu] when swapped: UpGeom) = (image s at
+// ((mu + 0.5) / os, (mv + 0.5) / os), row as int bits), clamp addressing,
+// nearest or bilinear as the back-projection reads it (sample_row;
+// meaningful for single-axis projections, which read it). The row depends on
+// the grid point and the projection only: it is formed once per grid point
+// and stored with the point's value in every slab image.
 __global__ void __launch_bounds__(256) k_upsample(const float* __restrict__ imgs, size_t img_stride, int count, int pw,
-                                                  int ph, int os, float inv, int linear, RowGeom rg,
+                                                  int ph, int os, float inv, int linear, RowGeom rg, int swapped,
                                                   float2* __restrict__ up, size_t up_stride) {
-  const int mv = blockIdx.x * blockDim.x + threadIdx.x;
-  const int mu = blockIdx.y;
-  const int upH = ph * os;
-  if (mv >= upH) return;
+  const int fast = blockIdx.x * blockDim.x + threadIdx.x, slow = blockIdx.y * blockDim.y + threadIdx.y;
+  const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
+  if (fast >= nf || slow >= ns) return;
+  const int mu = swapped ? fast : slow, mv = swapped ? slow : fast;
   const float px = ((float)mu + 0.5f) * inv, py = ((float)mv + 0.5f) * inv;
   const float row = __int_as_float(sample_row(rg, mu, mv));
-  float2* out = up + (size_t)mu * upH + mv;
+  float2* out = up + (size_t)slow * nf + fast;
 #pragma unroll 1
   for (int s = 0; s < count; ++s)
     out[(size_t)s * up_stride] =
@@ -302,17 +279,26 @@ cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float
       grd = dim3((nq + shape->bx - 1) / shape->bx, (ny + shape->by - 1) / shape->by,
                  shape->nz > 0 ? shape->nz : nz - z0);
     }
-#define ESB_AXIS(VT, UP)                                                                                          \
-  k_bp_axis<VT, UP><<<grd, blk, 0, st>>>(k, a, vol, imgs, img_stride, slabs, pw, ph, pitchE, lambda, os, inv, distMin, \
-                                         distMax, linear, transposed, ups, up_stride, z0)
     if (ups) {
-      if (vt == ESB_VOXEL_F32) ESB_AXIS(ESB_VOXEL_F32, true);
-      else if (vt == ESB_VOXEL_F16) ESB_AXIS(ESB_VOXEL_F16, true);
-      else ESB_AXIS(ESB_VOXEL_BF16, true);
+      const UpGeom u = make_up_geom(k, a, pw, ph, os, up_swapped(a));
+#define ESB_AXIS(VT)                                                                                                 \
+  do {                                                                                                               \
+    if (os == 1)                                                                                                     \
+      k_bp_up<VT, 2><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, z0); \
+    else                                                                                                             \
+      k_bp_up<VT, 3><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, z0); \
+  } while (0)
+      if (vt == ESB_VOXEL_F32) ESB_AXIS(ESB_VOXEL_F32);
+      else if (vt == ESB_VOXEL_F16) ESB_AXIS(ESB_VOXEL_F16);
+      else ESB_AXIS(ESB_VOXEL_BF16);
+#undef ESB_AXIS
     } else {
-      if (vt == ESB_VOXEL_F32) ESB_AXIS(ESB_VOXEL_F32, false);
-      else if (vt == ESB_VOXEL_F16) ESB_AXIS(ESB_VOXEL_F16, false);
-      else ESB_AXIS(ESB_VOXEL_BF16, false);
+#define ESB_AXIS(VT)                                                                                              \
+  k_bp_axis<VT><<<grd, blk, 0, st>>>(k, a, vol, imgs, img_stride, slabs, pw, ph, pitchE, lambda, os, inv, distMin, \
+                                     distMax, linear, transposed, z0)
+      if (vt == ESB_VOXEL_F32) ESB_AXIS(ESB_VOXEL_F32);
+      else if (vt == ESB_VOXEL_F16) ESB_AXIS(ESB_VOXEL_F16);
+      else ESB_AXIS(ESB_VOXEL_BF16);
     }
 #undef ESB_AXIS
     ESB_COUNT_LAUNCH();
@@ -367,16 +353,22 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
     BpSetItem& it = set.p[j];
     it.k = ks[j];
     it.a = make_axis_geom(ks[j], g, os);
+    it.g = make_up_geom(ks[j], it.a, pw, ph, os, up_swapped(it.a));
     it.up = ups[j];
     it.nslab = slabs[j].count;
     for (int b = 0; b <= it.nslab; ++b) it.bound[b] = slabs[j].bound[b];
   }
   const int bx = shape ? shape->bx : 32, by = shape ? shape->by : 4;
   const dim3 blk(bx, by, 1), grd((nq + bx - 1) / bx, (ny + by - 1) / by, nz);
-  const float inv = 1.0f / (float)os;
-  if (vt == ESB_VOXEL_F32) k_bp_axis_set<ESB_VOXEL_F32><<<grd, blk, 0, st>>>(set, vol, pw, ph, lambda, os, inv);
-  else if (vt == ESB_VOXEL_F16) k_bp_axis_set<ESB_VOXEL_F16><<<grd, blk, 0, st>>>(set, vol, pw, ph, lambda, os, inv);
-  else k_bp_axis_set<ESB_VOXEL_BF16><<<grd, blk, 0, st>>>(set, vol, pw, ph, lambda, os, inv);
+#define ESB_SET(VT)                                                                    \
+  do {                                                                                 \
+    if (os == 1) k_bp_axis_set<VT, 2><<<grd, blk, 0, st>>>(set, vol, pw, ph, lambda, os); \
+    else k_bp_axis_set<VT, 3><<<grd, blk, 0, st>>>(set, vol, pw, ph, lambda, os);         \
+  } while (0)
+  if (vt == ESB_VOXEL_F32) ESB_SET(ESB_VOXEL_F32);
+  else if (vt == ESB_VOXEL_F16) ESB_SET(ESB_VOXEL_F16);
+  else ESB_SET(ESB_VOXEL_BF16);
+#undef ESB_SET
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -387,9 +379,12 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
 cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_stride, int count, int pw, int ph, int os,
                             int linear, float2* up, size_t up_stride, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
-  dim3 blk(256), grd((ph * os + 255) / 256, pw * os, 1);
+  const BpGeom g = make_geom(k, os);
+  const int swapped = axis_eligible(k, g) && up_swapped(make_axis_geom(k, g, os)) ? 1 : 0;
+  const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
+  const dim3 blk(32, 8), grd((nf + 31) / 32, (ns + 7) / 8);
   k_upsample<<<grd, blk, 0, st>>>(imgs, img_stride, count, pw, ph, os, 1.0f / (float)os, linear, make_row_geom(k, os),
-                                  up, up_stride);
+                                  swapped, up, up_stride);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }

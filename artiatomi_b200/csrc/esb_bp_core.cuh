@@ -5,6 +5,8 @@
 
 #include <float.h>
 
+#include <type_traits>
+
 #include "esb_device.cuh"
 
 namespace esb {
@@ -543,50 +545,199 @@ __device__ __forceinline__ void axis_sums(const AxisGeom& g, float uc, float vc,
   dacc = da;
 }
 
-// axis_sums on images pre-sampled with the voxel row of every sample's ray
-// (k_upsample): read(mu, mv) returns (value, row as int bits), and a sample
-// counts for voxel row yrow when its row is yrow. One 8-byte load per sample;
-// the first 2 x 3 samples of a voxel's shadow are unrolled and read
-// unconditionally.
-template <class Read>
-__device__ __forceinline__ void axis_sums_rows(const AxisGeom& g, float uc, float vc, float fos, float inv, float dwv,
-                                               int yrow, int mu_min, int mu_max, int mv_min, int mv_max,
-                                               const Read& read, float& acc, float& dacc) {
-  const int mu0 = max((int)ceilf((uc - g.hu) * fos - 0.5f), mu_min);
-  const int mu1 = min((int)floorf((uc + g.hu) * fos - 0.5f), mu_max);
-  const int mv0 = max((int)ceilf((vc - g.hv) * fos - 0.5f), mv_min);
-  const int mv1 = min((int)floorf((vc + g.hv) * fos - 0.5f), mv_max);
-  const float dv0 = ((float)mv0 + 0.5f) * inv - vc;
-  float a = 0.f, da = 0.f;
-  // a voxel's shadow holds 2-3 sub-pixel samples per axis at OS 2
-  const int rows = mu1 - mu0 + 1;
-  const int cnt = mv1 - mv0 + 1;
-  auto row = [&](int mu) {
-    const float du = ((float)mu + 0.5f) * inv - uc;
-    const float w = du * g.wu + dv0 * g.wv;
-    auto body = [&](int j) {
-      const float ww = fmaf((float)j, dwv, w);
-      const float2 s = read(mu, mv0 + j);
-      float L = fminf(g.L0, fmaxf(0.f, fmaf(-fabsf(ww), g.K, g.w1K)));
-      L = __float_as_int(s.y) == yrow ? L : 0.f;
-      a = fmaf(s.x, L, a);
-      da += L;
-    };
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      if (j < cnt) body(j);
-#pragma unroll 1
-    for (int j = 3; j < cnt; ++j) body(j);
-  };
+// Geometry of the single-axis back-projection on pre-sampled images
+// (k_upsample), in steps of the sub-pixel grid. The grid's two axes are
+// called fast (contiguous in the pre-sampled image) and slow: the detector
+// axis along which a step in volume x moves more is the fast one (v without
+// in-plane rotation, u for a tilt axis across the image), so that
+// neighbouring voxels of a volume row read neighbouring samples.
+struct UpGeom {
+  double s0, sx, sy, sz;  // slow grid coordinate of voxel (x, y, z)'s centre: s0 + x sx + y sy + z sz (sample m at m)
+  double f0, fx, fy, fz;  // fast grid coordinate
+  float dsx, dfx;         // sx and fx in float
+  float hs, hf;           // half shadow extents
+  // Chord of the sample at offset (ds, df), relative to its plateau:
+  // sat(c - |ds ws + df wf|), the trapezoid of AxisGeom. The update divides
+  // by the chords' sum, so their scale cancels.
+  float ws, wf, c;
+  int smax, fmax;         // last sample that is read, per axis
+  int pitch;              // samples per slow step
+  int swapped;            // fast axis u
+};
+
+// Fast axis u: a step in x moves the projection further along u than along v.
+inline bool up_swapped(const AxisGeom& a) { return fabsf(a.U.x) > fabsf(a.V.x); }
+
+inline UpGeom make_up_geom(const KConst& k, const AxisGeom& a, int pw, int ph, int os, bool swapped) {
+  UpGeom g;
+  const double U[3] = {a.U.x, a.U.y, a.U.z}, V[3] = {a.V.x, a.V.y, a.V.z};
+  const double lo[3] = {k.bbMin.x, k.bbMin.y, k.bbMin.z}, vs[3] = {k.vs.x, k.vs.y, k.vs.z};
+  double u[4] = {os * (double)a.U0 - 0.5}, v[4] = {os * (double)a.V0 - 0.5};
+  for (int j = 0; j < 3; ++j) {
+    u[0] += os * U[j] * (lo[j] + 0.5 * vs[j]);
+    v[0] += os * V[j] * (lo[j] + 0.5 * vs[j]);
+    u[1 + j] = os * U[j] * vs[j];
+    v[1 + j] = os * V[j] * vs[j];
+  }
+  g.swapped = swapped ? 1 : 0;
+  const double* s = g.swapped ? v : u;
+  const double* f = g.swapped ? u : v;
+  g.s0 = s[0], g.sx = s[1], g.sy = s[2], g.sz = s[3];
+  g.f0 = f[0], g.fx = f[1], g.fy = f[2], g.fz = f[3];
+  g.dsx = (float)s[1];
+  g.dfx = (float)f[1];
+  g.hs = (g.swapped ? a.hv : a.hu) * os;
+  g.hf = (g.swapped ? a.hu : a.hv) * os;
+  const double scale = (double)a.K / a.L0 / os;
+  g.ws = (float)((g.swapped ? a.wv : a.wu) * scale);
+  g.wf = (float)((g.swapped ? a.wu : a.wv) * scale);
+  g.c = (float)((double)a.w1K / a.L0);
+  // the rectangle ends before the image's last pixel (macro_rect)
+  const int um = (pw - 1) * os - 1, vm = (ph - 1) * os - 1;
+  g.smax = g.swapped ? vm : um;
+  g.fmax = g.swapped ? um : vm;
+  g.pitch = (g.swapped ? pw : ph) * os;
+  return g;
+}
+
+// sum(sample * chord) and sum(chord) of one voxel whose centre lies at (s, f)
+// relative to a sample of the grid, over the samples of its shadow within
+// [slo, shi] x [flo, fhi] (relative too); on = false: none. at(is, jf, ..)
+// gives the reader of relative sample (is, jf): reader.load(r, j, take) the
+// sample r slow and j fast steps on, read where `take`;
+// reader.mine(t, r, j, taken) whether it counts for the voxel's row,
+// reader.value(t) its value.
+//
+// What bounds it: instruction issue, and the latency of the samples' loads.
+// The bounds are rounded by additions to 1.5 * 2^23 whose bits are the
+// integers (no conversions), the chord is one saturating addition, and the
+// row test predicates the two accumulations: about 6 instructions a sample.
+// The first 2 x NC samples are loaded under predicates before any is used,
+// so that their loads are in flight together.
+template <int NC, class At>
+__device__ __forceinline__ void grid_sums(const UpGeom& g, float s, float f, float slo, float shi, float flo,
+                                          float fhi, bool on, const At& at, float& acc, float& dacc) {
+  const float big = 12582912.0f;  // 1.5 * 2^23, bits 0x4B400000
+  const float sa = fmaxf(__fadd_ru(s - g.hs, big), big + slo), sb = fminf(__fadd_rd(s + g.hs, big), big + shi);
+  const float fa = fmaxf(__fadd_ru(f - g.hf, big), big + flo), fb = fminf(__fadd_rd(f + g.hf, big), big + fhi);
+  const float nf = fb - fa, ns = on && nf >= 0.f ? sb - sa : -1.f;  // samples - 1 per axis
+  const float w = fmaf((sa - big) - s, g.ws, __fmul_rn((fa - big) - f, g.wf));
+  const auto reader = at(__float_as_int(sa) - 0x4B400000, __float_as_int(fa) - 0x4B400000, sa - big, fa - big);
+  typename std::remove_const<decltype(reader)>::type::Raw t[2][NC];
 #pragma unroll
   for (int r = 0; r < 2; ++r)
-    if (r < rows) row(mu0 + r);
+#pragma unroll
+    for (int j = 0; j < NC; ++j) t[r][j] = reader.load(r, j, ns >= (float)r && nf >= (float)j);
+  float a = 0.f, da = 0.f;
+  auto add = [&](const auto& u, int r, int j, bool taken, float ww) {
+    const float L = __saturatef(g.c - fabsf(ww));
+    if (reader.mine(u, r, j, taken)) {
+      a = fmaf(reader.value(u), L, a);
+      da += L;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float wr = r ? w + g.ws : w;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) add(t[r][j], r, j, ns >= (float)r && nf >= (float)j, j ? fmaf((float)j, g.wf, wr) : wr);
+    if (nf >= (float)NC && ns >= (float)r)
 #pragma unroll 1
-  for (int r = 2; r < rows; ++r) row(mu0 + r);
+      for (int j = NC; (float)j <= nf; ++j) add(reader.load(r, j, true), r, j, true, fmaf((float)j, g.wf, wr));
+  }
+#pragma unroll 1
+  for (int r = 2; (float)r <= ns; ++r)
+#pragma unroll 1
+    for (int j = 0; (float)j <= nf; ++j)
+      add(reader.load(r, j, true), r, j, true, fmaf((float)j, g.wf, fmaf((float)r, g.ws, w)));
   acc = a;
   dacc = da;
 }
 
+// Samples (value, voxel row of the sample's ray as int bits): one counts for
+// the voxel's row when the rows are the same (RowGeom).
+struct RowSamples {
+  typedef float2 Raw;
+  const float2* __restrict__ p;
+  int pitch, yrow;
+  __device__ __forceinline__ Raw load(int r, int j, bool take) const {
+    float2 t = make_float2(0.f, __int_as_float(-1));
+    asm("{.reg .pred q; setp.ne.u32 q, %3, 0; @q ld.global.nc.v2.f32 {%0, %1}, [%2];}"
+        : "+f"(t.x), "+f"(t.y)
+        : "l"(p + (long)r * pitch + j), "r"((unsigned)take));
+    return t;
+  }
+  __device__ __forceinline__ bool mine(const Raw& t, int, int, bool) const { return __float_as_int(t.y) == yrow; }
+  __device__ __forceinline__ float value(const Raw& t) const { return t.x; }
+};
+
+// The 4 voxels of a thread on pre-sampled images: `lanes` (a power of two,
+// at most 32) neighbouring threads of a warp cover 4 x lanes consecutive
+// voxels of row (y, z) from x0, thread `lane` the voxels x0 + lane + lanes i.
+// Per quad of 4 voxels the CTF slab (slabs boundaries `bound`, count 0: none)
+// comes from its first corner's depth; thread `lane` forms it for quad `lane`
+// and the quad's voxels take it from there. Where the macro-cell rectangle
+// clips samples (AxisGeom::clips) it comes the same way; elsewhere it leaves
+// out no sample with a chord but those beyond the image. upd(i, value) adds
+// the update acc / dacc of voxel i where there is one. All threads of the
+// warp call it; active: the thread's row exists.
+template <int NC, class Update>
+__device__ __forceinline__ void up_voxels(const KConst& k, const AxisGeom& ag, const UpGeom& g, const float* bound,
+                                          int nslab, float distMin, float distMax, const float2* __restrict__ up,
+                                          size_t up_stride, int pw, int ph, int os, int x0, int lane, int lanes,
+                                          int y, int z, bool active, const Update& upd) {
+  const int nx4 = 4 * k.dimXQuarter;
+  const int xq = x0 + 4 * lane;
+  int slab = 0, r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+  if (active && xq < nx4) {
+    const float depth = macro_depth(k, xq, y, z);
+    if (nslab > 0) {
+      slab = -1;
+      if (depth >= bound[0] && depth < bound[nslab]) {
+        slab = 0;
+        while (slab + 1 < nslab && depth >= bound[slab + 1]) ++slab;
+      }
+    } else if (!(depth >= distMin && depth < distMax)) {
+      slab = -1;
+    }
+    if (ag.clips) {
+      float d;
+      macro_footprint(k, xq, y, z, pw, ph, d, r0, r1, r2, r3);
+    }
+  }
+  // the grid position of voxel x0, split into a sample and a remainder
+  const double ds = g.s0 + x0 * g.sx + y * g.sy + z * g.sz, df = g.f0 + x0 * g.fx + y * g.fy + z * g.fz;
+  const double is = floor(ds), jf = floor(df);
+  const float s0 = (float)(ds - is), f0 = (float)(df - jf);
+  const int ii = (int)is, jj = (int)jf;
+  const float2* at = up + ((long)ii * g.pitch + jj);
+  const float slo = (float)-ii, shi = (float)(g.smax - ii), flo = (float)-jj, fhi = (float)(g.fmax - jj);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int off = lane + lanes * i, quad = off >> 2;  // voxel and quad relative to x0
+    float a0 = slo, a1 = shi, b0 = flo, b1 = fhi;
+    int sl = 0;
+    sl = __shfl_sync(0xffffffffu, slab, quad, lanes);
+    if (ag.clips) {  // uniform
+      const int q0 = __shfl_sync(0xffffffffu, r0, quad, lanes) * os, q1 = __shfl_sync(0xffffffffu, r1, quad, lanes) * os - 1;
+      const int q2 = __shfl_sync(0xffffffffu, r2, quad, lanes) * os, q3 = __shfl_sync(0xffffffffu, r3, quad, lanes) * os - 1;
+      a0 = (float)((g.swapped ? q2 : q0) - ii);
+      a1 = (float)((g.swapped ? q3 : q1) - ii);
+      b0 = (float)((g.swapped ? q0 : q2) - jj);
+      b1 = (float)((g.swapped ? q1 : q3) - jj);
+    }
+    const bool on = active && x0 + off < nx4 && sl >= 0;
+    const float fx = (float)off;
+    float acc, dacc;
+    const float2* slab_at = at + (size_t)max(sl, 0) * up_stride;
+    grid_sums<NC>(g, fmaf(fx, g.dsx, s0), fmaf(fx, g.dfx, f0), a0, a1, b0, b1, on,
+                  [&](int is, int js, float, float) {
+                    return RowSamples{slab_at + (is * g.pitch + js), g.pitch, y};
+                  },
+                  acc, dacc);
+    if (dacc > 0.f) upd(i, acc, dacc);
+  }
+}
 
 // axis_sums for oversampling 2 with bilinear reads of an image whose samples
 // all lie in its interior (texel (ix, iy) at img + ix * sx + iy * sy). The
