@@ -1802,10 +1802,10 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
       const size_t pair = (size_t)p * np + index_list[ii];
       consts[i] = rec_const(r, pair_geoms[pair], sub_geoms[p], 1);
       act[i] = active ? (active[pair] != 0) : 1;
-    });
+    }, 512);
     if (subvol_batchable(n_particles, boxes, consts.data(), proj_count)) {
-      ESB_CK(subvol_batch_build(r->batch, n_particles, boxes, consts.data(), act.data(), proj_count, cf.oversampling,
-                                r->stream), "esb_subvolume_wbp");
+      ESB_CK(subvol_batch_build(r->batch, n_particles, boxes, consts.data(), act.data(), proj_count, W, H,
+                                cf.oversampling, r->stream), "esb_subvolume_wbp");
       if (!cf.ctf_mode) {
         // all projections of the list resident (transposed), a chunk of up
         // to 4 GiB of images per persistent launch
@@ -1824,26 +1824,28 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
         }
         return ok();
       }
+      std::vector<SlabTable> Ts(proj_count);
+      for (int ii = 0; ii < proj_count; ++ii)
+        if ((rc = rec_slab_table(r, full_vol, index_list[ii], Ts[ii]))) return rc;
+      bool planned = false;
       if (r->subvol_patches) {
         // every tilt's slab images filtered and the patches its pairs read
-        // gathered (up to 16 GiB), then all tilts in one persistent launch
-        std::vector<SlabTable> Ts(proj_count);
-        for (int ii = 0; ii < proj_count; ++ii)
-          if ((rc = rec_slab_table(r, full_vol, index_list[ii], Ts[ii]))) return rc;
-        bool planned = false;
-        ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, (size_t)16 << 30, r->stream, planned),
-               "esb_subvolume_wbp");
+        // evaluated (up to 16 GiB), then all tilts in one persistent launch
+        ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, true, (size_t)16 << 30, r->stream,
+                                 planned), "esb_subvolume_wbp");
         if (planned) {
           for (int ii = 0; ii < proj_count; ++ii) {
             const int index = index_list[ii];
             SlabTable T;
             if ((rc = rec_subvol_slab_images(r, full_vol, projections + (size_t)index * img, index, T))) return rc;
             PhaseScope ps(r, 3);
-            ESB_CK(subvol_patch_gather(r->batch, ii, r->slab_imgs, img, W, H, r->stream), "esb_subvolume_wbp");
+            ESB_CK(subvol_patch_sample(r->batch, ii, 0, n_particles, r->slab_imgs, img, W, H, cf.oversampling,
+                                       r->stream), "esb_subvolume_wbp");
           }
           {
             PhaseScope ps(r, 1);
-            ESB_CK(subvol_patch_launch(r->batch, W, H, cf.oversampling, 1, r->stream), "esb_subvolume_wbp");
+            ESB_CK(subvol_patch_launch(r->batch, 0, proj_count, 0, n_particles, W, H, cf.oversampling, r->stream),
+                   "esb_subvolume_wbp");
           }
           unsigned long long misses = 0;
           ESB_CK(subvol_patch_misses(r->batch, r->stream, misses), "esb_subvolume_wbp");
@@ -1852,6 +1854,30 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
                                                  " quad samples fell outside the planned CTF patches");
           return ok();
         }
+      }
+      // one tilt's patches (up to 4 GiB, else its particles in chunks), one
+      // launch per tilt
+      ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, false, (size_t)4 << 30, r->stream, planned),
+             "esb_subvolume_wbp");
+      if (planned) {
+        size_t c = 0;
+        for (int ii = 0; ii < proj_count; ++ii) {
+          const int index = index_list[ii];
+          SlabTable T;
+          if ((rc = rec_subvol_slab_images(r, full_vol, projections + (size_t)index * img, index, T))) return rc;
+          for (; c < r->batch.chunks.size() && r->batch.chunks[c].t == ii; ++c) {
+            const SubvolBatch::Chunk& ch = r->batch.chunks[c];
+            {
+              PhaseScope ps(r, 3);
+              ESB_CK(subvol_patch_sample(r->batch, ii, ch.p0, ch.p1, r->slab_imgs, img, W, H, cf.oversampling,
+                                         r->stream), "esb_subvolume_wbp");
+            }
+            PhaseScope ps(r, 1);
+            ESB_CK(subvol_patch_launch(r->batch, ii, 1, ch.p0, ch.p1, W, H, cf.oversampling, r->stream),
+                   "esb_subvolume_wbp");
+          }
+        }
+        return ok();
       }
       for (int ii = 0; ii < proj_count; ++ii) {
         const int index = index_list[ii];

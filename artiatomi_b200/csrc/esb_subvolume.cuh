@@ -50,10 +50,17 @@ struct SubvolBatch {
   // images that the box's quads read, gathered into one buffer
   void* pdev = nullptr;  // patch table, slab tables, miss counter
   size_t pcap = 0;
-  std::vector<unsigned char> phost;
+  unsigned char* phost = nullptr;  // pinned staging copy of them
+  size_t phost_cap = 0;
+  cudaEvent_t pcopied = nullptr;
   size_t off_slabs = 0, off_miss = 0;
   float* patches = nullptr;
-  size_t patches_cap = 0;  // floats
+  size_t patches_cap = 0;  // bytes
+  struct Chunk {
+    int t, p0, p1;  // list position, particles [p0, p1)
+  };
+  std::vector<Chunk> chunks;     // of a plan per list position
+  std::vector<int> first_work;   // first work item of every particle, and their number
 };
 
 // True when every box can be updated with aligned float4 accesses (x extent a
@@ -63,7 +70,7 @@ bool subvol_batchable(int n_particles, float* const* boxes, const KConst* consts
 // consts/active: [n_particles][n_list] for the list positions of one call;
 // active may be NULL (all pairs active).
 cudaError_t subvol_batch_build(SubvolBatch& b, int n_particles, float* const* boxes, const KConst* consts,
-                               const unsigned char* active, int n_list, int os, cudaStream_t st);
+                               const unsigned char* active, int n_list, int pw, int ph, int os, cudaStream_t st);
 
 // Adds list positions [t0, t0 + nt) to every box. Without slabs
 // (slabs.count == 0) position t reads image imgs + (t - t0) * img_stride;
@@ -75,19 +82,23 @@ cudaError_t subvol_batch_launch(const SubvolBatch& b, int t0, int nt, const floa
 // With CTF: plans, for every (particle, list position) pair, the patch of
 // the position's slab images (slabs[t], images transposed, pw x ph) that the
 // particle's quads read: the slabs its depth range meets, and the detector
-// rectangle of its box's shadow with a margin, out-of-image texels held as
-// their clamped values. ok is false (nothing planned) when some pair does
-// not take the single-axis sums or the patches exceed max_bytes.
-cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, int ph, size_t max_bytes,
-                              cudaStream_t st, bool& ok);
+// rectangle of its box's shadow with a margin, at every sub-pixel grid point.
+// all_tilts: the patches of all positions in one buffer; else a buffer for
+// one position, its particles in chunks (b.chunks) that fit max_bytes. ok is
+// false (nothing planned) when some pair does not take the single-axis sums
+// or, with all_tilts, the patches exceed max_bytes.
+cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, int ph, int os, bool all_tilts,
+                              size_t max_bytes, cudaStream_t st, bool& ok);
 
-// Copies list position t's patches out of its slab images.
-cudaError_t subvol_patch_gather(const SubvolBatch& b, int t, const float* imgs, size_t img_stride, int pw, int ph,
+// Evaluates list position t's slab images at the patches of particles
+// [p0, p1).
+cudaError_t subvol_patch_sample(const SubvolBatch& b, int t, int p0, int p1, const float* imgs, size_t img_stride,
+                                int pw, int ph, int os, cudaStream_t st);
+
+// Adds list positions [t0, t0 + nt) to the boxes of particles [p0, p1) in one
+// persistent launch, reading the patches.
+cudaError_t subvol_patch_launch(const SubvolBatch& b, int t0, int nt, int p0, int p1, int pw, int ph, int os,
                                 cudaStream_t st);
-
-// Adds every list position to every box in one persistent launch, reading
-// the patches.
-cudaError_t subvol_patch_launch(const SubvolBatch& b, int pw, int ph, int os, int linear, cudaStream_t st);
 
 // Number of (quad, position) pairs whose samples the plan did not cover
 // (skipped, so nothing was read outside the patches); synchronises.

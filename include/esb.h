@@ -384,13 +384,14 @@ int esb_reconstructor_enable_graphs(esb_reconstructor* rec, int enable);
  * projection; other subsets are back-projected one projection at a time. */
 int esb_reconstructor_fuse_subsets(esb_reconstructor* rec, int enable);
 
-/* esb_subvolume_wbp with CTF, batched: on, after each tilt's CTF chain the
- * parts of its slab images that each particle's box reads are gathered into
- * one patch buffer (up to 16 GiB), and one persistent launch adds every tilt
- * to every box, each box read and written once. Off (the default): one
- * launch per tilt over all boxes, which is as fast (the back-projection is
- * bound by instruction issue, not by box traffic). Both give the same boxes
- * bit for bit. */
+/* esb_subvolume_wbp with CTF, batched: after each tilt's CTF chain the parts
+ * of its slab images that each particle's box reads are evaluated on the
+ * sub-pixel grid into a patch buffer. On: the patches of all tilts in one
+ * buffer (up to 16 GiB, else as off) and one persistent launch that adds
+ * every tilt to every box, each box read and written once. Off (the
+ * default): one tilt's patches at a time and one launch per tilt over all
+ * boxes, which is as fast (the back-projection is bound by instruction issue,
+ * not by box traffic). Both give the same boxes bit for bit. */
 int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable);
 
 /* ResetProjectionsDevice (Reconstructor.cpp:1678-1682). */
