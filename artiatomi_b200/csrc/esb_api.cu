@@ -27,7 +27,8 @@ cudaError_t launch_march(const KConst& c, const void* vol, int vt, float* proj, 
                          int y0, int x1, int y1, cudaStream_t st);
 cudaError_t launch_slicer(const KConst& c, const void* vol, int vt, float* proj, size_t pitchE, float tmin, float tmax,
                           int x0, int y0, int x1, int y1, cudaStream_t st);
-cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, int y0, int x1, int y1, cudaStream_t st);
+cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, int y0, int x1, int y1, cudaStream_t st,
+                           int set = 0);
 cudaError_t launch_bp(const KConst& c, void* vol, int vt, const float* img, int pw, int ph, size_t pitchE, float lambda,
                       int os, float distMin, float distMax, int linear, cudaStream_t st);
 cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mode, float* proj, float* dist,
@@ -47,9 +48,13 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
                                size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
                                const BpShape* shape, cudaStream_t st);
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
-                                size_t pitchE, const SlabTable& slabs, int x0, int y0, int x1, int y1, cudaStream_t st, int nw = 4);
+                                size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1, int y1,
+                                cudaStream_t st, int nw = 4);
 cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, float* virt, const float* dist,
-                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st);
+                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st,
+                           float* copy = nullptr);
+cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, float2 cut, float2 dim, const int* p,
+                                 int os, float2* up, cudaStream_t st);
 cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2 cut, float2 dim, const int* p,
                                cudaStream_t st);
 cudaError_t launch_make_square(int pw, int ph, size_t strideE, const float* in, int maxsize, float* out, int bx, int by,
@@ -697,8 +702,7 @@ int esb_rec_reset_projections(esb_reconstructor* r) {
   if (!r) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_rec_reset_projections: NULL reconstructor");
   PhaseScope ps(r, 3);
   const size_t img = (size_t)r->cfg.proj_x * r->cfg.proj_y * sizeof(float);
-  ESB_CK(cudaMemsetAsync(r->proj_d, 0, img, r->stream), "esb_rec_reset_projections");
-  ESB_CK(cudaMemsetAsync(r->dist_d, 0, img, r->stream), "esb_rec_reset_projections");
+  ESB_CK(cudaMemsetAsync(r->proj_d, 0, 2 * img, r->stream), "esb_rec_reset_projections");  // with dist_d
   return ok();
 }
 
@@ -854,7 +858,7 @@ static int rec_slicer_nw(esb_reconstructor* r, const KConst& c, const void* vol,
                          const SlabTable& T) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y;
   const int i = rec_tuned(r, tune_key(r, 0, vt, c, 1), 3, 0, [&](int k) {
-    return launch_slicer_fused(c, vol, vt, r->slab_imgs, img, W, T, 0, 0, W, H, r->stream, kNw[k]);
+    return launch_slicer_fused(c, vol, vt, r->slab_imgs, img, W, T, 1, 0, 0, W, H, r->stream, kNw[k]);
   });
   return kNw[i];
 }
@@ -1097,12 +1101,12 @@ static int rec_subvol_slab_images(esb_reconstructor* r, const esb_vol_geom* full
   return ESB_OK;
 }
 
-// Pre-samples `count` transposed slab images for the back-projection
-// (launch_upsample); returns NULL when the geometry does not allow it
-// (oversampling not a power of two, magnification anisotropy) or the
-// images would exceed 8 GiB, and the back-projection then filters the slab
-// images itself. `up_stride` receives the (value, row) pairs per image.
-static const float2* rec_upsample(esb_reconstructor* r, const KConst& c, int count, int linear, size_t& up_stride) {
+// The buffer of `count` pre-sampled images (launch_upsample,
+// launch_crop_upsample); NULL when the geometry does not allow them
+// (oversampling not a power of two, magnification anisotropy) or they would
+// exceed 8 GiB, and the back-projection then filters the slab images itself.
+// `up_stride` receives the (value, row) pairs per image.
+static float2* rec_up_images(esb_reconstructor* r, const KConst& c, int count, size_t& up_stride) {
   const esb_recon_config& cf = r->cfg;
   const int os = cf.oversampling;
   up_stride = (size_t)cf.proj_x * os * (size_t)cf.proj_y * os;
@@ -1119,10 +1123,6 @@ static const float2* rec_upsample(esb_reconstructor* r, const KConst& c, int cou
     }
     r->up_cap = need;
   }
-  const size_t img = (size_t)cf.proj_x * cf.proj_y;
-  if (launch_upsample(c, r->slab_imgs, img, count, cf.proj_x, cf.proj_y, os, linear, r->up_imgs, up_stride,
-                      r->stream) != cudaSuccess)
-    return nullptr;
   return r->up_imgs;
 }
 
@@ -1145,6 +1145,7 @@ static int rec_forward(esb_reconstructor* r, const esb_vol_geom* vg, const void*
     roi[3] = std::min(roi_in[3], H);
     if (roi[2] <= roi[0] || roi[3] <= roi[1]) return ok();  // no ray in the region
   }
+  const bool whole = roi[0] == 0 && roi[1] == 0 && roi[2] == W && roi[3] == H;
   KConst c = rec_const(r, r->geoms[index], *vg, 0);
   if (volume_is_empty) {  // Reconstructor.cpp:465-470 / 622-627
     PhaseScope ps(r, 0);
@@ -1167,16 +1168,16 @@ static int rec_forward(esb_reconstructor* r, const esb_vol_geom* vg, const void*
     if ((rc = rec_slab_table(r, vg, index, T))) return rc;
     if ((rc = rec_slab_capacity(r, T.count))) return rc;
     const size_t img = (size_t)W * H;
-    {
+    const int nw = rec_slicer_nw(r, c, vol, voxel_type, img, T);  // (its trials write whole slab images)
+    if (!whole) {
       PhaseScope ps(r, 3);
       ESB_CK(cudaMemsetAsync(r->slab_imgs, 0, (size_t)T.count * img * sizeof(float), r->stream),
              where);
     }
     {
       PhaseScope ps(r, 0);
-      const int nw = rec_slicer_nw(r, c, vol, voxel_type, img, T);
-      ESB_CK(launch_slicer_fused(c, vol, voxel_type, r->slab_imgs, img, W, T, roi[0], roi[1], roi[2], roi[3],
-                                 r->stream, nw),
+      ESB_CK(launch_slicer_fused(c, vol, voxel_type, r->slab_imgs, img, W, T, whole ? 1 : 0, roi[0], roi[1], roi[2],
+                                 roi[3], r->stream, nw),
              where);
     }
     // each slab image through the CTF, added to proj_d in slab order
@@ -1197,12 +1198,12 @@ static int rec_forward(esb_reconstructor* r, const esb_vol_geom* vg, const void*
     }
     if ((rc = rec_ctf_chain(r, r->dist_d, 1, full, index, dmin, dmax, 1, nullptr, r->proj_d, 1, full))) return rc;
   }
-  {
+  if (!whole) {
     PhaseScope ps(r, 3);
     ESB_CK(cudaMemsetAsync(r->dist_d, 0, (size_t)W * H * sizeof(float), r->stream), where);
   }
   PhaseScope ps(r, 0);
-  ESB_CK(launch_travlen(c, r->dist_d, W, roi[0], roi[1], roi[2], roi[3], r->stream), where);
+  ESB_CK(launch_travlen(c, r->dist_d, W, roi[0], roi[1], roi[2], roi[3], r->stream, whole ? 1 : 0), where);
   return ok();
 }
 
@@ -1219,7 +1220,10 @@ int esb_rec_forward_projection_roi(esb_reconstructor* r, const esb_vol_geom* vg,
   return rec_forward(r, vg, vol, voxel_type, index, volume_is_empty, roi, "esb_rec_forward_projection_roi");
 }
 
-int esb_rec_compare(esb_reconstructor* r, const esb_vol_geom* vg, const float* real, int index) {
+}  // extern "C"
+
+// esb_rec_compare, with the residual also stored to `copy` (NULL: not).
+static int rec_compare(esb_reconstructor* r, const esb_vol_geom* vg, const float* real, int index, float* copy) {
   int rc;
   if ((rc = rec_check(r, vg, index, "esb_rec_compare"))) return rc;
   if (!real) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_rec_compare: real is NULL");
@@ -1233,11 +1237,13 @@ int esb_rec_compare(esb_reconstructor* r, const esb_vol_geom* vg, const float* r
   ESB_CK(launch_compare(cf.proj_x, cf.proj_y, cf.proj_x, real, r->proj_d, r->dist_d, len,
                         make_float4(cf.crop[0], cf.crop[1], cf.crop[2], cf.crop[3]),
                         make_float4(cf.crop_dim[0], cf.crop_dim[1], cf.crop_dim[2], cf.crop_dim[3]),
-                        cf.projection_scale_factor, r->stream), "esb_rec_compare");
+                        cf.projection_scale_factor, r->stream, copy), "esb_rec_compare");
   return ok();
 }
 
-}  // extern "C"
+extern "C" int esb_rec_compare(esb_reconstructor* r, const esb_vol_geom* vg, const float* real, int index) {
+  return rec_compare(r, vg, real, index, nullptr);
+}
 
 // BackProjection of image `img` (Reconstructor.cpp:871-887 and 920-969).
 static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, void* vol, int voxel_type, int index,
@@ -1249,24 +1255,29 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
   KConst c = rec_const(r, r->geoms[index], *vg, 1);
   const float lambda = cf.lambda / sirt_count;
   if (!cf.ctf_mode) {
+    const float2 cut = make_float2(cf.cut_length[0], cf.cut_length[1]);
+    const float2 dim = make_float2(cf.dim_length[0], cf.dim_length[1]);
+    size_t up_stride = 0;
+    float2* up = cf.variant == ESB_VARIANT_FAST ? rec_up_images(r, c, 1, up_stride) : nullptr;
+    ESB_CK(cudaGetLastError(), "back projection");
     {
       PhaseScope ps(r, 3);
-      ESB_CK(launch_crop_border(W, H, W, img, make_float2(cf.cut_length[0], cf.cut_length[1]),
-                                make_float2(cf.dim_length[0], cf.dim_length[1]), p, r->stream), "back projection");
+      if (up) {
+        ESB_CK(launch_crop_upsample(c, W, H, img, cut, dim, p, cf.oversampling, up, r->stream), "back projection");
+      } else {
+        ESB_CK(launch_crop_border(W, H, W, img, cut, dim, p, r->stream), "back projection");
+      }
     }
     if (cf.variant == ESB_VARIANT_FAST) {
-      int rc2;
-      if ((rc2 = rec_slab_capacity(r, 1))) return rc2;
-      {
+      if (!up) {
+        int rc2;
+        if ((rc2 = rec_slab_capacity(r, 1))) return rc2;
         PhaseScope ps(r, 3);
         ESB_CK(launch_transpose(img, W, H, W, r->slab_imgs, r->stream), "back projection");
       }
       SlabTable none;
       none.count = 0;
       PhaseScope ps(r, 1);
-      size_t up_stride = 0;
-      const float2* up = rec_upsample(r, c, 1, 0, up_stride);
-      ESB_CK(cudaGetLastError(), "back projection");
       const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, 0, none, 0, up, up_stride);
       ESB_CK(launch_bp_fast_slabs(c, vol, voxel_type, r->slab_imgs, 0, none, W, H, W, lambda, cf.oversampling, 0.0f,
                                   9999999999999.0f, 0, r->stream, 1, up, up_stride, &shape), "back projection");
@@ -1290,8 +1301,11 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
     if ((rc = rec_ctf_chain_slabs(r, T, index, img, 1, 1, p, 0, r->slab_imgs, nullptr, 1, p, 1))) return rc;
     PhaseScope ps(r, 1);
     size_t up_stride = 0;
-    const float2* up = rec_upsample(r, c, T.count, 1, up_stride);
+    float2* up = rec_up_images(r, c, T.count, up_stride);
     ESB_CK(cudaGetLastError(), "back projection");
+    if (up)
+      ESB_CK(launch_upsample(c, r->slab_imgs, (size_t)W * H, T.count, W, H, cf.oversampling, 1, up, up_stride,
+                             r->stream), "back projection");
     const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, (size_t)W * H, T, 1, up, up_stride);
     ESB_CK(launch_bp_fast_slabs(c, vol, voxel_type, r->slab_imgs, (size_t)W * H, T, W, H, W, lambda, cf.oversampling,
                                 0.f, 0.f, 1, r->stream, 1, up, up_stride, &shape), "back projection");
@@ -1376,13 +1390,9 @@ static int rec_back_project_subset(esb_reconstructor* r, const esb_vol_geom* vg,
         ESB_CK(launch_upsample(ks[j], r->slab_imgs, img, T[j].count, W, H, os, 1, up, up_stride, r->stream),
                "subset back projection");
       } else {
-        if ((rc = rec_slab_capacity(r, 1))) return rc;
         PhaseScope ps(r, 3);
-        ESB_CK(launch_crop_border(W, H, W, imgs[j], make_float2(cf.cut_length[0], cf.cut_length[1]),
-                                  make_float2(cf.dim_length[0], cf.dim_length[1]), p, r->stream),
-               "subset back projection");
-        ESB_CK(launch_transpose(imgs[j], W, H, W, r->slab_imgs, r->stream), "subset back projection");
-        ESB_CK(launch_upsample(ks[j], r->slab_imgs, img, 1, W, H, os, 0, up, up_stride, r->stream),
+        ESB_CK(launch_crop_upsample(ks[j], W, H, imgs[j], make_float2(cf.cut_length[0], cf.cut_length[1]),
+                                    make_float2(cf.dim_length[0], cf.dim_length[1]), p, os, up, r->stream),
                "subset back projection");
       }
       ups[j - ch.first] = up;
@@ -1426,9 +1436,7 @@ static int sart_iteration(esb_reconstructor* r, const esb_vol_geom* vg, void* vo
       const int index = index_list[s * sirt_count + i];
       if ((rc = esb_rec_reset_projections(r))) return rc;
       if ((rc = esb_rec_forward_projection(r, vg, vol, voxel_type, index, *volume_is_empty))) return rc;
-      if ((rc = esb_rec_compare(r, vg, projections + (size_t)index * img, index))) return rc;
-      ESB_CK(cudaMemcpyAsync(r->sirt_d[i], r->proj_d, img * sizeof(float), cudaMemcpyDeviceToDevice, r->stream),
-             "esb_sart_run");
+      if ((rc = rec_compare(r, vg, projections + (size_t)index * img, index, r->sirt_d[i]))) return rc;
     }
     const int in_subset = std::min(sirt_count, proj_count - s * sirt_count);
     bool fused = false;
@@ -1760,9 +1768,7 @@ int esb_sart_run_zslab(esb_reconstructor* r, const esb_vol_geom* vg, void* vol, 
         // the sums on every rank each forms the same residual itself)
         if ((rc = allreduce(r->proj_d, 2 * img, (void*)r->stream, user)))
           return fail(ESB_ERR_CUDA, std::string(where) + ": the all-reduce callback returned " + std::to_string(rc));
-        if ((rc = esb_rec_compare(r, vg, projections + (size_t)index * img, index))) return rc;
-        ESB_CK(cudaMemcpyAsync(r->sirt_d[i], r->proj_d, img * sizeof(float), cudaMemcpyDeviceToDevice, r->stream),
-               where);
+        if ((rc = rec_compare(r, vg, projections + (size_t)index * img, index, r->sirt_d[i]))) return rc;
       }
       const int in_subset = std::min(sirt_count, proj_count - s * sirt_count);
       bool fused = false;

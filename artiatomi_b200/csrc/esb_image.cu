@@ -5,7 +5,7 @@
 // storage conversions.
 #include <math.h>
 
-#include "esb_device.cuh"
+#include "esb_bp_core.cuh"
 
 namespace esb {
 
@@ -18,7 +18,8 @@ __device__ __forceinline__ float taper(float w) {
 // reference evaluate to w = (-y - cut)/dim <= 0, i.e. a hard zero band of
 // width dim+cut; the expressions are kept as written.
 __global__ void k_compare(int pw, int ph, size_t pitchE, const float* __restrict__ real, float* __restrict__ virt,
-                          const float* __restrict__ dist, float realLength, float4 cut, float4 dim, float scale) {
+                          const float* __restrict__ dist, float realLength, float4 cut, float4 dim, float scale,
+                          float* __restrict__ copy) {
   const unsigned x = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= (unsigned)pw || y >= (unsigned)ph) return;
@@ -33,7 +34,9 @@ __global__ void k_compare(int pw, int ph, size_t pitchE, const float* __restrict
   if (fy > (float)ph - dim.w - cut.w - 1.0f) ya = taper(((float)((unsigned)ph - y - 1u) - cut.w - (float)(ph - 1)) / dim.w);
   if (fx < cut.y + dim.y) xb = taper((fx - cut.y) / dim.y);
   if (fx > (float)pw - dim.x - cut.x - 1.0f) xa = taper(((float)((unsigned)pw - x - 1u) - cut.x - (float)(pw - 1)) / dim.x);
-  virt[i] = xa * xb * ya * yb * error;
+  const float r = xa * xb * ya * yb * error;
+  virt[i] = r;
+  if (copy) copy[i] = r;  // the residual kept for the subset's back-projection
 }
 
 __device__ __forceinline__ float seg_dist(int2 v, int2 w, int x, int y) {  // Compare.cu:137-163
@@ -245,6 +248,40 @@ __global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t p
 
 
 
+// The back-projection's image passes without CTF in one: cropBorder in place
+// (k_crop_border), the transposition and the pre-sampling by nearest texel of
+// k_upsample, with the voxel row of every grid point's ray. Tiles of 32 x 32
+// pixels: rows are read along x, grid points written along the fast axis of
+// the pre-sampled image (UpGeom). Detectors too small to fill the GPU with
+// those take tiles of 16 x 16, one pixel per thread.
+template <int TILE>
+__global__ void __launch_bounds__(256) k_crop_upsample(int pw, int ph, float* __restrict__ img, float2 cut, float2 dim,
+                                                       int2 p1, int2 p2, int2 p3, int2 p4, int os, bpcore::RowGeom rg,
+                                                       int swapped, float2* __restrict__ up) {
+  __shared__ float tile[TILE][TILE + 1];
+  const int bx = blockIdx.x * TILE, by = blockIdx.y * TILE;
+  for (int j = threadIdx.y; j < TILE; j += blockDim.y) {
+    const int x = bx + threadIdx.x, y = by + j;
+    if (x < pw && y < ph) {
+      const size_t i = (size_t)y * pw + x;
+      const float v = crop_factor(pw, ph, x, y, cut, dim, p1, p2, p3, p4) * img[i];
+      img[i] = v;
+      tile[j][threadIdx.x] = v;
+    }
+  }
+  __syncthreads();
+  const int n = TILE * os, nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
+  const int f0 = (swapped ? bx : by) * os, s0 = (swapped ? by : bx) * os;
+  for (int s = threadIdx.y; s < n; s += blockDim.y) {
+    for (int f = threadIdx.x; f < n; f += TILE) {
+      if (f0 + f >= nf || s0 + s >= ns) continue;
+      const int mu = swapped ? f0 + f : s0 + s, mv = swapped ? s0 + s : f0 + f;
+      const float v = swapped ? tile[s / os][f / os] : tile[f / os][s / os];
+      up[(size_t)(s0 + s) * nf + f0 + f] = make_float2(v, __int_as_float(bpcore::sample_row(rg, mu, mv)));
+    }
+  }
+}
+
 // Kernel `wbpWeighting` (wbpWeighting.cu:50-144).
 __global__ void k_wbp_weighting(float2* __restrict__ spec, int n, float s, float co, int fm) {
   const unsigned x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,9 +454,9 @@ __global__ void k_normalize(const float* __restrict__ in, float* __restrict__ ou
 static inline dim3 grid2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y - 1) / b.y); }
 
 cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, float* virt, const float* dist,
-                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st) {
+                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st, float* copy) {
   dim3 b(32, 8);
-  k_compare<<<grid2(pw, ph, b), b, 0, st>>>(pw, ph, pitchE, real, virt, dist, realLength, cut, dim, scale); ESB_COUNT_LAUNCH();
+  k_compare<<<grid2(pw, ph, b), b, 0, st>>>(pw, ph, pitchE, real, virt, dist, realLength, cut, dim, scale, copy); ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
@@ -428,6 +465,21 @@ cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2
   dim3 b(32, 8);
   k_crop_border<<<grid2(pw, ph, b), b, 0, st>>>(pw, ph, pitchE, img, cut, dim, make_int2(p[0], p[1]),
                                                  make_int2(p[2], p[3]), make_int2(p[4], p[5]), make_int2(p[6], p[7])); ESB_COUNT_LAUNCH();
+  return cudaGetLastError();
+}
+
+// k_crop_upsample of one projection (row-major, dense); k gives the rows.
+cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, float2 cut, float2 dim, const int* p,
+                                 int os, float2* up, cudaStream_t st) {
+  const bpcore::BpGeom g = bpcore::make_geom(k, os);
+  const int swapped = bpcore::axis_eligible(k, g) && bpcore::up_swapped(bpcore::make_axis_geom(k, g, os)) ? 1 : 0;
+  const int tile = (long)((pw + 31) / 32) * ((ph + 31) / 32) >= 296 ? 32 : 16;  // two 32 x 32 tiles per SM
+  const dim3 b(tile, 256 / tile), grd((pw + tile - 1) / tile, (ph + tile - 1) / tile);
+  const auto kernel = tile == 32 ? k_crop_upsample<32> : k_crop_upsample<16>;
+  kernel<<<grd, b, 0, st>>>(pw, ph, img, cut, dim, make_int2(p[0], p[1]), make_int2(p[2], p[3]),
+                            make_int2(p[4], p[5]), make_int2(p[6], p[7]), os, bpcore::make_row_geom(k, os), swapped,
+                            up);
+  ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 

@@ -18,11 +18,12 @@
 namespace esb {
 cudaError_t launch_march(const KConst& c, const void* vol, int vt, float* proj, float* dist, size_t pitchE, int x0,
                          int y0, int x1, int y1, cudaStream_t st);
-cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, int y0, int x1, int y1, cudaStream_t st);
+cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, int y0, int x1, int y1, cudaStream_t st,
+                           int set);
 cudaError_t launch_bp(const KConst& c, void* vol, int vt, const float* img, int pw, int ph, size_t pitchE, float lambda,
                       int os, float distMin, float distMax, int linear, cudaStream_t st);
 cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, float* virt, const float* dist,
-                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st);
+                           float realLength, float4 cut, float4 dim, float scale, cudaStream_t st, float* copy);
 cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2 cut, float2 dim, const int* p,
                                cudaStream_t st);
 cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mode, float* proj, float* dist,
@@ -136,7 +137,7 @@ extern "C" int esb_sart_projection_update_noalloc(const esb_recon_config* cfg, c
   // per block: the reconstructor's launch-shape trials write scratch buffers,
   // and the shape does not change the result)
   if (volume_is_empty)
-    e = launch_travlen(kf, dist, W, 0, 0, W, H, st);
+    e = launch_travlen(kf, dist, W, 0, 0, W, H, st, 0);
   else if (fast)
     e = launch_project_fast(kf, vol, voxel_type, 0, proj, dist, W, 0.f, 0.f, 0, 0, W, H, st, 4);
   else
@@ -148,7 +149,7 @@ extern "C" int esb_sart_projection_update_noalloc(const esb_recon_config* cfg, c
   const float len = fabsf((DIST - vg->full_bbox_min[2]) / zdir - (DIST - vg->full_bbox_max[2]) / zdir);
   e = launch_compare(W, H, W, real, proj, dist, len, make_float4(cfg->crop[0], cfg->crop[1], cfg->crop[2], cfg->crop[3]),
                      make_float4(cfg->crop_dim[0], cfg->crop_dim[1], cfg->crop_dim[2], cfg->crop_dim[3]),
-                     cfg->projection_scale_factor, st);
+                     cfg->projection_scale_factor, st, nullptr);
   if (e != cudaSuccess) return fail(ESB_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
   // Back-projection of the residual (Reconstructor.cpp:871-887)
   e = launch_crop_border(W, H, W, proj, make_float2(cfg->cut_length[0], cfg->cut_length[1]),

@@ -162,8 +162,10 @@ __global__ void __launch_bounds__(256) k_slicer(KConst c, const void* __restrict
 }
 
 // Kernel `volTraversalLength` (ForwardProjectionSlicer.cu:224-288).
+// set: the chord is stored (a whole image that would be cleared first), else
+// added.
 __global__ void __launch_bounds__(256) k_travlen(KConst c, float* __restrict__ dist, size_t pitchE, int x0, int y0,
-                                                 int x1, int y1) {
+                                                 int x1, int y1, int set) {
   const int x = x0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int y = y0 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (x >= x1 || y >= y1) return;
@@ -171,7 +173,8 @@ __global__ void __launch_bounds__(256) k_travlen(KConst c, float* __restrict__ d
   float tin, tout, val = 0.0f;
   box_hit(s, c.n, c.bbMin, c.bbMax, tin, tout);
   if (tout > tin) val = tout - tin;
-  dist[(size_t)y * pitchE + x] += val;
+  float* out = dist + (size_t)y * pitchE + x;
+  *out = set ? val : *out + val;
 }
 
 // One 4-voxel quad of kernel `backProjection` / `backProjectionFP16`
@@ -339,10 +342,10 @@ cudaError_t launch_slicer(const KConst& c, const void* vol, int vt, float* proj,
 }
 
 cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, int y0, int x1, int y1,
-                           cudaStream_t st) {
+                           cudaStream_t st, int set) {
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
   dim3 blk(32, 8), grd((x1 - x0 + 31) / 32, (y1 - y0 + 7) / 8);
-  k_travlen<<<grd, blk, 0, st>>>(c, dist, pitchE, x0, y0, x1, y1); ESB_COUNT_LAUNCH();
+  k_travlen<<<grd, blk, 0, st>>>(c, dist, pitchE, x0, y0, x1, y1, set); ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 

@@ -335,15 +335,23 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_project_fast(KConst c, con
   }
 }
 
+// Zero in the slab images that a pixel's rays do not meet (they meet
+// [klo, khi]).
+__device__ __forceinline__ void clear_slabs(float* img, size_t stride, int count, int klo, int khi) {
+  for (int k = 0; k < count; ++k)
+    if (k < klo || k > khi) img[(size_t)k * stride] = 0.0f;
+}
+
 // All defocus slabs of one projection in one launch: slab k's image gets
 // the slicer's integral over [bound[k], bound[k+1]] (ForwardProjectionSlicer.cu:57-220,
 // called once per slab by Reconstructor.cpp:515-585). The 4 lanes of a pixel
 // walk the union of their slab ranges together so each slab's sum keeps the
-// reference's sub-ray order.
+// reference's sub-ray order. clear: the pixels that no ray of a slab reaches
+// are set to 0 (else the caller clears the images first).
 template <int VT, class Off, int NW>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_slicer_fused(KConst c, const void* __restrict__ vol, float* __restrict__ imgs,
-                                                      size_t img_stride, size_t pitchE, SlabTable slabs, int x0, int y0,
-                                                      int x1, int y1) {
+                                                      size_t img_stride, size_t pitchE, SlabTable slabs, int clear, int x0,
+                                                      int y0, int x1, int y1) {
   const int lane = threadIdx.x & 31;
   const int sub = lane & 3;
   const int row = (threadIdx.x >> 2) & 7;
@@ -392,6 +400,7 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_slicer_fused(KConst c, con
     v = quad_sum_ordered(v);
     if (active && sub == 0 && k >= klo && k <= khi) imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
   }
+  if (clear && active && sub == 0) clear_slabs(imgs + pix, img_stride, slabs.count, klo, khi);
 }
 
 // ---------------------------------------------------------------------------
@@ -706,8 +715,8 @@ __global__ void __launch_bounds__(256, 4) k_project_axis(const __grid_constant__
 template <int VT, bool ZMAJ, int SM, int SN, class Off>
 __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
                                                      const void* __restrict__ vol, float* __restrict__ imgs,
-                                                     size_t img_stride, size_t pitchE, SlabTable slabs, int swap,
-                                                     int x0, int y0, int x1, int y1) {
+                                                     size_t img_stride, size_t pitchE, SlabTable slabs, int clear,
+                                                     int swap, int x0, int y0, int x1, int y1) {
   const AxisPixel P(swap, x0, y0, x1, y1);
   Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
   float3 s = make_float3(0.f, 0.f, 0.f);
@@ -751,6 +760,7 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
     if (P.active && P.sub == 0 && k >= klo && k <= khi)
       imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
   }
+  if (clear && P.active && P.sub == 0) clear_slabs(imgs + pix, img_stride, slabs.count, klo, khi);
 }
 
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.
@@ -795,14 +805,14 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
   } while (0)
 
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
-                                size_t pitchE, const SlabTable& slabs, int x0, int y0, int x1, int y1,
-                                cudaStream_t st, int nw) {
+                                size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1,
+                                int y1, cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0 || slabs.count <= 0) return cudaSuccess;
   if (axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
     const dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    ESB_AXIS_LAUNCH(k_slicer_axis, grd, blk, st, vol, imgs, img_stride, pitchE, slabs, swap, x0, y0, x1, y1);
+    ESB_AXIS_LAUNCH(k_slicer_axis, grd, blk, st, vol, imgs, img_stride, pitchE, slabs, clear, swap, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();
   }
@@ -810,7 +820,7 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
   if (big || (nw != 2 && nw != 8)) nw = 4;
   dim3 blk(32 * nw), grd((x1 - x0 + nw - 1) / nw, (y1 - y0 + 7) / 8);
 #define ESB_LAUNCH(VT, OFF, NW) \
-  k_slicer_fused<VT, OFF, NW><<<grd, blk, 0, st>>>(c, vol, imgs, img_stride, pitchE, slabs, x0, y0, x1, y1)
+  k_slicer_fused<VT, OFF, NW><<<grd, blk, 0, st>>>(c, vol, imgs, img_stride, pitchE, slabs, clear, x0, y0, x1, y1)
 #define ESB_LAUNCH_VT(OFF, NW)                                  \
   do {                                                          \
     if (vt == ESB_VOXEL_F32) ESB_LAUNCH(ESB_VOXEL_F32, OFF, NW);   \
