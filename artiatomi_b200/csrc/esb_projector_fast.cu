@@ -763,6 +763,453 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
   if (clear && P.active && P.sub == 0) clear_slabs(imgs + pix, img_stride, slabs.count, klo, khi);
 }
 
+// ---------------------------------------------------------------------------
+// Series with next to no in-plane rotation: k_project_planes, k_slicer_planes.
+//
+// The rays of a detector row differ in y, and in x-z by the tilt axis'
+// rotation against the detector: half a pixel along u moves a ray by half its
+// sine, 0.0026 voxels at 0.3 degrees. A thread walks one line of 2 G sub-rays
+// (G pixels along u) with the weights of its middle ray (axis_walk's). A
+// layer's weights are bilinear in the ray's offset (e, f) along the minor and
+// major axis as long as the samples stay in their cells, so with the weights'
+// derivatives the sums of every ray of the line follow from the sums over
+// the G + 2 y planes that the rays interpolate between,
+//   S + e Se + f Sf + e f Sef,
+// formed once per line; only the blend of two planes and the offset are a
+// ray's own. A sample that the offset carries across a cell's face (offsets
+// are kept below 1/64 voxel) is evaluated on the face's other side: the
+// interpolant is continuous there, and the difference, a kink times less than
+// 1/64 in one sample of a hundred, is a tenth of what the rounding of the
+// ray's float start point (5e-4 voxels, all samples) makes.
+//
+// Per ray and layer that leaves a 2 G-th of the weights, control and loads
+// of each plane in place of all of them for two planes. A warp holds 16
+// detector rows x 2 sub-rows, so that its loads of a plane are contiguous.
+// `swap` exchanges u and v (a tilt axis across the image).
+struct PlaneWalk {
+  int sM, sN;          // step signs
+  int nM, nN;          // voxels along the major and minor axis
+  unsigned dM, dN;     // their element strides
+};
+constexpr float kMaxShear = 1.0f / 64.0f;
+
+// Plane sums over samples j0 .. J-1 of one ray: S[0] of the weights, and with
+// SH > 0 S[1], S[2] of their derivatives along the mirrored minor and major
+// axis, with SH > 1 S[3] of the mixed one; yoff: element offsets of the
+// planes.
+template <int VT, int NP, int SH>
+__device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W, const void* __restrict__ vol,
+                                           const unsigned (&yoff)[NP], float Mq, float Nq, int j0, int J,
+                                           float (&S)[SH == 0 ? 1 : SH + 2][NP]) {
+  constexpr int NS = SH == 0 ? 1 : SH + 2;
+  typedef typename RawVoxel<VT>::T Raw;
+  constexpr int ES = VT == ESB_VOXEL_F32 ? 4 : 2;
+  const char* const base = (const char*)vol;
+  const float fj0 = (float)j0, jb = fj0 - 0.5f;
+  const float pM = __fmaf_rn(fj0, A.dM, Mq), pN = __fmaf_rn(fj0, A.dN, Nq);
+  const float fm = floorf(pM), fn = floorf(pN);
+  const float nM0 = ((fm + 1.f) - pM) * A.isM;
+  const float nN0 = A.isN > 0.f ? ((fn + 1.f) - pN) * A.isN : FLT_MAX;
+  const float Mt = (float)(J - j0);
+  float relN = __fmaf_rn(jb, A.dN, __fsub_rn(Nq, fn)), relM = __fmaf_rn(jb, A.dM, __fsub_rn(Mq, fm));
+  int im = W.sM * (int)fm, in = W.sN * (int)fn;
+  float k = 0.f, kn = 0.f, fm0 = 0.f;
+  float g[NS][3];  // far weights of the layer before, at n - 1, n, n + 1
+  bool Xp = false;
+  Raw va[NP], vd[NP];  // the outer positions, kept where a layer does not read them (weight 0)
+#pragma unroll
+  for (int p = 0; p < NP; ++p) va[p] = vd[p] = Raw(0);
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    g[q][0] = g[q][1] = g[q][2] = 0.f;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) S[q][p] = 0.f;
+  }
+  auto row = [&](const float (&w)[NS][4], bool first, bool last) {
+    const unsigned r = (unsigned)min(max(im, 0), W.nM - 1) * W.dM;
+    auto col = [&](int n) { return r + (unsigned)min(max(n, 0), W.nN - 1) * W.dN; };
+    const unsigned oa = col(in - W.sN), ob = col(in), oc = col(in + W.sN), od = col(in + 2 * W.sN);
+    Raw vb[NP], vc[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      vb[p] = ldraw<VT>(base + (size_t)ES * (ob + yoff[p]));
+      vc[p] = ldraw<VT>(base + (size_t)ES * (oc + yoff[p]));
+      ldraw_if<VT>(va[p], base + (size_t)ES * (oa + yoff[p]), first);
+      ldraw_if<VT>(vd[p], base + (size_t)ES * (od + yoff[p]), last);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const float a = cvt<VT>(va[p]), b = cvt<VT>(vb[p]), c = cvt<VT>(vc[p]), d = cvt<VT>(vd[p]);
+#pragma unroll
+      for (int q = 0; q < NS; ++q) {
+        S[q][p] = fmaf(b, w[q][1], S[q][p]);
+        S[q][p] = fmaf(c, w[q][2], S[q][p]);
+        S[q][p] = fmaf(a, w[q][0], S[q][p]);
+        S[q][p] = fmaf(d, w[q][3], S[q][p]);
+      }
+    }
+  };
+#pragma unroll 1
+  for (int guard = 0; guard < 1 << 20; ++guard) {
+    const float nMs = __fmaf_rn(k, A.isM, nM0), nNs = __fmaf_rn(kn, A.isN, nN0);
+    const bool X = nNs <= nMs;
+    const float tL = fminf(nMs, Mt);
+    const float2 f = ceil2(fminf(nNs, tL), tL);
+    const float MA = f.x - fm0, MB = f.y - f.x;
+    const float sA = fm0 + f.x, sB = f.x + f.y;
+    const float aA = fmaf(sA, A.hN, relN), aB = fmaf(sB, A.hN, relN - 1.f);
+    const float cA = fmaf(sA, A.hM, relM), cB = fmaf(sB, A.hM, relM);
+    const float MaA = MA * aA, MaB = MB * aB, McA = MA * cA, McB = MB * cB;
+    const float tA = MA * fmaf(aA, cA, fmaf(MA * MA, A.g, -A.g)), tB = MB * fmaf(aB, cB, fmaf(MB * MB, A.g, -A.g));
+    float n[NS][3], far[NS][3];  // near and far weights at n, n + 1, n + 2
+    const float uA = McA - tA, uB = McB - tB;
+    n[0][0] = (MA - MaA) - uA;
+    n[0][1] = (MaA - tA) + ((MB - MaB) - uB);
+    n[0][2] = MaB - tB;
+    far[0][0] = uA;
+    far[0][1] = tA + uB;
+    far[0][2] = tB;
+    if constexpr (SH > 0) {
+      const float vA = MA - McA, vB = MB - McB, wA = MA - MaA, wB = MB - MaB;
+      n[1][0] = -vA, n[1][1] = vA - vB, n[1][2] = vB;
+      far[1][0] = -McA, far[1][1] = McA - McB, far[1][2] = McB;
+      n[2][0] = -wA, n[2][1] = -(MaA + wB), n[2][2] = -MaB;
+      far[2][0] = wA, far[2][1] = MaA + wB, far[2][2] = MaB;
+    }
+    if constexpr (SH > 1) {
+      n[3][0] = MA, n[3][1] = MB - MA, n[3][2] = -MB;
+      far[3][0] = -MA, far[3][1] = MA - MB, far[3][2] = MB;
+    }
+    float w[NS][4];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      w[q][0] = g[q][0];
+      w[q][1] = g[q][1] + n[q][0];
+      w[q][2] = g[q][2] + n[q][1];
+      w[q][3] = n[q][2];
+    }
+    row(w, Xp, X);
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      g[q][0] = X ? far[q][0] : 0.f;
+      g[q][1] = X ? far[q][1] : far[q][0];
+      g[q][2] = X ? far[q][2] : far[q][1];
+    }
+    fm0 = f.y;
+    k += 1.f;
+    relM -= 1.f;
+    im += W.sM;
+    if (X) {
+      relN -= 1.f;
+      kn += 1.f;
+      in += W.sN;
+    }
+    Xp = X;
+    if (fm0 >= Mt) break;
+  }
+  float w[NS][4];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    w[q][0] = g[q][0], w[q][1] = g[q][1], w[q][2] = g[q][2];
+    w[q][3] = 0.f;
+  }
+  row(w, Xp, false);
+}
+
+// One thread's line of 2 G sub-rays (kept in local memory, read a few times
+// per walk).
+template <int G>
+struct PlaneLine {
+  static constexpr int N = 2 * G, NP = G + 2;
+  float3 s[N];           // starts
+  float tin[N], tout[N];
+  float b[N], source[N]; // weight of the upper plane, and the sample at the start
+  int cell[N];           // lower plane, relative to the line's first
+  unsigned in;           // sub-rays that meet the volume
+  // x, y: first pixel; the lane's sub-row along v (u with swap)
+  template <int VT>
+  __device__ __forceinline__ void init(const KConst& c, const void* vol, int x, int y, int swap, bool sources,
+                                       unsigned (&yoff)[NP]) {
+    in = 0;
+    int p0 = 1 << 30;
+    const float sub = (threadIdx.x & 1) ? 0.75f : 0.25f;
+    const Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
+#pragma unroll 1
+    for (int g = 0; g < N; ++g) {
+      const float step = (float)(g >> 1) + ((g & 1) ? 0.75f : 0.25f);
+      s[g] = swap ? ray_src(c, (float)x + sub, (float)y + step) : ray_src(c, (float)x + step, (float)y + sub);
+      hit(s[g], c.n, c.bbMin, c.bbMax, tin[g], tout[g]);
+      if (tout[g] - tin[g] > 0.0f) {
+        in |= 1u << g;
+        if (sources) {
+          const float3 q = interp_coord(c, s[g]);
+          source[g] = trilinear<VT>(C, q.x, q.y, q.z);
+        }
+      }
+      // y is constant along a ray (PlaneRay checks it)
+      const float t = (in >> g & 1u) ? tin[g] : 0.0f;
+      const float q = interp_coord(c, ray_point(c, s[g], t)).y;
+      const float fy = floorf(q);
+      b[g] = q - fy;
+      cell[g] = (int)fy;
+      p0 = min(p0, cell[g]);
+    }
+#pragma unroll 1
+    for (int g = 0; g < N; ++g) cell[g] -= p0;
+    const int ny = (int)c.dim.y, nx = (int)c.dim.x;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) yoff[p] = (unsigned)min(max(p0 + p, 0), ny - 1) * (unsigned)nx;
+  }
+};
+
+// Samples of one sub-ray over [t0, t1]: their count, the position of the
+// first, and whether they can join the line's walk.
+struct PlaneRay {
+  int J;
+  float3 q, dq;
+  bool ok;
+  __device__ __forceinline__ PlaneRay(const KConst& c, const AxisStep& A, float3 s, float t0, float t1, float b) {
+    float step;
+    J = progression(t0, t1, c.vs.x * 0.15f, step, ok);
+    q = interp_coord(c, ray_point(c, s, t0));
+    dq = interp_step(c, step);
+    const float fy = floorf(q.y);
+    ok = ok && step == A.step && fabsf(dq.y) * (float)J < 1e-5f && fy == floorf(qpos(q.y, J - 1, dq.y)) &&
+         fabsf((q.y - fy) - b) < 1e-4f;
+  }
+};
+
+// Sums v[] of the line's sub-rays, each over its [tin, tout] cut to [lo, hi]
+// (0 for those outside). slab: the first sample is the one at the ray's start.
+template <int VT, int G, int SH>
+__device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, const PlaneWalk& W, int zmaj,
+                                          const void* vol, const PlaneLine<G>& L, const unsigned (&yoff)[G + 2],
+                                          bool slab, float lo, float hi, float* v) {
+  constexpr int N = 2 * G, NP = G + 2, NS = SH == 0 ? 1 : SH + 2;
+  const int j0 = slab ? 1 : 0;
+  float S[NS][NP];
+#pragma unroll
+  for (int q = 0; q < NS; ++q)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) S[q][p] = 0.f;
+  // the middle ray
+  const float m0 = fmaxf(L.tin[G], lo), m1 = fminf(L.tout[G], hi);
+  bool mid = (L.in >> G & 1u) && m0 <= m1;
+  float bm = 0.f, bn = 0.f;
+  int Jm = 0;
+  if (mid) {
+    const PlaneRay R(c, A, L.s[G], m0, m1, L.b[G]);
+    mid = R.ok;
+    Jm = R.J;
+    bm = zmaj ? R.q.z : R.q.x;
+    bn = zmaj ? R.q.x : R.q.z;
+  }
+  if (mid && j0 < Jm)
+    plane_sums<VT, NP, SH>(A, W, vol, yoff, W.sM > 0 ? bm : -bm, W.sN > 0 ? bn : -bn, j0, Jm, S);
+  float P[NS][NP];  // (indexed by a ray's planes: local memory)
+#pragma unroll
+  for (int q = 0; q < NS; ++q)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) P[q][p] = S[q][p];
+#pragma unroll 1
+  for (int g = 0; g < N; ++g) {
+    v[g] = 0.f;
+    if (!(L.in >> g & 1u)) continue;
+    const float t0 = fmaxf(L.tin[g], lo), t1 = fminf(L.tout[g], hi);
+    if (!(t0 <= t1)) continue;
+    const PlaneRay R(c, A, L.s[g], t0, t1, L.b[g]);
+    const float f = ((zmaj ? R.q.z : R.q.x) - bm) * (float)W.sM, e = ((zmaj ? R.q.x : R.q.z) - bn) * (float)W.sN;
+    const bool joins = mid && R.ok && L.cell[g] <= G && abs(R.J - Jm) <= 1 &&
+                       (SH == 0 ? e == 0.f && f == 0.f : fabsf(e) <= kMaxShear && fabsf(f) <= kMaxShear);
+    if (!joins) {
+      v[g] = other_ray_sum<VT>(&c, vol, L.s[g], t0, t1, slab);
+      continue;
+    }
+    float sum[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = L.cell[g] + h;
+      sum[h] = P[0][p];
+      if constexpr (SH > 0) sum[h] = fmaf(e, P[1][p], fmaf(f, P[2][p], sum[h]));
+      if constexpr (SH > 1) sum[h] = fmaf(e * f, P[3][p], sum[h]);
+    }
+    float r = fmaf(L.b[g], sum[1], (1.0f - L.b[g]) * sum[0]);
+    if (R.J != Jm) {  // one sample more or less than the middle ray
+      const int j = min(R.J, Jm);
+      const Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
+      const float last = trilinear<VT>(C, qpos(R.q.x, j, R.dq.x), qpos(R.q.y, j, R.dq.y), qpos(R.q.z, j, R.dq.z));
+      if (j >= j0) r += R.J > Jm ? last : -last;
+    }
+    v[g] = slab ? r + L.source[g] : r;
+  }
+}
+
+// Pixels of a thread: G along u (v with swap) from x, y; a lane pair shares
+// them, one sub-row each.
+template <int G>
+struct PlanePixel {
+  int x, y;
+  bool active;
+  __device__ __forceinline__ PlanePixel(int swap, int x0, int y0, int x1, int y1) {
+    const int lane = threadIdx.x & 31;
+    const int across = G * (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    const int along = (int)blockIdx.y * 16 + (lane >> 1);
+    x = x0 + (swap ? along : across);
+    y = y0 + (swap ? across : along);
+    active = x < x1 && y < y1;
+  }
+};
+
+// Sum of pixel i's 4 sub-rays in the reference's order, valid in even lanes.
+__device__ __forceinline__ float pixel_sum(const float* v, int i, int swap) {
+  const float a = v[2 * i], b = v[2 * i + 1];
+  const float c = __shfl_down_sync(0xffffffffu, a, 1), d = __shfl_down_sync(0xffffffffu, b, 1);
+  return swap ? __fadd_rn(__fadd_rn(__fadd_rn(a, b), c), d) : __fadd_rn(__fadd_rn(__fadd_rn(a, c), b), d);
+}
+
+template <int VT, int G, int SH>
+__global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ KConst c,
+                                                        const __grid_constant__ AxisStep A,
+                                                        const __grid_constant__ PlaneWalk W, int zmaj, int swap,
+                                                        const void* __restrict__ vol, float* __restrict__ proj,
+                                                        float* __restrict__ dist, size_t pitchE, int x0, int y0,
+                                                        int x1, int y1) {
+  const PlanePixel<G> P(swap, x0, y0, x1, y1);
+  PlaneLine<G> L;
+  unsigned yoff[G + 2];
+  float v[2 * G];
+  L.in = 0;
+  if (P.active) {
+    L.template init<VT>(c, vol, P.x, P.y, swap, false, yoff);
+    line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, false, -FLT_MAX, FLT_MAX, v);
+  }
+#pragma unroll 1
+  for (int i = 0; i < G; ++i) {
+    float n[2], d[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int g = 2 * i + h;
+      const bool in = (L.in >> g & 1u) != 0;
+      n[h] = in ? 1.0f : 0.0f;
+      d[h] = in ? L.tout[g] - L.tin[g] : 0.0f;
+      if (!in) v[g] = 0.0f;
+    }
+    const float sum = pixel_sum(v, i, swap), gx = pixel_sum(n, 0, swap), gz = pixel_sum(d, 0, swap);
+    const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
+    if (P.active && !(threadIdx.x & 1) && x < x1 && y < y1) {
+      const size_t o = (size_t)y * pitchE + x;
+      proj[o] += sum * c.vs.x * 0.15f * 0.25f;
+      dist[o] = fmaxf(0.0f, gz / gx);
+    }
+  }
+}
+
+template <int VT, int G, int SH>
+__global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ KConst c,
+                                                       const __grid_constant__ AxisStep A,
+                                                       const __grid_constant__ PlaneWalk W, int zmaj, int swap,
+                                                       const void* __restrict__ vol, float* __restrict__ imgs,
+                                                       size_t img_stride, size_t pitchE,
+                                                       const __grid_constant__ SlabTable slabs, int clear, int x0,
+                                                       int y0, int x1, int y1) {
+  const PlanePixel<G> P(swap, x0, y0, x1, y1);
+  PlaneLine<G> L;
+  unsigned yoff[G + 2];
+  L.in = 0;
+  if (P.active) L.template init<VT>(c, vol, P.x, P.y, swap, true, yoff);
+  // slabs met by each pixel's rays, and the union over the warp's
+  int klo[G], khi[G], wlo = ESB_MAX_SLABS, whi = -1;
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    klo[i] = ESB_MAX_SLABS;
+    khi[i] = -1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (!(L.in >> (2 * i + h) & 1u)) continue;
+      const float t0 = L.tin[2 * i + h], t1 = L.tout[2 * i + h];
+      for (int k = 0; k < slabs.count; ++k) {
+        if (fmaxf(t0, slabs.bound[k]) <= fminf(t1, slabs.bound[k + 1])) {
+          klo[i] = min(klo[i], k);
+          khi[i] = max(khi[i], k);
+        }
+      }
+    }
+    klo[i] = min(klo[i], __shfl_xor_sync(0xffffffffu, klo[i], 1));
+    khi[i] = max(khi[i], __shfl_xor_sync(0xffffffffu, khi[i], 1));
+    wlo = min(wlo, klo[i]);
+    whi = max(whi, khi[i]);
+  }
+  for (int o = 2; o <= 16; o <<= 1) {
+    wlo = min(wlo, __shfl_xor_sync(0xffffffffu, wlo, o));
+    whi = max(whi, __shfl_xor_sync(0xffffffffu, whi, o));
+  }
+  const bool writer = P.active && !(threadIdx.x & 1);
+  for (int k = wlo; k <= whi; ++k) {
+    float v[2 * G];
+    if (L.in) {
+      line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, true, slabs.bound[k], slabs.bound[k + 1], v);
+    } else {
+#pragma unroll
+      for (int g = 0; g < 2 * G; ++g) v[g] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const float sum = pixel_sum(v, i, swap);
+      const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
+      if (writer && x < x1 && y < y1 && k >= klo[i] && k <= khi[i])
+        imgs[(size_t)k * img_stride + (size_t)y * pitchE + x] = sum * c.vs.x * 0.15f * 0.25f;
+    }
+  }
+  if (clear && writer) {
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
+      if (x < x1 && y < y1) clear_slabs(imgs + (size_t)y * pitchE + x, img_stride, slabs.count, klo[i], khi[i]);
+    }
+  }
+}
+
+// The plane kernels' launch: G pixels per thread (0: not taken), whether the
+// line's rays differ in y only.
+struct PlaneLaunch {
+  int G = 0, shear = 0, swap = 0, zmaj = 0;
+  AxisStep A;
+  PlaneWalk W;
+  PlaneLaunch(const KConst& c, int w, int h) {
+    bool z;
+    int sm, sn;
+    A = axis_step(c, z, sm, sn);
+    if (!axis_projection(c) || !(A.step > 0.0f) || (double)c.dim.x * c.dim.y * c.dim.z >= 1073741824.0) return;
+    swap = axis_swap(c);
+    zmaj = z ? 1 : 0;
+    // voxels that half a pixel along the line moves a ray in x, y, z
+    const float au = swap ? c.aniso[1] : c.aniso[0], av = swap ? c.aniso[4] : c.aniso[3];
+    const float ex = 0.5f * fabsf(au * c.u.x + av * c.v.x) * c.bbRcp.x * c.dim.x;
+    const float ey = 0.5f * fabsf(au * c.u.y + av * c.v.y) * c.bbRcp.y * c.dim.y;
+    const float ez = 0.5f * fabsf(au * c.u.z + av * c.v.z) * c.bbRcp.z * c.dim.z;
+    shear = ex > 0.f || ez > 0.f ? 1 : 0;
+    const int along = swap ? w : h, across = swap ? h : w;
+    for (int g = 4; g >= 2 && !G; g -= 2) {
+      // the offset of the line's outermost ray, taken at its start or along
+      // the ray to the volume's face, and its planes
+      const bool small = (float)g * (ex + ez) <= kMaxShear;
+      const bool planes = (float)(2 * g - 1) * ey < (float)g - 0.05f;
+      // 2 pixels per thread from 2 warps per scheduler on, 4 from 4 (measured:
+      // 128 warps of 2 pixels 25 us against the axis walk's 15, 2048 warps 113
+      // against 178; 1024 warps of 4 pixels 141 against the 113 of 2)
+      const bool enough = (double)((across + g - 1) / g) * ((along + 15) / 16) >= 148.0 * 4 * g;
+      if (small && planes && enough) G = g;
+    }
+    const unsigned sz = (unsigned)c.dim.x * (unsigned)c.dim.y;
+    W.sM = sm;
+    W.sN = sn;
+    W.nM = (int)(z ? c.dim.z : c.dim.x);
+    W.nN = (int)(z ? c.dim.x : c.dim.z);
+    W.dM = z ? sz : 1;
+    W.dN = z ? 1 : sz;
+  }
+};
+
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.
 bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 4294967295.0; }
 
@@ -789,6 +1236,28 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
     }                                                                           \
   } while (0)
 
+// A launch of a plane kernel (ESB_PLANES), 4 warps per block.
+#define ESB_PLANES_SH(VT, GG)              \
+  do {                                     \
+    if (L.shear) ESB_PLANES(VT, GG, 1);    \
+    else ESB_PLANES(VT, GG, 0);            \
+  } while (0)
+#define ESB_PLANES_VT(VT)                  \
+  do {                                     \
+    if (L.G == 4) ESB_PLANES_SH(VT, 4);    \
+    else ESB_PLANES_SH(VT, 2);             \
+  } while (0)
+#define ESB_PLANES_LAUNCH()                                                                          \
+  do {                                                                                               \
+    const int along = L.swap ? x1 - x0 : y1 - y0, across = L.swap ? y1 - y0 : x1 - x0;                \
+    const dim3 blk(128), grd((across + 4 * L.G - 1) / (4 * L.G), (along + 15) / 16);                  \
+    if (vt == ESB_VOXEL_F32) ESB_PLANES_VT(ESB_VOXEL_F32);                                           \
+    else if (vt == ESB_VOXEL_F16) ESB_PLANES_VT(ESB_VOXEL_F16);                                      \
+    else ESB_PLANES_VT(ESB_VOXEL_BF16);                                                              \
+    ESB_COUNT_LAUNCH();                                                                              \
+    return cudaGetLastError();                                                                       \
+  } while (0)
+
 // Volumes below 4 GiB take 32-bit byte offsets in the axis walk.
 #define ESB_AXIS_LAUNCH(KER, GRD, BLK, ST, ...)                                                                \
   do {                                                                                                        \
@@ -808,6 +1277,14 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
                                 size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1,
                                 int y1, cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0 || slabs.count <= 0) return cudaSuccess;
+  const PlaneLaunch L(c, x1 - x0, y1 - y0);
+  if (L.G) {
+#define ESB_PLANES(VT, GG, SH)                                                                                        \
+  k_slicer_planes<VT, GG, SH ? 2 : 0><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, imgs, img_stride, pitchE, \
+                                                           slabs, clear, x0, y0, x1, y1)
+    ESB_PLANES_LAUNCH();
+#undef ESB_PLANES
+  }
   if (axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
@@ -841,6 +1318,13 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
                                 size_t pitchE, float tmin, float tmax, int x0, int y0, int x1, int y1,
                                 cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
+  const PlaneLaunch L(c, x1 - x0, y1 - y0);
+  if (mode == 0 && L.G) {
+#define ESB_PLANES(VT, GG, SH) \
+  k_project_planes<VT, GG, SH><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, proj, dist, pitchE, x0, y0, x1, y1)
+    ESB_PLANES_LAUNCH();
+#undef ESB_PLANES
+  }
   if (mode == 0 && axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
