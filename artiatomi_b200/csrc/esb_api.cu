@@ -90,6 +90,12 @@ cudaError_t launch_bad_pixels(float* img, long n, float threshold, float value, 
 cudaError_t launch_window_div(const float* sq, size_t shift, int maxsize, int pw, int ph, float div, float* out,
                               cudaStream_t st);
 cudaError_t launch_normalize(const float* in, float* out, long n, float mean, float std_, cudaStream_t st);
+cudaError_t launch_prepare_square(const void* in, int type, int pw, int ph, int n, int bx, int by, int mirrorY,
+                                  float* sq, double* stats, cudaStream_t st);
+cudaError_t launch_prepare_bad(float* sq, long n, float bad_value, double* stats, cudaStream_t st);
+cudaError_t launch_prepare_stats(const float* sq, int n, int w, int h, float div, double* stats, cudaStream_t st);
+cudaError_t launch_prepare_normalize(const float* sq, int n, int pw, int ph, float div, const double* stats,
+                                     double count, int norm, float* out, cudaStream_t st);
 cudaError_t launch_crop_to_square_batch(int pw, int ph, float* images, size_t img_stride, int count, int apply_crop,
                                         int seq_crop, float2 cut, float2 dim, const int* p, int maxsize, float* sq,
                                         size_t sq_stride, int bx, int by, cudaStream_t st);
@@ -1466,7 +1472,7 @@ int esb_prepare_projection(esb_reconstructor* r, const esb_prepare_config* pc, c
   const long npx = (long)W * H, nsq = (long)N * N;
   cudaStream_t st = r->stream;
   // buffers (the CTF configuration already owns a square, a spectrum and plans)
-  if (!r->prep_img) ESB_CK(cudaMalloc(&r->prep_img, npx * sizeof(float)), "esb_prepare_projection");
+  if (pc->wbp && !r->prep_img) ESB_CK(cudaMalloc(&r->prep_img, npx * sizeof(float)), "esb_prepare_projection");
   if (!r->prep_stats) ESB_CK(cudaMalloc(&r->prep_stats, 4 * sizeof(double)), "esb_prepare_projection");
   float* sq = r->square_d;
   float* spec = r->fft_d;
@@ -1487,6 +1493,39 @@ int esb_prepare_projection(esb_reconstructor* r, const esb_prepare_config* pc, c
   ESB_FFT(cufftSetStream(r2c, st), "esb_prepare_projection");
   ESB_FFT(cufftSetStream(c2r, st), "esb_prepare_projection");
   double h[4];
+  if (!pc->wbp) {
+    // SART: every mean is taken on the device, one synchronisation at the end
+    // (:1192-1227, 1274-1372)
+    const char* where = "esb_prepare_projection";
+    ESB_CK(cudaMemsetAsync(r->prep_stats, 0, 4 * sizeof(double), st), where);
+    ESB_CK(launch_prepare_square(in, pc->input_type, W, H, N, r->borderX, r->borderY, pc->mirror_y, sq, r->prep_stats,
+                                 st), where);
+    if (pc->correct_bad_pixels)
+      ESB_CK(launch_prepare_bad(sq, nsq, pc->bad_pixel_value, r->prep_stats, st), where);
+    float normVal = 1.0f;
+    if (!pc->skip_filter) {
+      ESB_FFT(cufftExecR2C(r2c, (cufftReal*)sq, (cufftComplex*)spec), "esb_prepare_projection R2C");
+      ESB_CK(launch_fourier_filter(spec, N, pc->lp, pc->hp, pc->lps, pc->hps, st), where);
+      if (pc->dose_weighting)
+        ESB_CK(launch_dose_weighting(spec, N, pc->accumulated_dose, pc->pixel_size_nm * 10.0f, st), where);
+      ESB_FFT(cufftExecC2R(c2r, (cufftComplex*)spec, (cufftReal*)sq), "esb_prepare_projection C2R");
+      normVal = (float)N * (float)N;
+    }
+    const bool half = pc->normalization == ESB_PNM_NONE;  // the centre half's mean
+    const int sw = half ? W / 2 : W, sh = half ? H / 2 : H;
+    const float* window = sq + r->squareShift;
+    const double count = (double)sw * (double)sh;
+    ESB_CK(launch_prepare_stats(window + (half ? (size_t)(H / 4) * N + W / 4 : 0), N, sw, sh, normVal, r->prep_stats,
+                                st), where);
+    ESB_CK(launch_prepare_normalize(window, N, W, H, normVal, r->prep_stats, count, pc->normalization, out, st), where);
+    ESB_CK(cudaMemcpyAsync(h, r->prep_stats, 4 * sizeof(double), cudaMemcpyDeviceToHost, st), where);
+    ESB_CK(cudaStreamSynchronize(st), where);
+    const double mu = h[2] / count, var = h[3] / count - mu * mu;
+    if (mean_out) *mean_out = (float)mu;
+    if (std_out) *std_out = (float)sqrt(var > 0.0 ? var : 0.0);
+    if (bad_out) *bad_out = pc->correct_bad_pixels ? (int)h[1] : 0;
+    return ok();
+  }
   auto stats = [&](const float* img, size_t pitchE, int x0, int y0, int w, int hh) -> int {
     ESB_CK(cudaMemsetAsync(r->prep_stats, 0, 2 * sizeof(double), st), "esb_prepare_projection");
     ESB_CK(launch_window_stats(img, pitchE, x0, y0, w, hh, r->prep_stats, st), "esb_prepare_projection");
@@ -1518,7 +1557,7 @@ int esb_prepare_projection(esb_reconstructor* r, const esb_prepare_config* pc, c
     m = (float)mu;
     sd = (float)sqrt(var > 0.0 ? var : 0.0);
   };
-  if (pc->wbp) {  // statistics of the raw window (:1231-1270)
+  {  // statistics of the raw window (:1231-1270)
     ESB_CK(launch_window_div(sq, r->squareShift, N, W, H, 1.0f, r->prep_img, st), "esb_prepare_projection");
     if ((rc = stats(r->prep_img, W, 0, 0, W, H))) return rc;
     mean_std(h[0], h[1], (double)npx, meanValue, stdValue);
@@ -1532,36 +1571,18 @@ int esb_prepare_projection(esb_reconstructor* r, const esb_prepare_config* pc, c
     ESB_CK(launch_normalize(r->prep_img, out, npx, mean_hf, std_hf, st), "esb_prepare_projection");
     ESB_CK(launch_make_square(W, H, W, out, N, sq, r->borderX, r->borderY, 0, 0, st), "esb_prepare_projection");
   }
-  float normVal = 1.0f;
-  if (!pc->skip_filter || pc->wbp) {  // (:1274-1310)
+  {  // (:1274-1310)
     ESB_FFT(cufftExecR2C(r2c, (cufftReal*)sq, (cufftComplex*)spec), "esb_prepare_projection R2C");
     if (!pc->skip_filter)
       ESB_CK(launch_fourier_filter(spec, N, pc->lp, pc->hp, pc->lps, pc->hps, st), "esb_prepare_projection");
     if (pc->dose_weighting)
       ESB_CK(launch_dose_weighting(spec, N, pc->accumulated_dose, pc->pixel_size_nm * 10.0f, st),
              "esb_prepare_projection");
-    if (pc->wbp) ESB_CK(launch_wbp_weighting(spec, N, pc->psi_deg, pc->wbp_filter, st), "esb_prepare_projection");
+    ESB_CK(launch_wbp_weighting(spec, N, pc->psi_deg, pc->wbp_filter, st), "esb_prepare_projection");
     ESB_FFT(cufftExecC2R(c2r, (cufftComplex*)spec, (cufftReal*)sq), "esb_prepare_projection C2R");
-    normVal = (float)N * (float)N;
   }
   // normalise from the FFT (:1315-1316)
-  ESB_CK(launch_window_div(sq, r->squareShift, N, W, H, normVal, r->prep_img, st), "esb_prepare_projection");
-  if (!pc->wbp) {  // SART: statistics of the filtered window (:1320-1372)
-    if (pc->normalization == ESB_PNM_NONE) {
-      if ((rc = stats(r->prep_img, W, W / 4, H / 4, W / 2, H / 2))) return rc;
-      mean_std(h[0], h[1], (double)(W / 2) * (double)(H / 2), meanValue, stdValue);
-    } else {
-      if ((rc = stats(r->prep_img, W, 0, 0, W, H))) return rc;
-      mean_std(h[0], h[1], (double)npx, meanValue, stdValue);
-    }
-    float std_hf = stdValue, mean_hf = meanValue;
-    if (pc->normalization == ESB_PNM_MEAN) std_hf = meanValue;
-    if (pc->normalization == ESB_PNM_NONE) std_hf = 1;
-    ESB_CK(launch_normalize(r->prep_img, out, npx, mean_hf, std_hf, st), "esb_prepare_projection");
-  } else {
-    ESB_CK(cudaMemcpyAsync(out, r->prep_img, npx * sizeof(float), cudaMemcpyDeviceToDevice, st),
-           "esb_prepare_projection");
-  }
+  ESB_CK(launch_window_div(sq, r->squareShift, N, W, H, (float)N * (float)N, out, st), "esb_prepare_projection");
   if (mean_out) *mean_out = meanValue;
   if (std_out) *std_out = stdValue;
   if (bad_out) *bad_out = bad;

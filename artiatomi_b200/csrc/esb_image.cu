@@ -5,6 +5,8 @@
 // storage conversions.
 #include <math.h>
 
+#include <algorithm>
+
 #include "esb_bp_core.cuh"
 
 namespace esb {
@@ -450,6 +452,89 @@ __global__ void k_normalize(const float* __restrict__ in, float* __restrict__ ou
     out[i] = (in[i] - mean) / (-std_);
 }
 
+// The same passes for the SART branch without a round trip to the host: the
+// statistics stay on the device (stats: [0] sum of the square, [1] bad
+// pixels, [2] sum and [3] sum of squares of the filtered window), and each
+// pass that needs a mean takes it from there. Rows are walked by block rows,
+// so that no thread divides to find its pixel.
+
+// Raw image converted, padded by mirroring to the square (k_make_square) and
+// summed: one read and one write in place of three of each.
+template <typename T>
+__global__ void __launch_bounds__(256) k_prepare_square(const T* __restrict__ in, int pw, int ph, int n, int bx, int by,
+                                                        int mirrorY, float* __restrict__ sq,
+                                                        double* __restrict__ stats) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  double sum = 0.0;
+  if (x < n) {
+    int xi = x - bx;
+    if (xi < 0) xi = -xi - 1;
+    if (xi >= pw) xi = 2 * pw - xi - 1;
+    xi = min(max(xi, 0), pw - 1);  // (padding wider than the image)
+    for (int y = blockIdx.y; y < n; y += gridDim.y) {
+      int yi = y - by;
+      if (yi < 0) yi = -yi - 1;
+      if (yi >= ph) yi = 2 * ph - yi - 1;
+      yi = min(max(yi, 0), ph - 1);
+      if (mirrorY) yi = ph - yi - 1;
+      const float v = (float)in[(size_t)yi * pw + xi];
+      sq[(size_t)y * n + x] = v;
+      sum += v;
+    }
+  }
+  sum = block_sum(sum);
+  if (threadIdx.x == 0) atomicAdd(stats, sum);
+}
+
+// k_bad_pixels with the threshold bad_value * mean of the square's statistics.
+__global__ void __launch_bounds__(256) k_prepare_bad(float* __restrict__ sq, long n, float bad_value,
+                                                     double* __restrict__ stats) {
+  const float mean = (float)(stats[0] / (double)n), threshold = bad_value * mean;
+  double c = 0.0;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    if (sq[i] > threshold) {
+      sq[i] = mean;
+      c += 1.0;
+    }
+  }
+  c = block_sum(c);
+  if (threadIdx.x == 0 && c > 0.0) atomicAdd(stats + 1, c);
+}
+
+// Sum and sum of squares of sq / div over a w x h window.
+__global__ void __launch_bounds__(256) k_prepare_stats(const float* __restrict__ sq, int n, int w, int h, float div,
+                                                       double* __restrict__ stats) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  double s = 0.0, q = 0.0;
+  if (x < w) {
+    for (int y = blockIdx.y; y < h; y += gridDim.y) {
+      const double v = sq[(size_t)y * n + x] / div;
+      s += v;
+      q += v * v;
+    }
+  }
+  s = block_sum(s);
+  q = block_sum(q);
+  if (threadIdx.x == 0) {
+    atomicAdd(stats + 2, s);
+    atomicAdd(stats + 3, q);
+  }
+}
+
+// out = (sq / div - mean) / (-std) over the pw x ph window, mean and std from
+// the sums over `count` values (norm: ESB_PNM_*).
+__global__ void __launch_bounds__(256) k_prepare_normalize(const float* __restrict__ sq, int n, int pw, int ph,
+                                                           float div, const double* __restrict__ stats, double count,
+                                                           int norm, float* __restrict__ out) {
+  const double mu = stats[2] / count, var = stats[3] / count - mu * mu;
+  const float mean = (float)mu;
+  const float std_ = norm == ESB_PNM_MEAN ? mean : (norm == ESB_PNM_NONE ? 1.0f : (float)sqrt(var > 0.0 ? var : 0.0));
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= pw) return;
+  for (int y = blockIdx.y; y < ph; y += gridDim.y)
+    out[(size_t)y * pw + x] = (sq[(size_t)y * n + x] / div - mean) / (-std_);
+}
+
 // ----------------------------------------------------------------- launchers
 static inline dim3 grid2(int w, int h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h + b.y - 1) / b.y); }
 
@@ -605,6 +690,48 @@ cudaError_t launch_normalize(const float* in, float* out, long n, float mean, fl
 
 
 
+
+// Blocks of 256 columns, about 8 blocks per SM over the rows.
+static inline dim3 rows_grid(int w, int h) {
+  const int gx = (w + 255) / 256;
+  return dim3(gx, std::max(1, std::min(h, 148 * 8 / gx)));
+}
+
+cudaError_t launch_prepare_square(const void* in, int type, int pw, int ph, int n, int bx, int by, int mirrorY,
+                                  float* sq, double* stats, cudaStream_t st) {
+  const dim3 g = rows_grid(n, n);
+#define ESB_PREP(T) k_prepare_square<T><<<g, 256, 0, st>>>((const T*)in, pw, ph, n, bx, by, mirrorY, sq, stats)
+  switch (type) {
+    case ESB_PIX_S16: ESB_PREP(int16_t); break;
+    case ESB_PIX_U16: ESB_PREP(uint16_t); break;
+    case ESB_PIX_S32: ESB_PREP(int32_t); break;
+    case ESB_PIX_U32: ESB_PREP(uint32_t); break;
+    default: ESB_PREP(float); break;
+  }
+#undef ESB_PREP
+  ESB_COUNT_LAUNCH();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prepare_bad(float* sq, long n, float bad_value, double* stats, cudaStream_t st) {
+  k_prepare_bad<<<grid1(n), 256, 0, st>>>(sq, n, bad_value, stats);
+  ESB_COUNT_LAUNCH();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prepare_stats(const float* sq, int n, int w, int h, float div, double* stats, cudaStream_t st) {
+  if (w <= 0 || h <= 0) return cudaSuccess;
+  k_prepare_stats<<<rows_grid(w, h), 256, 0, st>>>(sq, n, w, h, div, stats);
+  ESB_COUNT_LAUNCH();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prepare_normalize(const float* sq, int n, int pw, int ph, float div, const double* stats,
+                                     double count, int norm, float* out, cudaStream_t st) {
+  k_prepare_normalize<<<rows_grid(pw, ph), 256, 0, st>>>(sq, n, pw, ph, div, stats, count, norm, out);
+  ESB_COUNT_LAUNCH();
+  return cudaGetLastError();
+}
 
 cudaError_t launch_wbp_weighting(float* spec, int n, float psi_deg, int fm, cudaStream_t st) {
   dim3 b(32, 8);
