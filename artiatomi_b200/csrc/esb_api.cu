@@ -42,7 +42,8 @@ cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float
 cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_stride, int count, int pw, int ph, int os,
                             int linear, float2* up, size_t up_stride, cudaStream_t st);
 bool bp_can_upsample(const KConst& k, int os);
-bool bp_uses_axis(const KConst& k, int os);
+bool bp_reads_at_samples(const KConst& k, int os);
+bool bp_uses_axis(const KConst& k, int os, bool up);
 bool bp_set_eligible(const KConst& k, int os, int nslab);
 cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const SlabTable* slabs, int count,
                                size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
@@ -888,7 +889,7 @@ static BpShape rec_bp_shape(esb_reconstructor* r, const KConst& c, int vt, const
                             const SlabTable& T, int linear, const float2* up, size_t up_stride) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y, os = r->cfg.oversampling;
   BpShape s{kBpShapes[0][0], kBpShapes[0][1], 0, 0};
-  if (!bp_uses_axis(c, os)) return s;
+  if (!bp_uses_axis(c, os, up != nullptr)) return s;
   const int nz = (int)c.dim.z, planes = std::min(nz, 32);
   const size_t plane = (size_t)c.dim.x * (size_t)c.dim.y * (vt == ESB_VOXEL_F32 ? 4 : 2);
   const int i = rec_tuned(r, tune_key(r, 2, vt, c, T.count > 0), kNBpShapes, 0, [&](int k) {
@@ -1109,8 +1110,7 @@ static int rec_subvol_slab_images(esb_reconstructor* r, const esb_vol_geom* full
 
 // The buffer of `count` pre-sampled images (launch_upsample,
 // launch_crop_upsample); NULL when the geometry does not allow them
-// (oversampling not a power of two, magnification anisotropy) or they would
-// exceed 8 GiB, and the back-projection then filters the slab images itself.
+// (oversampling not a power of two) or they would exceed 8 GiB, and the back-projection then filters the slab images itself.
 // `up_stride` receives the (value, row) pairs per image.
 static float2* rec_up_images(esb_reconstructor* r, const KConst& c, int count, size_t& up_stride) {
   const esb_recon_config& cf = r->cfg;
@@ -1266,16 +1266,17 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
     size_t up_stride = 0;
     float2* up = cf.variant == ESB_VARIANT_FAST ? rec_up_images(r, c, 1, up_stride) : nullptr;
     ESB_CK(cudaGetLastError(), "back projection");
+    const bool one_pass = up && bp_reads_at_samples(c, cf.oversampling);
     {
       PhaseScope ps(r, 3);
-      if (up) {
+      if (one_pass) {
         ESB_CK(launch_crop_upsample(c, W, H, img, cut, dim, p, cf.oversampling, up, r->stream), "back projection");
       } else {
         ESB_CK(launch_crop_border(W, H, W, img, cut, dim, p, r->stream), "back projection");
       }
     }
     if (cf.variant == ESB_VARIANT_FAST) {
-      if (!up) {
+      if (!one_pass) {
         int rc2;
         if ((rc2 = rec_slab_capacity(r, 1))) return rc2;
         PhaseScope ps(r, 3);
@@ -1284,6 +1285,9 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
       SlabTable none;
       none.count = 0;
       PhaseScope ps(r, 1);
+      if (up && !one_pass)
+        ESB_CK(launch_upsample(c, r->slab_imgs, 0, 1, W, H, cf.oversampling, 0, up, up_stride, r->stream),
+               "back projection");
       const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, 0, none, 0, up, up_stride);
       ESB_CK(launch_bp_fast_slabs(c, vol, voxel_type, r->slab_imgs, 0, none, W, H, W, lambda, cf.oversampling, 0.0f,
                                   9999999999999.0f, 0, r->stream, 1, up, up_stride, &shape), "back projection");

@@ -245,18 +245,22 @@ __global__ void __launch_bounds__(128) k_bp_axis_set(const __grid_constant__ BpS
 // and stored with the point's value in every slab image.
 __global__ void __launch_bounds__(256) k_upsample(const float* __restrict__ imgs, size_t img_stride, int count, int pw,
                                                   int ph, int os, float inv, int linear, RowGeom rg, int swapped,
-                                                  float2* __restrict__ up, size_t up_stride) {
+                                                  const __grid_constant__ KConst k, float2* __restrict__ up,
+                                                  size_t up_stride) {
   const int fast = blockIdx.x * blockDim.x + threadIdx.x, slow = blockIdx.y * blockDim.y + threadIdx.y;
   const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
   if (fast >= nf || slow >= ns) return;
   const int mu = swapped ? fast : slow, mv = swapped ? slow : fast;
   const float px = ((float)mu + 0.5f) * inv, py = ((float)mv + 0.5f) * inv;
+  // where the sample is read: through the inverse magnification anisotropy
+  const float xA = k.anisoInv[0] * px + k.anisoInv[1] * py + k.anisoInv[2];
+  const float yA = k.anisoInv[3] * px + k.anisoInv[4] * py + k.anisoInv[5];
   const float row = __int_as_float(sample_row(rg, mu, mv));
   float2* out = up + (size_t)slow * nf + fast;
 #pragma unroll 1
   for (int s = 0; s < count; ++s)
     out[(size_t)s * up_stride] =
-        make_float2(sample_image(imgs + (size_t)s * img_stride, pw, ph, (size_t)pw, px, py, linear != 0, true), row);
+        make_float2(sample_image(imgs + (size_t)s * img_stride, pw, ph, (size_t)pw, xA, yA, linear != 0, true), row);
 }
 
 }  // namespace
@@ -270,7 +274,7 @@ cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float
   const BpGeom g = make_geom(k, os);
   const float inv = 1.0f / (float)os;
   dim3 blk(32, 4, 1), grd((nq + 31) / 32, (ny + 3) / 4, nz);
-  if (axis_eligible(k, g)) {
+  if (ups ? axis_beam(k, g) : axis_eligible(k, g)) {
     const AxisGeom a = make_axis_geom(k, g, os);
     int z0 = 0;
     if (shape) {  // block of bx quads x by rows (bx * by <= 128); planes [z0, z0 + nz)
@@ -380,25 +384,28 @@ cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_strid
                             int linear, float2* up, size_t up_stride, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
   const BpGeom g = make_geom(k, os);
-  const int swapped = axis_eligible(k, g) && up_swapped(make_axis_geom(k, g, os)) ? 1 : 0;
+  const int swapped = axis_beam(k, g) && up_swapped(make_axis_geom(k, g, os)) ? 1 : 0;
   const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
   const dim3 blk(32, 8), grd((nf + 31) / 32, (ns + 7) / 8);
   k_upsample<<<grd, blk, 0, st>>>(imgs, img_stride, count, pw, ph, os, 1.0f / (float)os, linear, make_row_geom(k, os),
-                                  swapped, up, up_stride);
+                                  swapped, k, up, up_stride);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
-// Whether k_bp_fast may read pre-sampled images: the sub-pixel recurrence is
-// exact (power-of-two oversampling) and samples are read at (px, py) (no
-// magnification anisotropy).
-bool bp_can_upsample(const KConst& k, int os) {
-  const BpGeom g = make_geom(k, os);
-  return g.exact_grid && g.aniso_identity;
-}
+// Whether the back-projection may read pre-sampled images: the sub-pixel
+// recurrence is exact (power-of-two oversampling).
+bool bp_can_upsample(const KConst& k, int os) { return make_geom(k, os).exact_grid != 0; }
+
+// Whether samples are read where they lie (no magnification anisotropy):
+// launch_crop_upsample's case.
+bool bp_reads_at_samples(const KConst& k, int os) { return make_geom(k, os).aniso_identity != 0; }
 
 // Whether launch_bp_fast_slabs takes the single-axis kernel (whose launch
-// shape BpShape sets).
-bool bp_uses_axis(const KConst& k, int os) { return axis_eligible(k, make_geom(k, os)); }
+// shape BpShape sets), on pre-sampled images (up) or reading directly.
+bool bp_uses_axis(const KConst& k, int os, bool up) {
+  const BpGeom g = make_geom(k, os);
+  return up ? axis_beam(k, g) : axis_eligible(k, g);
+}
 
 }  // namespace esb

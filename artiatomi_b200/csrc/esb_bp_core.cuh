@@ -151,10 +151,10 @@ __device__ __forceinline__ float sample_interior(const float* __restrict__ img, 
 // clamps are skipped unless pbx or pbz is 0 under bilinear interpolation.
 //
 // up (may be NULL): the image pre-sampled at every point of the sub-pixel
-// grid, up[mu][mv] = image at ((mu + 0.5) / os, (mv + 0.5) / os) with row
-// length upH = ph * os (k_upsample). With a power-of-two oversampling and no
-// anisotropy the recurrence visits exactly those points, so each sample is
-// one load instead of a filtered read.
+// grid, up[mu][mv] = image where the sample at ((mu + 0.5) / os, (mv + 0.5) /
+// os) is read, with row length upH = ph * os (k_upsample). With a
+// power-of-two oversampling the recurrence visits exactly those points, so
+// each sample is one load instead of a filtered read.
 __device__ __forceinline__ void voxel_sums(const KConst& k, const BpGeom& g, const float* __restrict__ img, int pw,
                                            int ph, size_t pitchE, int os, float inv, bool linear, bool transposed,
                                            int x, int y, int z, int pbx, int pby, int pbz, int pbw, float& acc,
@@ -480,10 +480,10 @@ inline AxisGeom make_axis_geom(const KConst& k, const BpGeom& b, int os) {
 }
 
 // Whether a projection takes the single-axis sums: beam without a y
-// component, exact sub-pixel lattice, samples read at (px, py).
-inline bool axis_eligible(const KConst& k, const BpGeom& g) {
-  return g.exact_grid && g.aniso_identity && fabsf(k.n.y) <= 1e-6f;
-}
+// component and exact sub-pixel lattice, on pre-sampled images (axis_beam);
+// reading the images directly, also samples read at (px, py).
+inline bool axis_beam(const KConst& k, const BpGeom& g) { return g.exact_grid && fabsf(k.n.y) <= 1e-6f; }
+inline bool axis_eligible(const KConst& k, const BpGeom& g) { return axis_beam(k, g) && g.aniso_identity; }
 
 // row_offset of the samples of the voxels of one row (the 4 voxels of a
 // quad): formed once, at sample (mu, mv) near the first voxel's centre

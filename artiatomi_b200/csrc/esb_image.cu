@@ -553,11 +553,12 @@ cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2
   return cudaGetLastError();
 }
 
-// k_crop_upsample of one projection (row-major, dense); k gives the rows.
+// k_crop_upsample of one projection (row-major, dense) without magnification
+// anisotropy; k gives the rows.
 cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, float2 cut, float2 dim, const int* p,
                                  int os, float2* up, cudaStream_t st) {
   const bpcore::BpGeom g = bpcore::make_geom(k, os);
-  const int swapped = bpcore::axis_eligible(k, g) && bpcore::up_swapped(bpcore::make_axis_geom(k, g, os)) ? 1 : 0;
+  const int swapped = bpcore::axis_beam(k, g) && bpcore::up_swapped(bpcore::make_axis_geom(k, g, os)) ? 1 : 0;
   const int tile = (long)((pw + 31) / 32) * ((ph + 31) / 32) >= 296 ? 32 : 16;  // two 32 x 32 tiles per SM
   const dim3 b(tile, 256 / tile), grd((pw + tile - 1) / tile, (ph + tile - 1) / tile);
   const auto kernel = tile == 32 ? k_crop_upsample<32> : k_crop_upsample<16>;
