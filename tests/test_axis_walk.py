@@ -124,3 +124,83 @@ def test_axis_adjoint_small_and_odd(dims, psi):
             lhs, rhs = float((ax.double() * y.double()).sum()), float((x.double() * aty.double()).sum())
             assert abs(lhs - rhs) <= 1e-5 * float(ax.double().norm() * y.double().norm()), (i, shift, lhs, rhs)
             assert rel_l2(host(grad), host(atax)) <= 1e-5, (i, shift)
+
+
+@pytest.mark.parametrize("dims,W,H", [((389, 97, 7), 101, 397), ((389, 421, 6), 431, 397)])
+@pytest.mark.parametrize("psi", [0.0, 0.3, -0.29, 90.2, 179.6])
+def test_lines_of_rays(dims, W, H, psi):
+    """Next to no in-plane rotation: k_project_planes and k_slicer_planes
+    (2 pixels per thread on the small detector, 4 on the large one; 179.6
+    degrees allows 2 on either) against the faithful march and slicer over
+    the same voxels, for every voxel type, a detector region and slabs; the
+    bound as above, of which the lines' expansion takes a tenth."""
+    import torch
+
+    import artiatomi_b200 as E
+
+    c = _case(dims, psi, W, H)
+    n = len(TILTS)
+    roi = (3, 5, W - 4, H - 1)
+    for i in range(n):
+        k = E.set_constant_values(c["pg"][i], c["vg"])
+        for dtype in (torch.float32, torch.float16, torch.bfloat16):
+            vol = cuda(c["vol"]).to(dtype)
+            (p, d), (q, e), (r, s) = [[torch.full((H, W), 0.25, device="cuda") for _ in range(2)] for _ in range(3)]
+            E.forward_project(k, vol, p, d, fast=True)
+            E.forward_project(k, vol, q, e)
+            E.forward_project(k, vol, r, s, roi=roi, fast=True)
+            torch.cuda.synchronize()
+            p, d, q, e, r, s = (host(t) for t in (p, d, q, e, r, s))
+            assert rel_l2(p - 0.25, q - 0.25) <= 5e-4, (i, dtype, rel_l2(p - 0.25, q - 0.25))
+            assert np.array_equal(d, e)
+            inside = np.zeros((H, W), bool)
+            inside[roi[1]:roi[3], roi[0]:roi[2]] = True
+            assert np.all(r[~inside] == 0.25) and np.all(s[~inside] == 0.25)
+            assert rel_l2(r[inside] - 0.25, q[inside] - 0.25) <= 5e-4 and np.array_equal(s[inside], e[inside])
+    defocus = np.tile(np.array([2900.0, 3100.0, 20.0], np.float32), n)
+    kw = dict(ctf_mode=True, pixel_size_nm=0.27, ctf_slice_thickness_nm=1.9, ctf_beta_fac=(10.0, 0.0, 0.008, 0.0),
+              cut_length=(1.0, 1.0), dim_length=(2.0, 2.0))
+    got = []
+    for variant in (E.VARIANT_FAST, E.VARIANT_FAITHFUL):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=variant, **kw), c["pg"], TILTS, defocus)
+        rec.reset_projections()
+        rec.forward_projection(c["vg"], cuda(c["vol"]), 2)
+        torch.cuda.synchronize()
+        got.append(host(rec.views()[0]).copy())
+        rec.close()
+    assert np.abs(got[1]).max() > 0
+    assert rel_l2(got[0], got[1]) <= 5e-4, rel_l2(got[0], got[1])
+
+
+@pytest.mark.parametrize("dims", [(3, 5, 2), (4, 9, 1), (33, 17, 5), (5, 8, 40)])
+@pytest.mark.parametrize("phi,tilt_x", [(0.02, 0.0), (0.8, 0.0), (0.0, 13.5)])
+def test_declined_beam_small_and_odd(dims, phi, tilt_x):
+    """tilted_sum: rays whose y moves slowly, by nearly nothing and by up to
+    nearly a quarter of a layer per layer (13.5 degrees about the tilt axis'
+    normal; the series' projections beyond take the walk from cell to cell),
+    against the nearer of the oracle's marches (above)."""
+    import torch
+
+    import artiatomi_b200 as E
+    from oracle import driver as D, geometry as G
+
+    W, H, n = 26, 22, len(TILTS)
+    c = _case(dims, 0.0, W, H)
+    psi = np.linspace(-9.0, 11.0, n).astype(np.float32)
+    pg = E.projection_geometry(E.Markers(TILTS, None, None, None, psi), W, H, E.TiltConfig(phi_angle=phi, add_tilt_x_angle=tilt_x))
+    og = G.projection_geometry(TILTS, None, None, None, psi, W, H,
+                               cfg={"phi_angle": phi, "add_tilt_x_angle": tilt_x})
+    for i in range(n):
+        k = E.set_constant_values(pg[i], c["vg"])
+        g = G.orc_geom(og[i], c["vo"])
+        marches = []
+        for precision in (0, 1):
+            p = np.zeros((H, W), np.float32)
+            D.fp_march(g, c["vol"], 0, W, H, p, np.zeros_like(p), precision=precision)
+            marches.append(p)
+        for dtype, tol in ((torch.float32, 5e-4), (torch.float16, 1e-3)):
+            proj, dist = torch.zeros((H, W), device="cuda"), torch.zeros((H, W), device="cuda")
+            E.forward_project(k, cuda(c["vol"]).to(dtype), proj, dist, fast=True)
+            d = [np.abs(host(proj) - p) for p in marches]
+            err = np.linalg.norm(np.minimum(*d)) / np.linalg.norm(marches[1])
+            assert err <= tol, (i, dtype, err)
