@@ -69,7 +69,9 @@ inline AxisStep axis_step(const KConst& c, bool& zmaj, int& sm, int& sn) {
 
 // Whether the warps of the axis kernels span detector columns (u) instead of
 // rows: when a pixel step along u moves the ray less across the volume's y
-// planes than one along v.
+// planes than one along v. 1024 x 1024 x 64 at 84 degrees, where rows cross
+// 8 planes a warp and lose half the lanes: 1905 us with rows, 844 with columns
+// and the walk's other changes (worth 20 % where rows stay in one plane).
 inline int axis_swap(const KConst& c) {
   const float uy = c.aniso[0] * c.u.y + c.aniso[3] * c.v.y, vy = c.aniso[1] * c.u.y + c.aniso[4] * c.v.y;
   return fabsf(uy) < fabsf(vy) ? 1 : 0;

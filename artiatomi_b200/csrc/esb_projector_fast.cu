@@ -6,8 +6,10 @@
 // the interpolation lattice the interpolant is a trilinear polynomial of the
 // cell-local coordinates, and these are linear in j. So the sum over the
 // samples inside a cell has a closed form in the power sums of j. Rays of a
-// single-axis series stay in one y plane and take the branch-free layer walk
-// (layer_sum_xz: one layer of the major axis per step, two cells per layer);
+// single-axis series stay in one y plane and take the layer walk (axis_walk:
+// one layer of the major axis per step, its samples as weights of two rows of
+// voxels; plane_sums the same for a line of rays), rays whose y moves slowly
+// a walk like it (tilted_sum);
 // other rays walk the cells they cross with a 3-D DDA (cell_sum), loading
 // each cell's 8 corners once (4 when it enters through a face shared with
 // the previous cell). Either replaces ~5 trilinear evaluations (40 loads)
@@ -24,6 +26,7 @@
 //
 // One thread per sub-ray. The 4 sub-rays of a pixel sit in adjacent lanes and
 // are combined with warp shuffles.
+#include <algorithm>
 #include <float.h>
 
 #include "esb_axis.cuh"
@@ -261,6 +264,8 @@ __device__ float cell_sum_xz(const Cell<VT>& C, float qx, float b, int iy, float
 // far row's weights are applied before the planes change. Against the walk
 // from cell to cell a step has no case distinction but that one, and reads 8
 // voxels at most where a cell reads 4 to 8 and there are 1.5 cells a layer.
+// What bounds it: instruction issue. 256 x 240 x 96 at 0.8 degrees, 12
+// projections: 4.2 -> 3.05 ms.
 template <int VT>
 __device__ __noinline__ float tilted_sum(const Cell<VT>& C, float qx, float qy, float qz, float dqx, float dqy,
                                          float dqz, int j0, int J) {
@@ -603,7 +608,11 @@ __device__ __forceinline__ float cvt(typename RawVoxel<VT>::T r) {
 // are read only by the lanes whose ray needs them, the next row's loads are
 // in flight during a layer's arithmetic, and layers whose rows and window
 // lie inside the volume and wholly inside the ray take no clamps, no index
-// arithmetic and no end test.
+// arithmetic and no end test. 64 registers and 32 warps per SM: with 80 and
+// 24 warps 974 us where this takes 866.
+// 1024 x 1024 x 64 FP32, one projection, against the sums of the interpolant
+// per cell that it replaces: in-plane rotation 0.2 degrees, tilts 0 / 24 /
+// -40 / -50: 1090 / 1047 / 926 / 1046 -> 866 / 854 / 772 / 922 us.
 template <int VT, bool ZMAJ, int SM, int SN, class Off>
 __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C, float Mq, float Nq, float b, int iy,
                                            int j0, int J) {
@@ -771,13 +780,35 @@ __device__ __noinline__ float other_ray_sum(const KConst* c, const void* vol, fl
   return ray_sum<VT, unsigned long long>(*c, C, s, t0, tout, first_at_source);
 }
 
+// First sample of run `seg` of J samples in `segs` runs.
+__device__ __forceinline__ int run_start(int J, int seg, int segs) { return (int)((long long)J * seg / segs); }
+
+// A block's warps in groups of `segs` that sum one run of the same rays each:
+// adds the group's sums in the runs' order, valid in its first warp.
+template <int N>
+__device__ __forceinline__ void sum_runs(float (&v)[N], int segs) {
+  __shared__ float part[8][N][32];
+  if (segs == 1) return;  // uniform
+  const int w = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31), seg = w & (segs - 1);
+#pragma unroll
+  for (int i = 0; i < N; ++i) part[w][i][lane] = v[i];
+  __syncthreads();
+  if (seg == 0)
+    for (int r = 1; r < segs; ++r)
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] += part[w + r][i][lane];
+}
+
 // Sum over the samples of one sub-ray from t0 to tout (ray_sum) with the
 // axis walk when the ray fits the launch's instance (its y in one cell, its
 // step the launch's), else other_ray_sum. With first_at_source the first
-// sample is the one at the ray's start, whose value is `source`.
+// sample is the one at the ray's start, whose value is `source`. seg, segs:
+// without first_at_source the samples are cut into `segs` runs, and this is
+// the sum over run `seg`.
 template <int VT, bool ZMAJ, int SM, int SN, class Off>
 __device__ __forceinline__ float axis_ray_sum(const KConst& c, const AxisStep& A, const Cell<VT>& C, float3 s,
-                                              float t0, float tout, bool first_at_source, float source) {
+                                              float t0, float tout, bool first_at_source, float source, int seg,
+                                              int segs) {
   if (!(t0 <= tout)) return 0.0f;
   const float h = c.vs.x * 0.15f;
   float step;
@@ -788,26 +819,28 @@ __device__ __forceinline__ float axis_ray_sum(const KConst& c, const AxisStep& A
   const float ylast = qpos(q0.y, J - 1, dqy);
   const float fy = floorf(q0.y);
   if (!(ok && step == A.step && fabsf(dqy) * (float)J < 1e-5f && fy == floorf(ylast)))
-    return other_ray_sum<VT>(&c, C.vol, s, t0, tout, first_at_source);
+    return seg == 0 ? other_ray_sum<VT>(&c, C.vol, s, t0, tout, first_at_source) : 0.0f;
   const float sum = first_at_source ? source : 0.0f;
-  const int j0 = first_at_source ? 1 : 0;
-  if (j0 >= J) return sum;
+  const int j0 = first_at_source ? 1 : run_start(J, seg, segs), j1 = first_at_source ? J : run_start(J, seg + 1, segs);
+  if (j0 >= j1) return sum;
   const float qm = ZMAJ ? q0.z : q0.x, qn = ZMAJ ? q0.x : q0.z;
-  return sum + axis_walk<VT, ZMAJ, SM, SN, Off>(A, C, SM > 0 ? qm : -qm, SN > 0 ? qn : -qn, q0.y - fy, (int)fy, j0, J);
+  return sum + axis_walk<VT, ZMAJ, SM, SN, Off>(A, C, SM > 0 ? qm : -qm, SN > 0 ? qn : -qn, q0.y - fy, (int)fy, j0, j1);
 }
 
 // Pixel of a thread in the axis kernels: the 4 sub-rays of a pixel in
 // adjacent lanes, a warp spans 8 pixels along the detector axis that crosses
 // the tilt axis (v, or u when `swap`), so that its rays lie in few y planes;
-// the warps of a block step along the other axis.
+// the warps of a block step along the other axis, `segs` warps (a power of
+// two) for the same pixels.
 struct AxisPixel {
-  int sub, x, y;
+  int sub, x, y, seg;
   bool active;
-  __device__ __forceinline__ AxisPixel(int swap, int x0, int y0, int x1, int y1) {
+  __device__ __forceinline__ AxisPixel(int swap, int segs, int x0, int y0, int x1, int y1) {
     const int lane = threadIdx.x & 31;
     sub = lane & 3;
     const int along = (int)blockIdx.y * 8 + (lane >> 2);
-    const int across = (int)blockIdx.x * (blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    const int w = (int)blockIdx.x * (blockDim.x >> 5) + (int)(threadIdx.x >> 5), across = w / segs;
+    seg = w - across * segs;
     x = x0 + (swap ? along : across);
     y = y0 + (swap ? across : along);
     active = x < x1 && y < y1;
@@ -818,9 +851,9 @@ struct AxisPixel {
 template <int VT, bool ZMAJ, int SM, int SN, class Off>
 __global__ void __launch_bounds__(256, 4) k_project_axis(const __grid_constant__ KConst c, const __grid_constant__ AxisStep A,
                                                       const void* __restrict__ vol, float* __restrict__ proj,
-                                                      float* __restrict__ dist, size_t pitchE, int swap, int x0,
-                                                      int y0, int x1, int y1) {
-  const AxisPixel P(swap, x0, y0, x1, y1);
+                                                      float* __restrict__ dist, size_t pitchE, int swap, int segs,
+                                                      int x0, int y0, int x1, int y1) {
+  const AxisPixel P(swap, segs, x0, y0, x1, y1);
   Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
   float sum = 0.0f, gx = 0.0f, gz = 0.0f;
   if (P.active) {
@@ -831,17 +864,26 @@ __global__ void __launch_bounds__(256, 4) k_project_axis(const __grid_constant__
     if (tout - tin > 0.0f) {
       gx = 1.0f;
       gz = tout - tin;
-      sum = axis_ray_sum<VT, ZMAJ, SM, SN, Off>(c, A, C, s, tin, tout, false, 0.0f);
+      sum = axis_ray_sum<VT, ZMAJ, SM, SN, Off>(c, A, C, s, tin, tout, false, 0.0f, P.seg, segs);
     }
   }
-  sum = quad_sum_ordered(sum);
+  float runs[1] = {sum};
+  sum_runs(runs, segs);
+  sum = quad_sum_ordered(runs[0]);
   gx = quad_sum_ordered(gx);
   gz = quad_sum_ordered(gz);
-  if (P.active && P.sub == 0) {
+  if (P.active && P.sub == 0 && P.seg == 0) {
     const size_t i = (size_t)P.y * pitchE + P.x;
     proj[i] += sum * c.vs.x * 0.15f * 0.25f;
     dist[i] = fmaxf(0.0f, gz / gx);
   }
+}
+
+// The slabs ka .. kb - 1 of wlo .. whi that this block of gridDim.z walks.
+__device__ __forceinline__ void slab_part(int wlo, int whi, int& ka, int& kb) {
+  const int n = max(whi - wlo + 1, 0), z = (int)blockIdx.z, nz = (int)gridDim.z;
+  ka = wlo + n * z / nz;
+  kb = wlo + n * (z + 1) / nz;
 }
 
 // k_slicer_fused for single-axis series; pixels as k_project_axis. The
@@ -851,7 +893,7 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
                                                      const void* __restrict__ vol, float* __restrict__ imgs,
                                                      size_t img_stride, size_t pitchE, SlabTable slabs, int clear,
                                                      int swap, int x0, int y0, int x1, int y1) {
-  const AxisPixel P(swap, x0, y0, x1, y1);
+  const AxisPixel P(swap, 1, x0, y0, x1, y1);
   Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
   float3 s = make_float3(0.f, 0.f, 0.f);
   float tin = 0.f, tout = -1.f, source = 0.f;
@@ -885,16 +927,18 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
     whi = max(whi, __shfl_xor_sync(0xffffffffu, whi, o));
   }
   const size_t pix = (size_t)P.y * pitchE + P.x;
-  for (int k = wlo; k <= whi; ++k) {
+  int ka, kb;
+  slab_part(wlo, whi, ka, kb);
+  for (int k = ka; k < kb; ++k) {
     float v = 0.0f;
     if (hitray && k >= klo && k <= khi)
       v = axis_ray_sum<VT, ZMAJ, SM, SN, Off>(c, A, C, s, fmaxf(tin, slabs.bound[k]), fminf(tout, slabs.bound[k + 1]),
-                                              true, source);
+                                              true, source, 0, 1);
     v = quad_sum_ordered(v);
     if (P.active && P.sub == 0 && k >= klo && k <= khi)
       imgs[(size_t)k * img_stride + pix] = v * c.vs.x * 0.15f * 0.25f;
   }
-  if (clear && P.active && P.sub == 0) clear_slabs(imgs + pix, img_stride, slabs.count, klo, khi);
+  if (clear && blockIdx.z == 0 && P.active && P.sub == 0) clear_slabs(imgs + pix, img_stride, slabs.count, klo, khi);
 }
 
 // ---------------------------------------------------------------------------
@@ -917,27 +961,31 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
 // ray's float start point (5e-4 voxels, all samples) makes.
 //
 // Per ray and layer that leaves a 2 G-th of the weights, control and loads
-// of each plane in place of all of them for two planes. A warp holds 16
+// of each plane in place of all of them for two planes. What bounds it: the
+// latency of a layer's loads at 12 to 16 warps per SM (issue 52 % busy, FMA
+// pipe 35 %); caps of 96 and 80 registers (20 and 24 warps) spill and took
+// 33.5 and 44.3 ms where 128 take 33.3. 1024 x 1024 x 256, 16 tilts with 0.3
+// degrees jitter, CTF slabs: 61.1 ms with k_slicer_axis -> 33.3; 256 x 256 x
+// 128, 41 tilts: 7.3 ms with k_project_axis -> 3.2 (4 runs). A warp holds 16
 // detector rows x 2 sub-rows, so that its loads of a plane are contiguous.
 // `swap` exchanges u and v (a tilt axis across the image).
 struct PlaneWalk {
   int sM, sN;          // step signs
   int nM, nN;          // voxels along the major and minor axis
-  unsigned dM, dN;     // their element strides
+  unsigned dM, dN;     // their strides in bytes
 };
 constexpr float kMaxShear = 1.0f / 64.0f;
 
 // Plane sums over samples j0 .. J-1 of one ray: S[0] of the weights, and with
 // SH > 0 S[1], S[2] of their derivatives along the mirrored minor and major
-// axis, with SH > 1 S[3] of the mixed one; yoff: element offsets of the
-// planes.
+// axis, with SH > 1 S[3] of the mixed one; yoff: byte offsets of the planes
+// (32-bit: the volume is below 4 GiB).
 template <int VT, int NP, int SH>
 __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W, const void* __restrict__ vol,
                                            const unsigned (&yoff)[NP], float Mq, float Nq, int j0, int J,
                                            float (&S)[SH == 0 ? 1 : SH + 2][NP]) {
   constexpr int NS = SH == 0 ? 1 : SH + 2;
   typedef typename RawVoxel<VT>::T Raw;
-  constexpr int ES = VT == ESB_VOXEL_F32 ? 4 : 2;
   const char* const base = (const char*)vol;
   const float fj0 = (float)j0, jb = fj0 - 0.5f;
   const float pM = __fmaf_rn(fj0, A.dM, Mq), pN = __fmaf_rn(fj0, A.dN, Nq);
@@ -959,18 +1007,20 @@ __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W
 #pragma unroll
     for (int p = 0; p < NP; ++p) S[q][p] = 0.f;
   }
-  auto row = [&](const float (&w)[NS][4], bool first, bool last) {
+  Raw vb[NP], vc[NP];
+  auto load_row = [&](bool first, bool last) {
     const unsigned r = (unsigned)min(max(im, 0), W.nM - 1) * W.dM;
     auto col = [&](int n) { return r + (unsigned)min(max(n, 0), W.nN - 1) * W.dN; };
     const unsigned oa = col(in - W.sN), ob = col(in), oc = col(in + W.sN), od = col(in + 2 * W.sN);
-    Raw vb[NP], vc[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      vb[p] = ldraw<VT>(base + (size_t)ES * (ob + yoff[p]));
-      vc[p] = ldraw<VT>(base + (size_t)ES * (oc + yoff[p]));
-      ldraw_if<VT>(va[p], base + (size_t)ES * (oa + yoff[p]), first);
-      ldraw_if<VT>(vd[p], base + (size_t)ES * (od + yoff[p]), last);
+      vb[p] = ldraw<VT>(base + (ob + yoff[p]));
+      vc[p] = ldraw<VT>(base + (oc + yoff[p]));
+      ldraw_if<VT>(va[p], base + (oa + yoff[p]), first);
+      ldraw_if<VT>(vd[p], base + (od + yoff[p]), last);
     }
+  };
+  auto add_row = [&](const float (&w)[NS][4]) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const float a = cvt<VT>(va[p]), b = cvt<VT>(vb[p]), c = cvt<VT>(vc[p]), d = cvt<VT>(vd[p]);
@@ -987,6 +1037,7 @@ __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W
   for (int guard = 0; guard < 1 << 20; ++guard) {
     const float nMs = __fmaf_rn(k, A.isM, nM0), nNs = __fmaf_rn(kn, A.isN, nN0);
     const bool X = nNs <= nMs;
+    load_row(Xp, X);  // in flight during the weights' arithmetic
     const float tL = fminf(nMs, Mt);
     const float2 f = ceil2(fminf(nNs, tL), tL);
     const float MA = f.x - fm0, MB = f.y - f.x;
@@ -1022,7 +1073,7 @@ __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W
       w[q][2] = g[q][2] + n[q][1];
       w[q][3] = n[q][2];
     }
-    row(w, Xp, X);
+    add_row(w);
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       g[q][0] = X ? far[q][0] : 0.f;
@@ -1047,7 +1098,8 @@ __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W
     w[q][0] = g[q][0], w[q][1] = g[q][1], w[q][2] = g[q][2];
     w[q][3] = 0.f;
   }
-  row(w, Xp, false);
+  load_row(Xp, false);
+  add_row(w);
 }
 
 // One thread's line of 2 G sub-rays (kept in local memory, read a few times
@@ -1091,8 +1143,9 @@ struct PlaneLine {
 #pragma unroll 1
     for (int g = 0; g < N; ++g) cell[g] -= p0;
     const int ny = (int)c.dim.y, nx = (int)c.dim.x;
+    constexpr unsigned ES = VT == ESB_VOXEL_F32 ? 4 : 2;
 #pragma unroll
-    for (int p = 0; p < NP; ++p) yoff[p] = (unsigned)min(max(p0 + p, 0), ny - 1) * (unsigned)nx;
+    for (int p = 0; p < NP; ++p) yoff[p] = (unsigned)min(max(p0 + p, 0), ny - 1) * (unsigned)nx * ES;
   }
 };
 
@@ -1114,13 +1167,13 @@ struct PlaneRay {
 };
 
 // Sums v[] of the line's sub-rays, each over its [tin, tout] cut to [lo, hi]
-// (0 for those outside). slab: the first sample is the one at the ray's start.
+// (0 for those outside). slab: the first sample is the one at the ray's
+// start; else run `seg` of `segs` of the samples (axis_ray_sum).
 template <int VT, int G, int SH>
 __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, const PlaneWalk& W, int zmaj,
                                           const void* vol, const PlaneLine<G>& L, const unsigned (&yoff)[G + 2],
-                                          bool slab, float lo, float hi, float* v) {
+                                          bool slab, float lo, float hi, int seg, int segs, float* v) {
   constexpr int N = 2 * G, NP = G + 2, NS = SH == 0 ? 1 : SH + 2;
-  const int j0 = slab ? 1 : 0;
   float S[NS][NP];
 #pragma unroll
   for (int q = 0; q < NS; ++q)
@@ -1138,8 +1191,9 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
     bm = zmaj ? R.q.z : R.q.x;
     bn = zmaj ? R.q.x : R.q.z;
   }
-  if (mid && j0 < Jm)
-    plane_sums<VT, NP, SH>(A, W, vol, yoff, W.sM > 0 ? bm : -bm, W.sN > 0 ? bn : -bn, j0, Jm, S);
+  const int j0 = slab ? 1 : run_start(Jm, seg, segs), j1 = slab ? Jm : run_start(Jm, seg + 1, segs);
+  if (mid && j0 < j1)
+    plane_sums<VT, NP, SH>(A, W, vol, yoff, W.sM > 0 ? bm : -bm, W.sN > 0 ? bn : -bn, j0, j1, S);
   float P[NS][NP];  // (indexed by a ray's planes: local memory)
 #pragma unroll
   for (int q = 0; q < NS; ++q)
@@ -1156,7 +1210,7 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
     const bool joins = mid && R.ok && L.cell[g] <= G && abs(R.J - Jm) <= 1 &&
                        (SH == 0 ? e == 0.f && f == 0.f : fabsf(e) <= kMaxShear && fabsf(f) <= kMaxShear);
     if (!joins) {
-      v[g] = other_ray_sum<VT>(&c, vol, L.s[g], t0, t1, slab);
+      if (seg == 0) v[g] = other_ray_sum<VT>(&c, vol, L.s[g], t0, t1, slab);
       continue;
     }
     float sum[2];
@@ -1168,25 +1222,26 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
       if constexpr (SH > 1) sum[h] = fmaf(e * f, P[3][p], sum[h]);
     }
     float r = fmaf(L.b[g], sum[1], (1.0f - L.b[g]) * sum[0]);
-    if (R.J != Jm) {  // one sample more or less than the middle ray
+    if (R.J != Jm && seg == segs - 1) {  // one sample more or less than the middle ray
       const int j = min(R.J, Jm);
       const Cell<VT> C{vol, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z, (long)c.dim.x, (long)c.dim.x * (long)c.dim.y};
       const float last = trilinear<VT>(C, qpos(R.q.x, j, R.dq.x), qpos(R.q.y, j, R.dq.y), qpos(R.q.z, j, R.dq.z));
-      if (j >= j0) r += R.J > Jm ? last : -last;
+      if (j >= (slab ? 1 : 0)) r += R.J > Jm ? last : -last;
     }
     v[g] = slab ? r + L.source[g] : r;
   }
 }
 
 // Pixels of a thread: G along u (v with swap) from x, y; a lane pair shares
-// them, one sub-row each.
+// them, one sub-row each, and `segs` warps the same.
 template <int G>
 struct PlanePixel {
-  int x, y;
+  int x, y, seg;
   bool active;
-  __device__ __forceinline__ PlanePixel(int swap, int x0, int y0, int x1, int y1) {
+  __device__ __forceinline__ PlanePixel(int swap, int segs, int x0, int y0, int x1, int y1) {
     const int lane = threadIdx.x & 31;
-    const int across = G * (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    const int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), across = G * (w / segs);
+    seg = w % segs;
     const int along = (int)blockIdx.y * 16 + (lane >> 1);
     x = x0 + (swap ? along : across);
     y = y0 + (swap ? across : along);
@@ -1204,19 +1259,23 @@ __device__ __forceinline__ float pixel_sum(const float* v, int i, int swap) {
 template <int VT, int G, int SH>
 __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ KConst c,
                                                         const __grid_constant__ AxisStep A,
-                                                        const __grid_constant__ PlaneWalk W, int zmaj, int swap,
+                                                        const __grid_constant__ PlaneWalk W, int zmaj, int swap, int segs,
                                                         const void* __restrict__ vol, float* __restrict__ proj,
                                                         float* __restrict__ dist, size_t pitchE, int x0, int y0,
                                                         int x1, int y1) {
-  const PlanePixel<G> P(swap, x0, y0, x1, y1);
+  const PlanePixel<G> P(swap, segs, x0, y0, x1, y1);
   PlaneLine<G> L;
   unsigned yoff[G + 2];
   float v[2 * G];
   L.in = 0;
   if (P.active) {
     L.template init<VT>(c, vol, P.x, P.y, swap, false, yoff);
-    line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, false, -FLT_MAX, FLT_MAX, v);
+    line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, false, -FLT_MAX, FLT_MAX, P.seg, segs, v);
+  } else {
+#pragma unroll
+    for (int g = 0; g < 2 * G; ++g) v[g] = 0.0f;
   }
+  sum_runs(v, segs);
 #pragma unroll 1
   for (int i = 0; i < G; ++i) {
     float n[2], d[2];
@@ -1230,7 +1289,7 @@ __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ 
     }
     const float sum = pixel_sum(v, i, swap), gx = pixel_sum(n, 0, swap), gz = pixel_sum(d, 0, swap);
     const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
-    if (P.active && !(threadIdx.x & 1) && x < x1 && y < y1) {
+    if (P.active && P.seg == 0 && !(threadIdx.x & 1) && x < x1 && y < y1) {
       const size_t o = (size_t)y * pitchE + x;
       proj[o] += sum * c.vs.x * 0.15f * 0.25f;
       dist[o] = fmaxf(0.0f, gz / gx);
@@ -1246,7 +1305,7 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
                                                        size_t img_stride, size_t pitchE,
                                                        const __grid_constant__ SlabTable slabs, int clear, int x0,
                                                        int y0, int x1, int y1) {
-  const PlanePixel<G> P(swap, x0, y0, x1, y1);
+  const PlanePixel<G> P(swap, 1, x0, y0, x1, y1);
   PlaneLine<G> L;
   unsigned yoff[G + 2];
   L.in = 0;
@@ -1278,10 +1337,12 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
     whi = max(whi, __shfl_xor_sync(0xffffffffu, whi, o));
   }
   const bool writer = P.active && !(threadIdx.x & 1);
-  for (int k = wlo; k <= whi; ++k) {
+  int ka, kb;
+  slab_part(wlo, whi, ka, kb);
+  for (int k = ka; k < kb; ++k) {
     float v[2 * G];
     if (L.in) {
-      line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, true, slabs.bound[k], slabs.bound[k + 1], v);
+      line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, true, slabs.bound[k], slabs.bound[k + 1], 0, 1, v);
     } else {
 #pragma unroll
       for (int g = 0; g < 2 * G; ++g) v[g] = 0.f;
@@ -1294,7 +1355,7 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
         imgs[(size_t)k * img_stride + (size_t)y * pitchE + x] = sum * c.vs.x * 0.15f * 0.25f;
     }
   }
-  if (clear && writer) {
+  if (clear && blockIdx.z == 0 && writer) {
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
@@ -1303,13 +1364,31 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
   }
 }
 
+// Parts that each ray is cut into, up to max_parts, for `warps` warps to
+// become `full`, the warps that the GPU holds at once: a small launch waits
+// for the loads of one layer after the other (64 x 64 x 32: 15.4 us a
+// projection with whole rays, 9.6 in 4 runs).
+int parts_for(double warps, double full, int max_parts) {
+  return std::max(1, std::min(max_parts, (int)(full / warps + 0.5)));
+}
+
+// Runs that a ray's samples may be cut into: at least 8 layers in each, a
+// power of two up to `most`.
+int max_runs(const KConst& c, bool zmaj, int most) {
+  int n = 1;
+  while (2 * n <= most && 16 * n <= (int)(zmaj ? c.dim.z : c.dim.x)) n *= 2;
+  return n;
+}
+
 // The plane kernels' launch: G pixels per thread (0: not taken), whether the
 // line's rays differ in y only.
 struct PlaneLaunch {
-  int G = 0, shear = 0, swap = 0, zmaj = 0;
+  int G = 0, parts = 1, shear = 0, swap = 0, zmaj = 0;
   AxisStep A;
   PlaneWalk W;
-  PlaneLaunch(const KConst& c, int w, int h) {
+  // runs: how often a ray's samples may be cut into runs; max_parts: parts of
+  // either kind, runs or slabs
+  PlaneLaunch(const KConst& c, int vt, int w, int h, int runs, int max_parts) {
     bool z;
     int sm, sn;
     A = axis_step(c, z, sm, sn);
@@ -1328,19 +1407,24 @@ struct PlaneLaunch {
       // the ray to the volume's face, and its planes
       const bool small = (float)g * (ex + ez) <= kMaxShear;
       const bool planes = (float)(2 * g - 1) * ey < (float)g - 0.05f;
-      // 2 pixels per thread from 2 warps per scheduler on, 4 from 4 (measured:
-      // 128 warps of 2 pixels 25 us against the axis walk's 15, 2048 warps 113
-      // against 178; 1024 warps of 4 pixels 141 against the 113 of 2)
-      const bool enough = (double)((across + g - 1) / g) * ((along + 15) / 16) >= 148.0 * 4 * g;
+      // 2 pixels per thread from 2 warps per scheduler on, 4 from 4, runs
+      // counted. Measured without runs: 128 warps of 2 pixels 25 us against
+      // the axis walk's 15, 2048 warps 113 against 178, 1024 warps of 4
+      // pixels 141, and with 4 runs 78. Slabs do not count: they are few
+      // layers each, and 1024 warps of 4 pixels with their slabs spread took
+      // 105 us where 2048 of 2 pixels take 72.
+      const double warps = (double)((across + g - 1) / g) * ((along + 15) / 16);
+      const bool enough = warps * runs >= 148.0 * 4 * g;
+      parts = parts_for(warps, 148.0 * 16, max_parts);
       if (small && planes && enough) G = g;
     }
-    const unsigned sz = (unsigned)c.dim.x * (unsigned)c.dim.y;
+    const unsigned es = vt == ESB_VOXEL_F32 ? 4 : 2, sz = es * (unsigned)c.dim.x * (unsigned)c.dim.y;
     W.sM = sm;
     W.sN = sn;
     W.nM = (int)(z ? c.dim.z : c.dim.x);
     W.nN = (int)(z ? c.dim.x : c.dim.z);
-    W.dM = z ? sz : 1;
-    W.dN = z ? 1 : sz;
+    W.dM = z ? sz : es;
+    W.dN = z ? es : sz;
   }
 };
 
@@ -1384,7 +1468,8 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
 #define ESB_PLANES_LAUNCH()                                                                          \
   do {                                                                                               \
     const int along = L.swap ? x1 - x0 : y1 - y0, across = L.swap ? y1 - y0 : x1 - x0;                \
-    const dim3 blk(128), grd((across + 4 * L.G - 1) / (4 * L.G), (along + 15) / 16);                  \
+    const int cols = 4 / segs * L.G; /* across a block of 4 warps */                                  \
+    const dim3 blk(128), grd((across + cols - 1) / cols, (along + 15) / 16, slab_parts);              \
     if (vt == ESB_VOXEL_F32) ESB_PLANES_VT(ESB_VOXEL_F32);                                           \
     else if (vt == ESB_VOXEL_F16) ESB_PLANES_VT(ESB_VOXEL_F16);                                      \
     else ESB_PLANES_VT(ESB_VOXEL_BF16);                                                              \
@@ -1392,7 +1477,8 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
     return cudaGetLastError();                                                                       \
   } while (0)
 
-// Volumes below 4 GiB take 32-bit byte offsets in the axis walk.
+// Volumes below 4 GiB take 32-bit byte offsets in the axis walk (an address
+// is one addition instead of a 64-bit one and its carries).
 #define ESB_AXIS_LAUNCH(KER, GRD, BLK, ST, ...)                                                                \
   do {                                                                                                        \
     const double bytes_ = (double)c.dim.x * c.dim.y * c.dim.z * (vt == ESB_VOXEL_F32 ? 4.0 : 2.0);            \
@@ -1411,8 +1497,9 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
                                 size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1,
                                 int y1, cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0 || slabs.count <= 0) return cudaSuccess;
-  const PlaneLaunch L(c, x1 - x0, y1 - y0);
+  const PlaneLaunch L(c, vt, x1 - x0, y1 - y0, 1, slabs.count);
   if (L.G) {
+    const int segs = 1, slab_parts = L.parts;
 #define ESB_PLANES(VT, GG, SH)                                                                                        \
   k_slicer_planes<VT, GG, SH ? 2 : 0><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, imgs, img_stride, pitchE, \
                                                            slabs, clear, x0, y0, x1, y1)
@@ -1422,7 +1509,8 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
   if (axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
-    const dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
+    dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
+    grd.z = parts_for((double)grd.x * grd.y * nw, 148.0 * 32, slabs.count);
     ESB_AXIS_LAUNCH(k_slicer_axis, grd, blk, st, vol, imgs, img_stride, pitchE, slabs, clear, swap, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();
@@ -1452,18 +1540,28 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
                                 size_t pitchE, float tmin, float tmax, int x0, int y0, int x1, int y1,
                                 cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
-  const PlaneLaunch L(c, x1 - x0, y1 - y0);
+  bool zmaj;
+  int sm, sn;
+  axis_step(c, zmaj, sm, sn);
+  const PlaneLaunch L(c, vt, x1 - x0, y1 - y0, max_runs(c, zmaj, 4), 4);
   if (mode == 0 && L.G) {
+    const int segs = max_runs(c, zmaj, L.parts), slab_parts = 1;
 #define ESB_PLANES(VT, GG, SH) \
-  k_project_planes<VT, GG, SH><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, proj, dist, pitchE, x0, y0, x1, y1)
+  k_project_planes<VT, GG, SH><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, segs, vol, proj, dist, pitchE, x0, y0, x1, y1)
     ESB_PLANES_LAUNCH();
 #undef ESB_PLANES
   }
   if (mode == 0 && axis_projection(c)) {  // the axis walk, one sub-ray per thread
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
-    const dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    ESB_AXIS_LAUNCH(k_project_axis, grd, blk, st, vol, proj, dist, pitchE, swap, x0, y0, x1, y1);
+    dim3 grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
+    const int segs = max_runs(c, zmaj, parts_for((double)grd.x * grd.y * nw, 148.0 * 32, 8));
+    if (segs > 1) {
+      nw = 8;
+      grd = axis_grid(swap, nw / segs, x1 - x0, y1 - y0);
+    }
+    const dim3 blk(32 * nw);
+    ESB_AXIS_LAUNCH(k_project_axis, grd, blk, st, vol, proj, dist, pitchE, swap, segs, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();
   }
