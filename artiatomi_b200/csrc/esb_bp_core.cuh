@@ -563,7 +563,12 @@ struct UpGeom {
   int smax, fmax;         // last sample that is read, per axis
   int pitch;              // samples per slow step
   int swapped;            // fast axis u
+  int fits;               // at most up_columns(os) samples of a shadow along the fast axis
 };
+
+// Samples along the fast axis that grid_sums takes together (NC): a shadow is
+// at most 1.42 os wide with the tilt axis along the slow one.
+inline int up_columns(int os) { return os == 1 ? 2 : 3; }
 
 // Fast axis u: a step in x moves the projection further along u than along v.
 inline bool up_swapped(const AxisGeom& a) { return fabsf(a.U.x) > fabsf(a.V.x); }
@@ -588,6 +593,9 @@ inline UpGeom make_up_geom(const KConst& k, const AxisGeom& a, int pw, int ph, i
   g.dfx = (float)f[1];
   g.hs = (g.swapped ? a.hv : a.hu) * os;
   g.hf = (g.swapped ? a.hu : a.hv) * os;
+  // (the samples taken together end within one of the shadow's end: the reach
+  // that a sub-volume's patch is planned with)
+  g.fits = 2.0f * g.hf < (float)up_columns(os) && 2.0f * g.hf >= (float)up_columns(os) - 1.0f && 2.0f * g.hs >= 1.0f;
   const double scale = (double)a.K / a.L0 / os;
   g.ws = (float)((g.swapped ? a.wv : a.wu) * scale);
   g.wf = (float)((g.swapped ? a.wu : a.wv) * scale);
@@ -603,53 +611,89 @@ inline UpGeom make_up_geom(const KConst& k, const AxisGeom& a, int pw, int ph, i
 // sum(sample * chord) and sum(chord) of one voxel whose centre lies at (s, f)
 // relative to a sample of the grid, over the samples of its shadow within
 // [slo, shi] x [flo, fhi] (relative too); on = false: none. at(is, jf, ..)
-// gives the reader of relative sample (is, jf): reader.load(r, j, take) the
-// sample r slow and j fast steps on, read where `take`;
+// gives the reader of relative sample (is, jf): reader.fetch(r, j) the
+// sample r slow and j fast steps on, reader.load(r, j, take) the same, read
+// where `take`;
 // reader.mine(t, r, j, taken) whether it counts for the voxel's row,
 // reader.value(t) its value.
 //
-// What bounds it: instruction issue, and the latency of the samples' loads.
-// The bounds are rounded by additions to 1.5 * 2^23 whose bits are the
-// integers (no conversions), the chord is one saturating addition, and the
-// row test predicates the two accumulations: about 6 instructions a sample.
-// The first 2 x NC samples are loaded under predicates before any is used,
-// so that their loads are in flight together.
+// What bounds it: instruction issue (the ALU pipe first), and the latency of
+// the samples' loads. The bounds are rounded by additions to 1.5 * 2^23 whose
+// bits are the integers (no conversions), the chord is one saturating
+// addition, and the row test predicates the two accumulations: about 6
+// instructions a sample.
+// Where no limit is near, the first 2 x NC samples are taken as they are: one
+// outside the shadow has no chord or another row (g.fits: the shadow is at
+// most NC samples wide). Elsewhere, at the image's edges and in clipped
+// rectangles, each is read under a predicate (branches around each load made
+// the whole kernel 18 % slower).
+// 1024 x 1024 x 256, oversampling 2, 16 tilts: 32.0 ms before, 30.0 with
+// predicates, 30.1 with the plain reads; 256 x 256 x 128, oversampling 1, 41
+// tilts: 2.13 -> 2.02 ms.
 template <int NC, class At>
 __device__ __forceinline__ void grid_sums(const UpGeom& g, float s, float f, float slo, float shi, float flo,
                                           float fhi, bool on, const At& at, float& acc, float& dacc) {
   const float big = 12582912.0f;  // 1.5 * 2^23, bits 0x4B400000
-  const float sa = fmaxf(__fadd_ru(s - g.hs, big), big + slo), sb = fminf(__fadd_rd(s + g.hs, big), big + shi);
-  const float fa = fmaxf(__fadd_ru(f - g.hf, big), big + flo), fb = fminf(__fadd_rd(f + g.hf, big), big + fhi);
-  const float nf = fb - fa, ns = on && nf >= 0.f ? sb - sa : -1.f;  // samples - 1 per axis
-  const float w = fmaf((sa - big) - s, g.ws, __fmul_rn((fa - big) - f, g.wf));
-  const auto reader = at(__float_as_int(sa) - 0x4B400000, __float_as_int(fa) - 0x4B400000, sa - big, fa - big);
-  typename std::remove_const<decltype(reader)>::type::Raw t[2][NC];
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int j = 0; j < NC; ++j) t[r][j] = reader.load(r, j, ns >= (float)r && nf >= (float)j);
+  const float sc = __fadd_ru(s - g.hs, big), fc = __fadd_ru(f - g.hf, big);
   float a = 0.f, da = 0.f;
-  auto add = [&](const auto& u, int r, int j, bool taken, float ww) {
+  auto add = [&](const auto& u, const auto& reader, int r, int j, bool taken, float ww) {
     const float L = __saturatef(g.c - fabsf(ww));
     if (reader.mine(u, r, j, taken)) {
       a = fmaf(reader.value(u), L, a);
       da += L;
     }
   };
+  auto first = [&](float sa, float fa) {
+    return at(__float_as_int(sa) - 0x4B400000, __float_as_int(fa) - 0x4B400000, sa - big, fa - big);
+  };
+  typedef typename std::remove_const<decltype(first(sc, fc))>::type Reader;
+  if (on && g.fits && sc >= big + slo && sc < big + shi && fc >= big + flo && fc <= big + (fhi - (float)(NC - 1))) {
+    const Reader reader = first(sc, fc);
+    const float w = fmaf((sc - big) - s, g.ws, __fmul_rn((fc - big) - f, g.wf));
+    typename Reader::Raw t[2][NC];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const float wr = r ? w + g.ws : w;
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int j = 0; j < NC; ++j) add(t[r][j], r, j, ns >= (float)r && nf >= (float)j, j ? fmaf((float)j, g.wf, wr) : wr);
-    if (nf >= (float)NC && ns >= (float)r)
+      for (int j = 0; j < NC; ++j) t[r][j] = reader.fetch(r, j);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float wr = r ? w + g.ws : w;
+#pragma unroll
+      for (int j = 0; j < NC; ++j) add(t[r][j], reader, r, j, true, j ? fmaf((float)j, g.wf, wr) : wr);
+    }
+    const float ns = fminf(__fadd_rd(s + g.hs, big), big + shi) - sc;
 #pragma unroll 1
-      for (int j = NC; (float)j <= nf; ++j) add(reader.load(r, j, true), r, j, true, fmaf((float)j, g.wf, wr));
+    for (int r = 2; (float)r <= ns; ++r)
+#pragma unroll
+      for (int j = 0; j < NC; ++j)
+        add(reader.fetch(r, j), reader, r, j, true, fmaf((float)j, g.wf, fmaf((float)r, g.ws, w)));
+  } else if (on) {
+    const float sa = fmaxf(sc, big + slo), sb = fminf(__fadd_rd(s + g.hs, big), big + shi);
+    const float fa = fmaxf(fc, big + flo), fb = fminf(__fadd_rd(f + g.hf, big), big + fhi);
+    const float nf = fb - fa, ns = nf >= 0.f ? sb - sa : -1.f;  // samples - 1 per axis
+    const float w = fmaf((sa - big) - s, g.ws, __fmul_rn((fa - big) - f, g.wf));
+    const Reader reader = first(sa, fa);
+    typename Reader::Raw t[2][NC];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) t[r][j] = reader.load(r, j, ns >= (float)r && nf >= (float)j);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float wr = r ? w + g.ws : w;
+#pragma unroll
+      for (int j = 0; j < NC; ++j)
+        add(t[r][j], reader, r, j, ns >= (float)r && nf >= (float)j, j ? fmaf((float)j, g.wf, wr) : wr);
+      if (nf >= (float)NC && ns >= (float)r)
+#pragma unroll 1
+        for (int j = NC; (float)j <= nf; ++j) add(reader.fetch(r, j), reader, r, j, true, fmaf((float)j, g.wf, wr));
+    }
+#pragma unroll 1
+    for (int r = 2; (float)r <= ns; ++r)
+#pragma unroll 1
+      for (int j = 0; (float)j <= nf; ++j)
+        add(reader.fetch(r, j), reader, r, j, true, fmaf((float)j, g.wf, fmaf((float)r, g.ws, w)));
   }
-#pragma unroll 1
-  for (int r = 2; (float)r <= ns; ++r)
-#pragma unroll 1
-    for (int j = 0; (float)j <= nf; ++j)
-      add(reader.load(r, j, true), r, j, true, fmaf((float)j, g.wf, fmaf((float)r, g.ws, w)));
   acc = a;
   dacc = da;
 }
@@ -660,6 +704,7 @@ struct RowSamples {
   typedef float2 Raw;
   const float2* __restrict__ p;
   int pitch, yrow;
+  __device__ __forceinline__ Raw fetch(int r, int j) const { return __ldg(p + (long)r * pitch + j); }
   __device__ __forceinline__ Raw load(int r, int j, bool take) const {
     float2 t = make_float2(0.f, __int_as_float(-1));
     asm("{.reg .pred q; setp.ne.u32 q, %3, 0; @q ld.global.nc.v2.f32 {%0, %1}, [%2];}"
