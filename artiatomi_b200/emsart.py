@@ -459,7 +459,7 @@ class Reconstructor:
         check(lib.esb_reconstructor_fuse_subsets(self._h, -1 if on is None else int(bool(on))))
 
     def subvolume_patches(self, on: bool = True):
-        """subvolume_wbp with CTF: all tilts in one launch from gathered
+        """subvolume_wbp with CTF: all tilts in one launch from sampled
         slab-image patches, else (the default) one launch per tilt; the
         same boxes bit for bit."""
         check(lib.esb_reconstructor_subvolume_patches(self._h, int(on)))

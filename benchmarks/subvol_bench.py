@@ -13,8 +13,8 @@ an ellipsoid plus Gaussian noise, made on the GPU.
 
 All paths run through esb_subvolume_wbp: batched = 1 (FAST variant) runs
 one persistent launch over all particles and all tilts (with CTF from the
-slab-image patches gathered after each tilt's CTF chain); with CTF the
-per_tilt arm runs it once per tilt over the whole slab images
+slab-image patches sampled after each tilt's CTF chain); with CTF the
+per_tilt arm runs it once per tilt from that tilt's patches
 (esb_reconstructor_subvolume_patches off); batched = 0 launches the
 back-projection once per particle per tilt, with the FAST kernel (all slabs
 of a tilt in one launch, --plain fast) or, as the reference does, with the
@@ -115,7 +115,7 @@ def main(argv=None):
     plain_cfg = dataclasses.replace(w["cfg"], variant=E.VARIANT_FAST if a.plain == "fast" else E.VARIANT_FAITHFUL)
     # arms: plain (one launch per particle per tilt), per_tilt (batched, one
     # launch per tilt over all boxes), batched (with CTF: all tilts in one
-    # launch from the gathered slab-image patches)
+    # launch from the sampled slab-image patches)
     arms = ("plain", "per_tilt", "batched") if not a.no_ctf else ("plain", "batched")
     recs = {}
     for arm in arms:
