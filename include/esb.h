@@ -391,7 +391,8 @@ int esb_reconstructor_fuse_subsets(esb_reconstructor* rec, int enable);
  * every tilt to every box, each box read and written once. Off (the
  * default): one tilt's patches at a time and one launch per tilt over all
  * boxes, which is as fast (the back-projection is bound by instruction issue,
- * not by box traffic). Both give the same boxes bit for bit. */
+ * not by box traffic); calls of at most 4 particles work as on where the
+ * patches fit 64 MiB. Both give the same boxes bit for bit. */
 int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable);
 
 /* ResetProjectionsDevice (Reconstructor.cpp:1678-1682). */
