@@ -750,8 +750,11 @@ __device__ __forceinline__ void up_voxels(const KConst& k, const AxisGeom& ag, c
       macro_footprint(k, xq, y, z, pw, ph, d, r0, r1, r2, r3);
     }
   }
-  // the grid position of voxel x0, split into a sample and a remainder
-  const double ds = g.s0 + x0 * g.sx + y * g.sy + z * g.sz, df = g.f0 + x0 * g.fx + y * g.fy + z * g.fz;
+  // the grid position of the first voxel of x0's 128, split into a sample and
+  // a remainder: the same voxel whatever the group's width, so that a voxel's
+  // position, stepped from there in float, does not depend on the block shape
+  const int xa = x0 & ~127;
+  const double ds = g.s0 + xa * g.sx + y * g.sy + z * g.sz, df = g.f0 + xa * g.fx + y * g.fy + z * g.fz;
   const double is = floor(ds), jf = floor(df);
   const float s0 = (float)(ds - is), f0 = (float)(df - jf);
   const int ii = (int)is, jj = (int)jf;
@@ -772,7 +775,7 @@ __device__ __forceinline__ void up_voxels(const KConst& k, const AxisGeom& ag, c
       b1 = (float)((g.swapped ? q1 : q3) - jj);
     }
     const bool on = active && x0 + off < nx4 && sl >= 0;
-    const float fx = (float)off;
+    const float fx = (float)(x0 - xa + off);
     float acc, dacc;
     const float2* slab_at = at + (size_t)max(sl, 0) * up_stride;
     grid_sums<NC>(g, fmaf(fx, g.dsx, s0), fmaf(fx, g.dfx, f0), a0, a1, b0, b1, on,

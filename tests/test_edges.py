@@ -299,3 +299,39 @@ def test_autotuned_launch_shapes_do_not_change_results(ctf):
     for v in vols[1:]:
         np.testing.assert_array_equal(v, vols[0])
     assert "bp_axis" in report and ("fp_slicer_fused" if ctf else "fp_march") in report, report
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ctf", [False, True])
+@pytest.mark.parametrize("psi", [0.3, 88.0])
+def test_autotuned_block_shapes_on_long_rows(ctf, psi):
+    """The back-projector's block shapes on volume rows of several groups of
+    threads (260 voxels: 64 or 128 to a group), with the image's fast axis
+    along either detector axis: the same volume bit for bit."""
+    import artiatomi_b200 as E
+    from tests.test_parity_recon import _ctf_cfg
+
+    dims, W, H, tilt = (260, 21, 9), 240, 224, np.array([-48.0, 3.0, 40.0], np.float32)
+    n = len(tilt)
+    pg = E.projection_geometry(E.Markers(tilt, None, None, None, np.full(n, psi, np.float32)), W, H)
+    vg = E.volume_geometry(dims)
+    defocus = np.tile(np.array([3000.0, 3080.0, 25.0], np.float32), n) if ctf else None
+    cfgd = dict(_ctf_cfg(max(W, H))) if ctf else {}
+    imgs = cuda(np.random.default_rng(6).normal(size=(n, H, W)).astype(np.float32))
+    vols = []
+    try:
+        for k in range(5):
+            E.autotune(2 + k)
+            rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, lambda_=0.5, oversampling=2, **cfgd),
+                                  pg, tilt, defocus)
+            v = cuda(np.zeros(dims[::-1], np.float32))
+            for i in range(n):
+                rec.views()[0].copy_(imgs[i])
+                rec.back_projection(vg, v, i)
+            vols.append(host(v))
+            rec.close()
+    finally:
+        E.autotune(1)
+    assert np.abs(vols[0]).max() > 0
+    for v in vols[1:]:
+        np.testing.assert_array_equal(v, vols[0])
