@@ -1555,7 +1555,10 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
     dim3 grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    const int segs = max_runs(c, zmaj, parts_for((double)grd.x * grd.y * nw, 148.0 * 32, 8));
+    // (warps of one pixel across, not blocks of nw: the runs, and with them the
+    // order of a ray's sum, do not depend on the block shape)
+    const dim3 warps = axis_grid(swap, 1, x1 - x0, y1 - y0);
+    const int segs = max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 148.0 * 32, 8));
     if (segs > 1) {
       nw = 8;
       grd = axis_grid(swap, nw / segs, x1 - x0, y1 - y0);
