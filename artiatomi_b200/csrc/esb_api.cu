@@ -32,7 +32,8 @@ cudaError_t launch_travlen(const KConst& c, float* dist, size_t pitchE, int x0, 
 cudaError_t launch_bp(const KConst& c, void* vol, int vt, const float* img, int pw, int ph, size_t pitchE, float lambda,
                       int os, float distMin, float distMax, int linear, cudaStream_t st);
 cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mode, float* proj, float* dist,
-                                size_t pitchE, float tmin, float tmax, int x0, int y0, int x1, int y1, cudaStream_t st, int nw = 4);
+                                size_t pitchE, float tmin, float tmax, int pw, int ph, int x0, int y0, int x1, int y1,
+                                cudaStream_t st, int nw = 4);
 cudaError_t launch_bp_fast(const KConst& k, void* vol, int vt, const float* img, int pw, int ph, size_t pitchE,
                            float lambda, int os, float distMin, float distMax, int linear, cudaStream_t st);
 cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float* imgs, size_t img_stride,
@@ -49,8 +50,8 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
                                size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
                                const BpShape* shape, cudaStream_t st);
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
-                                size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1, int y1,
-                                cudaStream_t st, int nw = 4);
+                                size_t pitchE, const SlabTable& slabs, int clear, int pw, int ph, int x0, int y0,
+                                int x1, int y1, cudaStream_t st, int nw = 4);
 cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, float* virt, const float* dist,
                            float realLength, float4 cut, float4 dim, float scale, cudaStream_t st,
                            float* copy = nullptr);
@@ -262,8 +263,8 @@ int esb_fp_fast(const esb_constants* c, const void* vol, int voxel_type, int pro
   roi_y0 = roi_y0 < 0 ? 0 : roi_y0;
   roi_x1 = roi_x1 > proj_x ? proj_x : roi_x1;
   roi_y1 = roi_y1 > proj_y ? proj_y : roi_y1;
-  ESB_CK(launch_project_fast(to_kconst(*c), vol, voxel_type, 0, proj, dist, pitch / 4, 0.f, 0.f, roi_x0, roi_y0, roi_x1,
-                             roi_y1, as_stream(stream)), "esb_fp_fast");
+  ESB_CK(launch_project_fast(to_kconst(*c), vol, voxel_type, 0, proj, dist, pitch / 4, 0.f, 0.f, proj_x, proj_y,
+                             roi_x0, roi_y0, roi_x1, roi_y1, as_stream(stream)), "esb_fp_fast");
   return ok();
 }
 
@@ -278,8 +279,8 @@ int esb_fp_slicer_fast(const esb_constants* c, const void* vol, int voxel_type, 
   roi_y0 = roi_y0 < 0 ? 0 : roi_y0;
   roi_x1 = roi_x1 > proj_x ? proj_x : roi_x1;
   roi_y1 = roi_y1 > proj_y ? proj_y : roi_y1;
-  ESB_CK(launch_project_fast(to_kconst(*c), vol, voxel_type, 1, proj, nullptr, pitch / 4, tmin, tmax, roi_x0, roi_y0,
-                             roi_x1, roi_y1, as_stream(stream)), "esb_fp_slicer_fast");
+  ESB_CK(launch_project_fast(to_kconst(*c), vol, voxel_type, 1, proj, nullptr, pitch / 4, tmin, tmax, proj_x, proj_y,
+                             roi_x0, roi_y0, roi_x1, roi_y1, as_stream(stream)), "esb_fp_slicer_fast");
   return ok();
 }
 
@@ -865,7 +866,7 @@ static int rec_slicer_nw(esb_reconstructor* r, const KConst& c, const void* vol,
                          const SlabTable& T) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y;
   const int i = rec_tuned(r, tune_key(r, 0, vt, c, 1), 3, 0, [&](int k) {
-    return launch_slicer_fused(c, vol, vt, r->slab_imgs, img, W, T, 1, 0, 0, W, H, r->stream, kNw[k]);
+    return launch_slicer_fused(c, vol, vt, r->slab_imgs, img, W, T, 1, W, H, 0, 0, W, H, r->stream, kNw[k]);
   });
   return kNw[i];
 }
@@ -878,7 +879,7 @@ static int rec_march_nw(esb_reconstructor* r, const KConst& c, const void* vol, 
   const int i = rec_tuned(r, tune_key(r, 1, vt, c, 0), 3, 0, [&](int k) {
     float* s = (float*)rec_tune_scratch(r, 2 * img * sizeof(float));
     if (!s) return cudaErrorMemoryAllocation;
-    return launch_project_fast(c, vol, vt, 0, s, s + img, W, 0.f, 0.f, 0, 0, W, H, r->stream, kNw[k]);
+    return launch_project_fast(c, vol, vt, 0, s, s + img, W, 0.f, 0.f, W, H, 0, 0, W, H, r->stream, kNw[k]);
   });
   return kNw[i];
 }
@@ -910,15 +911,16 @@ static BpShape rec_bp_shape(esb_reconstructor* r, const KConst& c, int vt, const
 static cudaError_t rec_march(esb_reconstructor* r, const KConst& c, const void* vol, int vt, const int* roi) {
   const int W = r->cfg.proj_x;
   if (r->cfg.variant == ESB_VARIANT_FAST)
-    return launch_project_fast(c, vol, vt, 0, r->proj_d, r->dist_d, W, 0.f, 0.f, roi[0], roi[1], roi[2], roi[3],
-                               r->stream, rec_march_nw(r, c, vol, vt));
+    return launch_project_fast(c, vol, vt, 0, r->proj_d, r->dist_d, W, 0.f, 0.f, W, r->cfg.proj_y, roi[0], roi[1],
+                               roi[2], roi[3], r->stream, rec_march_nw(r, c, vol, vt));
   return launch_march(c, vol, vt, r->proj_d, r->dist_d, W, roi[0], roi[1], roi[2], roi[3], r->stream);
 }
 static cudaError_t rec_slicer(esb_reconstructor* r, const KConst& c, const void* vol, int vt, float* out, float t0,
                               float t1, const int* roi) {
   const int W = r->cfg.proj_x;
   if (r->cfg.variant == ESB_VARIANT_FAST)
-    return launch_project_fast(c, vol, vt, 1, out, nullptr, W, t0, t1, roi[0], roi[1], roi[2], roi[3], r->stream);
+    return launch_project_fast(c, vol, vt, 1, out, nullptr, W, t0, t1, W, r->cfg.proj_y, roi[0], roi[1], roi[2],
+                               roi[3], r->stream);
   return launch_slicer(c, vol, vt, out, W, t0, t1, roi[0], roi[1], roi[2], roi[3], r->stream);
 }
 static cudaError_t rec_bp(esb_reconstructor* r, const KConst& c, void* vol, int vt, const float* img, float lambda,
@@ -1182,8 +1184,8 @@ static int rec_forward(esb_reconstructor* r, const esb_vol_geom* vg, const void*
     }
     {
       PhaseScope ps(r, 0);
-      ESB_CK(launch_slicer_fused(c, vol, voxel_type, r->slab_imgs, img, W, T, whole ? 1 : 0, roi[0], roi[1], roi[2],
-                                 roi[3], r->stream, nw),
+      ESB_CK(launch_slicer_fused(c, vol, voxel_type, r->slab_imgs, img, W, T, whole ? 1 : 0, W, H, roi[0], roi[1],
+                                 roi[2], roi[3], r->stream, nw),
              where);
     }
     // each slab image through the CTF, added to proj_d in slab order

@@ -27,7 +27,7 @@ cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, flo
 cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2 cut, float2 dim, const int* p,
                                cudaStream_t st);
 cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mode, float* proj, float* dist,
-                                size_t pitchE, float tmin, float tmax, int x0, int y0, int x1, int y1,
+                                size_t pitchE, float tmin, float tmax, int pw, int ph, int x0, int y0, int x1, int y1,
                                 cudaStream_t st, int nw);
 cudaError_t launch_bp_fast(const KConst& k, void* vol, int vt, const float* img, int pw, int ph, size_t pitchE,
                            float lambda, int os, float distMin, float distMax, int linear, cudaStream_t st);
@@ -139,7 +139,7 @@ extern "C" int esb_sart_projection_update_noalloc(const esb_recon_config* cfg, c
   if (volume_is_empty)
     e = launch_travlen(kf, dist, W, 0, 0, W, H, st, 0);
   else if (fast)
-    e = launch_project_fast(kf, vol, voxel_type, 0, proj, dist, W, 0.f, 0.f, 0, 0, W, H, st, 4);
+    e = launch_project_fast(kf, vol, voxel_type, 0, proj, dist, W, 0.f, 0.f, W, H, 0, 0, W, H, st, 4);
   else
     e = launch_march(kf, vol, voxel_type, proj, dist, W, 0, 0, W, H, st);
   if (e != cudaSuccess) return fail(ESB_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));

@@ -1232,21 +1232,29 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
   }
 }
 
+// First pixel of the line of G that holds pixel i: lines start at multiples
+// of G of the detector, whatever the launched region, so that a pixel is
+// summed with the same middle ray in every region.
+__host__ __device__ __forceinline__ int line_start(int i, int G) { return i & ~(G - 1); }
+
 // Pixels of a thread: G along u (v with swap) from x, y; a lane pair shares
-// them, one sub-row each, and `segs` warps the same.
+// them, one sub-row each, and `segs` warps the same. The region's pixels
+// among them (`inside`) are written.
 template <int G>
 struct PlanePixel {
-  int x, y, seg;
+  int x, y, seg, x0, y0, x1, y1;
   bool active;
-  __device__ __forceinline__ PlanePixel(int swap, int segs, int x0, int y0, int x1, int y1) {
+  __device__ __forceinline__ PlanePixel(int swap, int segs, int x0_, int y0_, int x1_, int y1_)
+      : x0(x0_), y0(y0_), x1(x1_), y1(y1_) {
     const int lane = threadIdx.x & 31;
     const int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), across = G * (w / segs);
     seg = w % segs;
     const int along = (int)blockIdx.y * 16 + (lane >> 1);
-    x = x0 + (swap ? along : across);
-    y = y0 + (swap ? across : along);
+    x = swap ? x0 + along : line_start(x0, G) + across;
+    y = swap ? line_start(y0, G) + across : y0 + along;
     active = x < x1 && y < y1;
   }
+  __device__ __forceinline__ bool inside(int px, int py) const { return px >= x0 && py >= y0 && px < x1 && py < y1; }
 };
 
 // Sum of pixel i's 4 sub-rays in the reference's order, valid in even lanes.
@@ -1289,7 +1297,7 @@ __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ 
     }
     const float sum = pixel_sum(v, i, swap), gx = pixel_sum(n, 0, swap), gz = pixel_sum(d, 0, swap);
     const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
-    if (P.active && P.seg == 0 && !(threadIdx.x & 1) && x < x1 && y < y1) {
+    if (P.active && P.seg == 0 && !(threadIdx.x & 1) && P.inside(x, y)) {
       const size_t o = (size_t)y * pitchE + x;
       proj[o] += sum * c.vs.x * 0.15f * 0.25f;
       dist[o] = fmaxf(0.0f, gz / gx);
@@ -1351,7 +1359,7 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
     for (int i = 0; i < G; ++i) {
       const float sum = pixel_sum(v, i, swap);
       const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
-      if (writer && x < x1 && y < y1 && k >= klo[i] && k <= khi[i])
+      if (writer && P.inside(x, y) && k >= klo[i] && k <= khi[i])
         imgs[(size_t)k * img_stride + (size_t)y * pitchE + x] = sum * c.vs.x * 0.15f * 0.25f;
     }
   }
@@ -1359,7 +1367,7 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       const int x = P.x + (swap ? 0 : i), y = P.y + (swap ? i : 0);
-      if (x < x1 && y < y1) clear_slabs(imgs + (size_t)y * pitchE + x, img_stride, slabs.count, klo[i], khi[i]);
+      if (P.inside(x, y)) clear_slabs(imgs + (size_t)y * pitchE + x, img_stride, slabs.count, klo[i], khi[i]);
     }
   }
 }
@@ -1381,14 +1389,22 @@ int max_runs(const KConst& c, bool zmaj, int most) {
 }
 
 // The plane kernels' launch: G pixels per thread (0: not taken), whether the
-// line's rays differ in y only.
+// line's rays differ in y only. Chosen by the detector (w x h), not by the
+// region of it that is launched: a region's pixels are the whole detector's
+// bit for bit.
 struct PlaneLaunch {
-  int G = 0, parts = 1, shear = 0, swap = 0, zmaj = 0;
+  int G = 0, shear = 0, swap = 0, zmaj = 0;
   AxisStep A;
   PlaneWalk W;
-  // runs: how often a ray's samples may be cut into runs; max_parts: parts of
-  // either kind, runs or slabs
-  PlaneLaunch(const KConst& c, int vt, int w, int h, int runs, int max_parts) {
+  // Warps of g pixels per thread that a region of w x h takes.
+  double warps(int w, int h, int g) const {
+    const int along = swap ? w : h, across = swap ? h : w;
+    return (double)((across + g - 1) / g) * ((along + 15) / 16);
+  }
+  // Parts, runs or slabs, for them to fill the GPU.
+  int parts(int w, int h, int max_parts) const { return parts_for(warps(w, h, G), 148.0 * 16, max_parts); }
+  // runs: how often a ray's samples may be cut into runs
+  PlaneLaunch(const KConst& c, int vt, int w, int h, int runs) {
     bool z;
     int sm, sn;
     A = axis_step(c, z, sm, sn);
@@ -1401,7 +1417,6 @@ struct PlaneLaunch {
     const float ey = 0.5f * fabsf(au * c.u.y + av * c.v.y) * c.bbRcp.y * c.dim.y;
     const float ez = 0.5f * fabsf(au * c.u.z + av * c.v.z) * c.bbRcp.z * c.dim.z;
     shear = ex > 0.f || ez > 0.f ? 1 : 0;
-    const int along = swap ? w : h, across = swap ? h : w;
     for (int g = 4; g >= 2 && !G; g -= 2) {
       // the offset of the line's outermost ray, taken at its start or along
       // the ray to the volume's face, and its planes
@@ -1413,9 +1428,7 @@ struct PlaneLaunch {
       // pixels 141, and with 4 runs 78. Slabs do not count: they are few
       // layers each, and 1024 warps of 4 pixels with their slabs spread took
       // 105 us where 2048 of 2 pixels take 72.
-      const double warps = (double)((across + g - 1) / g) * ((along + 15) / 16);
-      const bool enough = warps * runs >= 148.0 * 4 * g;
-      parts = parts_for(warps, 148.0 * 16, max_parts);
+      const bool enough = warps(w, h, g) * runs >= 148.0 * 4 * g;
       if (small && planes && enough) G = g;
     }
     const unsigned es = vt == ESB_VOXEL_F32 ? 4 : 2, sz = es * (unsigned)c.dim.x * (unsigned)c.dim.y;
@@ -1467,7 +1480,8 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
   } while (0)
 #define ESB_PLANES_LAUNCH()                                                                          \
   do {                                                                                               \
-    const int along = L.swap ? x1 - x0 : y1 - y0, across = L.swap ? y1 - y0 : x1 - x0;                \
+    const int along = L.swap ? x1 - x0 : y1 - y0;                                                     \
+    const int across = L.swap ? y1 - line_start(y0, L.G) : x1 - line_start(x0, L.G);                  \
     const int cols = 4 / segs * L.G; /* across a block of 4 warps */                                  \
     const dim3 blk(128), grd((across + cols - 1) / cols, (along + 15) / 16, slab_parts);              \
     if (vt == ESB_VOXEL_F32) ESB_PLANES_VT(ESB_VOXEL_F32);                                           \
@@ -1494,12 +1508,12 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
   } while (0)
 
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
-                                size_t pitchE, const SlabTable& slabs, int clear, int x0, int y0, int x1,
-                                int y1, cudaStream_t st, int nw) {
+                                size_t pitchE, const SlabTable& slabs, int clear, int pw, int ph, int x0, int y0,
+                                int x1, int y1, cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0 || slabs.count <= 0) return cudaSuccess;
-  const PlaneLaunch L(c, vt, x1 - x0, y1 - y0, 1, slabs.count);
+  const PlaneLaunch L(c, vt, pw, ph, 1);
   if (L.G) {
-    const int segs = 1, slab_parts = L.parts;
+    const int segs = 1, slab_parts = L.parts(x1 - x0, y1 - y0, slabs.count);
 #define ESB_PLANES(VT, GG, SH)                                                                                        \
   k_slicer_planes<VT, GG, SH ? 2 : 0><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, imgs, img_stride, pitchE, \
                                                            slabs, clear, x0, y0, x1, y1)
@@ -1537,15 +1551,15 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
 }
 
 cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mode, float* proj, float* dist,
-                                size_t pitchE, float tmin, float tmax, int x0, int y0, int x1, int y1,
+                                size_t pitchE, float tmin, float tmax, int pw, int ph, int x0, int y0, int x1, int y1,
                                 cudaStream_t st, int nw) {
   if (x1 <= x0 || y1 <= y0) return cudaSuccess;
   bool zmaj;
   int sm, sn;
   axis_step(c, zmaj, sm, sn);
-  const PlaneLaunch L(c, vt, x1 - x0, y1 - y0, max_runs(c, zmaj, 4), 4);
+  const PlaneLaunch L(c, vt, pw, ph, max_runs(c, zmaj, 4));
   if (mode == 0 && L.G) {
-    const int segs = max_runs(c, zmaj, L.parts), slab_parts = 1;
+    const int segs = max_runs(c, zmaj, L.parts(pw, ph, 4)), slab_parts = 1;
 #define ESB_PLANES(VT, GG, SH) \
   k_project_planes<VT, GG, SH><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, segs, vol, proj, dist, pitchE, x0, y0, x1, y1)
     ESB_PLANES_LAUNCH();
@@ -1555,9 +1569,10 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
     dim3 grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    // (warps of one pixel across, not blocks of nw: the runs, and with them the
-    // order of a ray's sum, do not depend on the block shape)
-    const dim3 warps = axis_grid(swap, 1, x1 - x0, y1 - y0);
+    // (the whole detector's warps of one pixel across: the runs, and with them
+    // the order of a ray's sum, depend neither on the block shape nor on the
+    // region)
+    const dim3 warps = axis_grid(swap, 1, pw, ph);
     const int segs = max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 148.0 * 32, 8));
     if (segs > 1) {
       nw = 8;
