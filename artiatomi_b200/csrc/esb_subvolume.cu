@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kQuadsPerItem, 6) k_subvol_grid(
                       acc, dacc);
         // lambda = 1 (weighted back-projection)
         if (dacc > 0.f) {
-          v[i] += __fdividef(acc, dacc);
+          v[i] += acc / dacc;
           touched |= 1u << i;
         }
       }

@@ -323,6 +323,18 @@ def test_subvolume_ctf_patches_match_per_tilt(psi_deg):
         np.testing.assert_array_equal(b, a)
 
 
+@pytest.mark.parametrize("os_", [1, 2])
+def test_batched_subvolume_of_constant_images(os_):
+    """Images of ones: a voxel's sum of samples times chords is its sum of
+    chords, so every update is exactly 1 (a correctly rounded division)."""
+    c = _subvolume_case(False, [16, 32, 48], n=7, psi_deg=3.0)
+    c["cfgd"]["oversampling"] = os_
+    c["projs"] = np.ones_like(c["projs"])
+    for t in range(c["n"]):
+        for b in _subvolume_gpu(c, True, np.array([t], np.int32)):
+            assert (b == 1.0).any() and set(np.unique(b)) <= {0.0, 1.0}
+
+
 def test_batched_subvolume_ragged_box_runs_per_particle():
     """A box whose x extent is not a multiple of 4 cannot take the batched
     kernel's float4 layout; the call then runs the per-particle launches."""
