@@ -39,15 +39,16 @@ cudaError_t launch_bp_fast(const KConst& k, void* vol, int vt, const float* img,
 cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float* imgs, size_t img_stride,
                                  const SlabTable& slabs, int pw, int ph, size_t pitchE, float lambda, int os,
                                  float distMin, float distMax, int linear, cudaStream_t st, int transposed,
-                                 const float2* ups = nullptr, size_t up_stride = 0, const BpShape* shape = nullptr);
+                                 const float2* ups = nullptr, size_t up_stride = 0, OddFlag odd = {nullptr, 0},
+                                 const BpShape* shape = nullptr);
 cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_stride, int count, int pw, int ph, int os,
-                            int linear, float2* up, size_t up_stride, cudaStream_t st);
+                            int linear, float2* up, size_t up_stride, OddFlag odd, cudaStream_t st);
 bool bp_can_upsample(const KConst& k, int os);
 bool bp_reads_at_samples(const KConst& k, int os);
 bool bp_uses_axis(const KConst& k, int os, bool up);
 bool bp_set_eligible(const KConst& k, int os, int nslab);
-cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const SlabTable* slabs, int count,
-                               size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
+cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const OddFlag* odd, const SlabTable* slabs,
+                               int count, size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
                                const BpShape* shape, cudaStream_t st);
 cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float* imgs, size_t img_stride,
                                 size_t pitchE, const SlabTable& slabs, int clear, int pw, int ph, int x0, int y0,
@@ -56,7 +57,7 @@ cudaError_t launch_compare(int pw, int ph, size_t pitchE, const float* real, flo
                            float realLength, float4 cut, float4 dim, float scale, cudaStream_t st,
                            float* copy = nullptr);
 cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, float2 cut, float2 dim, const int* p,
-                                 int os, float2* up, cudaStream_t st);
+                                 int os, float2* up, OddFlag odd, cudaStream_t st);
 cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2 cut, float2 dim, const int* p,
                                cudaStream_t st);
 cudaError_t launch_make_square(int pw, int ph, size_t strideE, const float* in, int maxsize, float* out, int bx, int by,
@@ -66,7 +67,8 @@ cudaError_t launch_crop_to_square(int pw, int ph, size_t pitchE, float* img, int
 cudaError_t launch_square_to_image(const float* sq, int maxsize, size_t shift, float inv_norm, int pw, int ph,
                                    size_t pitchE, float* out, float* accum, int apply_crop, float2 cut, float2 dim,
                                    const int* p, cudaStream_t st, int transpose_out);
-cudaError_t launch_transpose(const float* in, int w, int h, size_t pitchE, float* out, cudaStream_t st);
+cudaError_t launch_transpose(const float* in, int w, int h, size_t pitchE, float* out, cudaStream_t st,
+                             OddFlag odd = {nullptr, 0});
 cudaError_t launch_square_to_image_batch(const float* sq, int count, int maxsize, size_t shift, float inv_norm, int pw,
                                          int ph, size_t pitchE, float* out, size_t out_stride, int transpose_out,
                                          cudaStream_t st);
@@ -460,6 +462,8 @@ struct esb_reconstructor {
   size_t slab_cap = 0;         // capacity in images
   float2* up_imgs = nullptr;   // the slab images pre-sampled on the sub-pixel grid, with sample rows
   size_t up_cap = 0;           // capacity in floats
+  unsigned* odd_d = nullptr;   // flags of the up to ESB_BP_SET_MAX pre-sampled projections (OddFlag)
+  unsigned odd_epoch = 0;      // passes so far
   void* tune_scratch = nullptr;  // the autotuner's trial outputs
   size_t tune_cap = 0;           // capacity in bytes
   SubvolBatch batch;           // tables of the batched sub-volume launch
@@ -524,6 +528,9 @@ static int rec_alloc(esb_reconstructor* r) {
   ESB_CK(cudaMalloc(&r->real_d, img), "esb_reconstructor_create");
   ESB_CK(cudaMemset(r->proj_d, 0, img), "esb_reconstructor_create");
   ESB_CK(cudaMemset(r->dist_d, 0, img), "esb_reconstructor_create");
+  const size_t flags = ESB_BP_SET_MAX * sizeof(unsigned);
+  ESB_CK(cudaMalloc(&r->odd_d, flags), "esb_reconstructor_create");
+  ESB_CK(cudaMemset(r->odd_d, 0, flags), "esb_reconstructor_create");
   if (r->cfg.ctf_mode) {
     const int N = r->N;
     ESB_CK(cudaMalloc(&r->square_d, (size_t)N * N * sizeof(float)), "esb_reconstructor_create");
@@ -551,6 +558,7 @@ static void rec_free(esb_reconstructor* r) {
   r->slab_imgs = nullptr;
   r->slab_cap = 0;
   cudaFree(r->up_imgs);
+  cudaFree(r->odd_d);
   cudaFree(r->tune_scratch);
   r->up_imgs = nullptr;
   r->up_cap = 0;
@@ -887,7 +895,7 @@ static int rec_march_nw(esb_reconstructor* r, const KConst& c, const void* vol, 
 // Block shape of the single-axis back-projection for this problem; trials on
 // a scratch slab of up to 32 planes from the middle of the volume.
 static BpShape rec_bp_shape(esb_reconstructor* r, const KConst& c, int vt, const float* imgs, size_t img_stride,
-                            const SlabTable& T, int linear, const float2* up, size_t up_stride) {
+                            const SlabTable& T, int linear, const float2* up, size_t up_stride, OddFlag odd) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y, os = r->cfg.oversampling;
   BpShape s{kBpShapes[0][0], kBpShapes[0][1], 0, 0};
   if (!bp_uses_axis(c, os, up != nullptr)) return s;
@@ -898,7 +906,7 @@ static BpShape rec_bp_shape(esb_reconstructor* r, const KConst& c, int vt, const
     if (!slab) return cudaErrorMemoryAllocation;
     const BpShape t{kBpShapes[k][0], kBpShapes[k][1], std::max(0, nz / 2 - planes / 2), planes};
     return launch_bp_fast_slabs(c, slab, vt, imgs, img_stride, T, W, H, W, 0.0f, os, 0.0f, 9999999999999.0f, linear,
-                                r->stream, 1, up, up_stride, &t);
+                                r->stream, 1, up, up_stride, odd, &t);
   });
   s.bx = kBpShapes[i][0];
   s.by = kBpShapes[i][1];
@@ -1112,8 +1120,9 @@ static int rec_subvol_slab_images(esb_reconstructor* r, const esb_vol_geom* full
 
 // The buffer of `count` pre-sampled images (launch_upsample,
 // launch_crop_upsample); NULL when the geometry does not allow them
-// (oversampling not a power of two) or they would exceed 8 GiB, and the back-projection then filters the slab images itself.
-// `up_stride` receives the (value, row) pairs per image.
+// (oversampling not a power of two) or they would exceed 8 GiB, and the
+// back-projection then filters the slab images itself. `up_stride` receives
+// the (value, row) pairs per image.
 static float2* rec_up_images(esb_reconstructor* r, const KConst& c, int count, size_t& up_stride) {
   const esb_recon_config& cf = r->cfg;
   const int os = cf.oversampling;
@@ -1262,6 +1271,7 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
   esb_compute_hit_points(&r->geoms[index], vg, p);
   KConst c = rec_const(r, r->geoms[index], *vg, 1);
   const float lambda = cf.lambda / sirt_count;
+  const OddFlag odd{r->odd_d, ++r->odd_epoch};
   if (!cf.ctf_mode) {
     const float2 cut = make_float2(cf.cut_length[0], cf.cut_length[1]);
     const float2 dim = make_float2(cf.dim_length[0], cf.dim_length[1]);
@@ -1272,7 +1282,8 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
     {
       PhaseScope ps(r, 3);
       if (one_pass) {
-        ESB_CK(launch_crop_upsample(c, W, H, img, cut, dim, p, cf.oversampling, up, r->stream), "back projection");
+        ESB_CK(launch_crop_upsample(c, W, H, img, cut, dim, p, cf.oversampling, up, odd, r->stream),
+               "back projection");
       } else {
         ESB_CK(launch_crop_border(W, H, W, img, cut, dim, p, r->stream), "back projection");
       }
@@ -1288,11 +1299,11 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
       none.count = 0;
       PhaseScope ps(r, 1);
       if (up && !one_pass)
-        ESB_CK(launch_upsample(c, r->slab_imgs, 0, 1, W, H, cf.oversampling, 0, up, up_stride, r->stream),
+        ESB_CK(launch_upsample(c, r->slab_imgs, 0, 1, W, H, cf.oversampling, 0, up, up_stride, odd, r->stream),
                "back projection");
-      const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, 0, none, 0, up, up_stride);
+      const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, 0, none, 0, up, up_stride, odd);
       ESB_CK(launch_bp_fast_slabs(c, vol, voxel_type, r->slab_imgs, 0, none, W, H, W, lambda, cf.oversampling, 0.0f,
-                                  9999999999999.0f, 0, r->stream, 1, up, up_stride, &shape), "back projection");
+                                  9999999999999.0f, 0, r->stream, 1, up, up_stride, odd, &shape), "back projection");
       return ESB_OK;
     }
     PhaseScope ps(r, 1);
@@ -1316,11 +1327,11 @@ static int rec_back_project_image(esb_reconstructor* r, const esb_vol_geom* vg, 
     float2* up = rec_up_images(r, c, T.count, up_stride);
     ESB_CK(cudaGetLastError(), "back projection");
     if (up)
-      ESB_CK(launch_upsample(c, r->slab_imgs, (size_t)W * H, T.count, W, H, cf.oversampling, 1, up, up_stride,
+      ESB_CK(launch_upsample(c, r->slab_imgs, (size_t)W * H, T.count, W, H, cf.oversampling, 1, up, up_stride, odd,
                              r->stream), "back projection");
-    const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, (size_t)W * H, T, 1, up, up_stride);
+    const BpShape shape = rec_bp_shape(r, c, voxel_type, r->slab_imgs, (size_t)W * H, T, 1, up, up_stride, odd);
     ESB_CK(launch_bp_fast_slabs(c, vol, voxel_type, r->slab_imgs, (size_t)W * H, T, W, H, W, lambda, cf.oversampling,
-                                0.f, 0.f, 1, r->stream, 1, up, up_stride, &shape), "back projection");
+                                0.f, 0.f, 1, r->stream, 1, up, up_stride, odd, &shape), "back projection");
     return ESB_OK;
   }
   for (float ray = t_in; ray < t_out; ray += step) {
@@ -1388,23 +1399,25 @@ static int rec_back_project_subset(esb_reconstructor* r, const esb_vol_geom* vg,
   const float lambda = cf.lambda / sirt_count;
   for (const auto& ch : chunks) {
     const float2* ups[ESB_BP_SET_MAX];
+    OddFlag odd[ESB_BP_SET_MAX];
     size_t off = 0;
     for (int j = ch.first; j < ch.first + ch.second; ++j) {
       const int index = indices[j];
       int p[8];
       esb_compute_hit_points(&r->geoms[index], vg, p);
       float2* up = r->up_imgs + off * up_stride;
+      const OddFlag o = odd[j - ch.first] = OddFlag{r->odd_d + (j - ch.first), ++r->odd_epoch};
       if (cf.ctf_mode) {
         if ((rc = rec_slab_capacity(r, T[j].count))) return rc;
         // cropBorder(proj_d) is re-applied to the residual on every slab (:954)
         if ((rc = rec_ctf_chain_slabs(r, T[j], index, imgs[j], 1, 1, p, 0, r->slab_imgs, nullptr, 1, p, 1))) return rc;
         PhaseScope ps(r, 1);
-        ESB_CK(launch_upsample(ks[j], r->slab_imgs, img, T[j].count, W, H, os, 1, up, up_stride, r->stream),
+        ESB_CK(launch_upsample(ks[j], r->slab_imgs, img, T[j].count, W, H, os, 1, up, up_stride, o, r->stream),
                "subset back projection");
       } else {
         PhaseScope ps(r, 3);
         ESB_CK(launch_crop_upsample(ks[j], W, H, imgs[j], make_float2(cf.cut_length[0], cf.cut_length[1]),
-                                    make_float2(cf.dim_length[0], cf.dim_length[1]), p, os, up, r->stream),
+                                    make_float2(cf.dim_length[0], cf.dim_length[1]), p, os, up, o, r->stream),
                "subset back projection");
       }
       ups[j - ch.first] = up;
@@ -1413,8 +1426,8 @@ static int rec_back_project_subset(esb_reconstructor* r, const esb_vol_geom* vg,
     PhaseScope ps(r, 1);
     const int f = ch.first;
     const BpShape shape =
-        rec_bp_shape(r, ks[f], voxel_type, r->slab_imgs, img, T[f], cf.ctf_mode ? 1 : 0, ups[0], up_stride);
-    ESB_CK(launch_bp_axis_set(&ks[f], ups, &T[f], ch.second, up_stride, vol, voxel_type, W, H, lambda, os, &shape,
+        rec_bp_shape(r, ks[f], voxel_type, r->slab_imgs, img, T[f], cf.ctf_mode ? 1 : 0, ups[0], up_stride, odd[0]);
+    ESB_CK(launch_bp_axis_set(&ks[f], ups, odd, &T[f], ch.second, up_stride, vol, voxel_type, W, H, lambda, os, &shape,
                               r->stream),
            "subset back projection");
   }
@@ -1850,7 +1863,7 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
           const int nt = std::min(chunk, proj_count - t0);
           for (int t = 0; t < nt; ++t)
             ESB_CK(launch_transpose(projections + (size_t)index_list[t0 + t] * img, W, H, W, r->slab_imgs + t * img,
-                                    r->stream), "esb_subvolume_wbp");
+                                    r->stream, subvol_odd(r->batch)), "esb_subvolume_wbp");
           PhaseScope ps(r, 1);
           ESB_CK(subvol_batch_launch(r->batch, t0, nt, r->slab_imgs, img, none, W, H, cf.oversampling, 0, r->stream),
                  "esb_subvolume_wbp");

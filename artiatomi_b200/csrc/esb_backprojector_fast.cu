@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(128, 9) k_bp_up(const __grid_constant__ KConst
                                                const __grid_constant__ UpGeom g, void* __restrict__ vol,
                                                const __grid_constant__ SlabTable slabs, int pw, int ph, float lambda,
                                                int os, float distMin, float distMax, const float2* __restrict__ ups,
-                                               size_t up_stride, int z0) {
+                                               size_t up_stride, OddFlag odd, int z0) {
   // plane z0 + blockIdx.z of the geometry, stored at plane blockIdx.z of vol
   // (z0 = 0 but for the autotuner's trial launches on a scratch slab)
   const UpThread t;
@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(128, 9) k_bp_up(const __grid_constant__ KConst
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     v[i] = active && t.x0 + t.lane + t.lanes * i < 4 * k.dimXQuarter ? Voxel<VT>::loadrw(vol, base + t.lanes * i) : 0.f;
-  up_voxels<NC>(k, a, g, slabs.bound, slabs.count, distMin, distMax, ups, up_stride, pw, ph, os, t.x0, t.lane, t.lanes,
-                t.y, z, active, [&](int i, float acc, float dacc) {
+  up_voxels<NC>(k, a, g, slabs.bound, slabs.count, distMin, distMax, ups, up_stride, odd, pw, ph, os, t.x0, t.lane,
+                t.lanes, t.y, z, active, [&](int i, float acc, float dacc) {
                   Voxel<VT>::store(vol, base + t.lanes * i, v[i] + __fdividef(lambda * acc, dacc));
                 });
 }
@@ -208,6 +208,7 @@ struct BpSetItem {
   AxisGeom a;
   UpGeom g;
   const float2* up;  // pre-sampled slab images of this projection
+  OddFlag odd;
   int nslab;         // 0: no CTF slabs
   float bound[ESB_BP_SET_MAX_SLABS + 1];
 };
@@ -234,8 +235,8 @@ __global__ void __launch_bounds__(128, 8) k_bp_axis_set(const __grid_constant__ 
 #pragma unroll 1
   for (int j = 0; j < set.count; ++j) {
     const BpSetItem& it = set.p[j];
-    up_voxels<NC>(it.k, it.a, it.g, it.bound, it.nslab, -FLT_MAX, FLT_MAX, it.up, set.up_stride, pw, ph, os, t.x0, t.lane,
-              t.lanes, t.y, z, active, [&](int i, float acc, float dacc) {
+    up_voxels<NC>(it.k, it.a, it.g, it.bound, it.nslab, -FLT_MAX, FLT_MAX, it.up, set.up_stride, it.odd, pw, ph, os,
+              t.x0, t.lane, t.lanes, t.y, z, active, [&](int i, float acc, float dacc) {
                 v[i] += __fdividef(lambda * acc, dacc);
                 touched |= 1u << i;
               });
@@ -252,11 +253,11 @@ __global__ void __launch_bounds__(128, 8) k_bp_axis_set(const __grid_constant__ 
 // nearest or bilinear as the back-projection reads it (sample_row;
 // meaningful for single-axis projections, which read it). The row depends on
 // the grid point and the projection only: it is formed once per grid point
-// and stored with the point's value in every slab image.
+// and stored with the point's value in every slab image. odd: see OddFlag.
 __global__ void __launch_bounds__(256) k_upsample(const float* __restrict__ imgs, size_t img_stride, int count, int pw,
                                                   int ph, int os, float inv, int linear, RowGeom rg, int swapped,
                                                   const __grid_constant__ KConst k, float2* __restrict__ up,
-                                                  size_t up_stride) {
+                                                  size_t up_stride, OddFlag odd) {
   const int fast = blockIdx.x * blockDim.x + threadIdx.x, slow = blockIdx.y * blockDim.y + threadIdx.y;
   const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
   if (fast >= nf || slow >= ns) return;
@@ -268,9 +269,11 @@ __global__ void __launch_bounds__(256) k_upsample(const float* __restrict__ imgs
   const float row = __int_as_float(sample_row(rg, mu, mv));
   float2* out = up + (size_t)slow * nf + fast;
 #pragma unroll 1
-  for (int s = 0; s < count; ++s)
-    out[(size_t)s * up_stride] =
-        make_float2(sample_image(imgs + (size_t)s * img_stride, pw, ph, (size_t)pw, xA, yA, linear != 0, true), row);
+  for (int s = 0; s < count; ++s) {
+    const float v = sample_image(imgs + (size_t)s * img_stride, pw, ph, (size_t)pw, xA, yA, linear != 0, true);
+    odd.see(v);
+    out[(size_t)s * up_stride] = make_float2(v, row);
+  }
 }
 
 }  // namespace
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(256) k_upsample(const float* __restrict__ imgs
 cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float* imgs, size_t img_stride,
                                  const SlabTable& slabs, int pw, int ph, size_t pitchE, float lambda, int os,
                                  float distMin, float distMax, int linear, cudaStream_t st, int transposed,
-                                 const float2* ups, size_t up_stride, const BpShape* shape) {
+                                 const float2* ups, size_t up_stride, OddFlag odd, const BpShape* shape) {
   const int nq = k.dimXQuarter, ny = (int)k.dim.y, nz = (int)k.dim.z;
   if (nq <= 0 || ny <= 0 || nz <= 0) return cudaSuccess;
   const BpGeom g = make_geom(k, os);
@@ -298,9 +301,9 @@ cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float
 #define ESB_AXIS(VT)                                                                                                 \
   do {                                                                                                               \
     if (os == 1)                                                                                                     \
-      k_bp_up<VT, 2><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, z0); \
+      k_bp_up<VT, 2><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, odd, z0); \
     else                                                                                                             \
-      k_bp_up<VT, 3><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, z0); \
+      k_bp_up<VT, 3><<<grd, blk, 0, st>>>(k, a, u, vol, slabs, pw, ph, lambda, os, distMin, distMax, ups, up_stride, odd, z0); \
   } while (0)
       if (vt == ESB_VOXEL_F32) ESB_AXIS(ESB_VOXEL_F32);
       else if (vt == ESB_VOXEL_F16) ESB_AXIS(ESB_VOXEL_F16);
@@ -331,7 +334,7 @@ cudaError_t launch_bp_fast(const KConst& k, void* vol, int vt, const float* img,
   SlabTable none;
   none.count = 0;
   return launch_bp_fast_slabs(k, vol, vt, img, 0, none, pw, ph, pitchE, lambda, os, distMin, distMax, linear, st, 0,
-                              nullptr, 0, nullptr);
+                              nullptr, 0, OddFlag{nullptr, 0}, nullptr);
 }
 
 // Whether projection k can join a subset launch (launch_bp_axis_set): the
@@ -344,12 +347,13 @@ bool bp_set_eligible(const KConst& k, int os, int nslab) {
 
 // The back-projections of `count` (<= ESB_BP_SET_MAX) projections of one
 // ordered subset in one launch (k_bp_axis_set): ks[j] the constants of
-// projection j, ups[j] its pre-sampled slab images (up_stride apart),
+// projection j, ups[j] its pre-sampled slab images (up_stride apart) and odd[j]
+// their flag,
 // slabs[j] its CTF slabs (count 0: none); all bp_set_eligible, all on the
 // same volume geometry. The block shape is shape's (bx, by); its planes are
 // the whole volume.
-cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const SlabTable* slabs, int count,
-                               size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
+cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const OddFlag* odd, const SlabTable* slabs,
+                               int count, size_t up_stride, void* vol, int vt, int pw, int ph, float lambda, int os,
                                const BpShape* shape, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
   if (count > ESB_BP_SET_MAX) return cudaErrorInvalidValue;
@@ -369,6 +373,7 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
     it.a = make_axis_geom(ks[j], g, os);
     it.g = make_up_geom(ks[j], it.a, pw, ph, os, up_swapped(it.a));
     it.up = ups[j];
+    it.odd = odd[j];
     it.nslab = slabs[j].count;
     for (int b = 0; b <= it.nslab; ++b) it.bound[b] = slabs[j].bound[b];
   }
@@ -391,14 +396,14 @@ cudaError_t launch_bp_axis_set(const KConst* ks, const float2* const* ups, const
 // images, up_stride (value, row) pairs per output image of (pw * os) x
 // (ph * os)); k gives the geometry of the rows.
 cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_stride, int count, int pw, int ph, int os,
-                            int linear, float2* up, size_t up_stride, cudaStream_t st) {
+                            int linear, float2* up, size_t up_stride, OddFlag odd, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
   const BpGeom g = make_geom(k, os);
   const int swapped = axis_beam(k, g) && up_swapped(make_axis_geom(k, g, os)) ? 1 : 0;
   const int nf = (swapped ? pw : ph) * os, ns = (swapped ? ph : pw) * os;
   const dim3 blk(32, 8), grd((nf + 31) / 32, (ns + 7) / 8);
   k_upsample<<<grd, blk, 0, st>>>(imgs, img_stride, count, pw, ph, os, 1.0f / (float)os, linear, make_row_geom(k, os),
-                                  swapped, k, up, up_stride);
+                                  swapped, k, up, up_stride, odd);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }

@@ -55,6 +55,19 @@ struct SlabTable {
   float bound[ESB_MAX_SLABS + 1];
 };
 
+// Set by the kernel that writes a projection's samples when one of them is
+// infinite or NaN: *flag = epoch, a number of its own per pass, so that
+// nothing has to clear it. (A graph replays its numbers: a flag that an
+// earlier replay set stays set, which costs time only.)
+struct OddFlag {
+  unsigned* flag;  // NULL: not recorded
+  unsigned epoch;
+  __device__ __forceinline__ void see(float v) const {
+    if (!(fabsf(v) <= 3.402823466e38f) && flag) *flag = epoch;
+  }
+  __device__ __forceinline__ bool set() const { return flag && *flag == epoch; }
+};
+
 // The subset back-projection (launch_bp_axis_set): up to ESB_BP_SET_MAX
 // projections in one launch, each with up to ESB_BP_SET_MAX_SLABS CTF slabs.
 #define ESB_BP_SET_MAX 8

@@ -234,12 +234,18 @@ __global__ void k_square_to_image_many(const float* __restrict__ sq, size_t sq_s
 }
 
 // out[x][y] = in[y][x] for a W x H image (32x32 tiles through shared memory).
-__global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t pitchE, float* __restrict__ out) {
+// odd: see OddFlag.
+__global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t pitchE, float* __restrict__ out,
+                            OddFlag odd) {
   __shared__ float tile[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
     const int x = bx + threadIdx.x, y = by + j;
-    if (x < w && y < h) tile[j][threadIdx.x] = in[(size_t)y * pitchE + x];
+    if (x < w && y < h) {
+      const float v = in[(size_t)y * pitchE + x];
+      odd.see(v);
+      tile[j][threadIdx.x] = v;
+    }
   }
   __syncthreads();
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -252,7 +258,7 @@ __global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t p
 
 // The back-projection's image passes without CTF in one: cropBorder in place
 // (k_crop_border), the transposition and the pre-sampling by nearest texel of
-// k_upsample, with the voxel row of every grid point's ray. Tiles of 32 x 32
+// k_upsample, with the voxel row of every grid point's ray (odd: see OddFlag). Tiles of 32 x 32
 // pixels: rows are read along x, grid points written along the fast axis of
 // the pre-sampled image (UpGeom). Detectors too small to fill the GPU with
 // those take tiles of 16 x 16, one pixel per thread (64 x 64: 7.8 us with 32,
@@ -261,7 +267,7 @@ __global__ void k_transpose(const float* __restrict__ in, int w, int h, size_t p
 template <int TILE>
 __global__ void __launch_bounds__(256) k_crop_upsample(int pw, int ph, float* __restrict__ img, float2 cut, float2 dim,
                                                        int2 p1, int2 p2, int2 p3, int2 p4, int os, bpcore::RowGeom rg,
-                                                       int swapped, float2* __restrict__ up) {
+                                                       int swapped, float2* __restrict__ up, OddFlag odd) {
   __shared__ float tile[TILE][TILE + 1];
   const int bx = blockIdx.x * TILE, by = blockIdx.y * TILE;
   for (int j = threadIdx.y; j < TILE; j += blockDim.y) {
@@ -269,6 +275,7 @@ __global__ void __launch_bounds__(256) k_crop_upsample(int pw, int ph, float* __
     if (x < pw && y < ph) {
       const size_t i = (size_t)y * pw + x;
       const float v = crop_factor(pw, ph, x, y, cut, dim, p1, p2, p3, p4) * img[i];
+      odd.see(v);
       img[i] = v;
       tile[j][threadIdx.x] = v;
     }
@@ -560,7 +567,7 @@ cudaError_t launch_crop_border(int pw, int ph, size_t pitchE, float* img, float2
 // k_crop_upsample of one projection (row-major, dense) without magnification
 // anisotropy; k gives the rows.
 cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, float2 cut, float2 dim, const int* p,
-                                 int os, float2* up, cudaStream_t st) {
+                                 int os, float2* up, OddFlag odd, cudaStream_t st) {
   const bpcore::BpGeom g = bpcore::make_geom(k, os);
   const int swapped = bpcore::axis_beam(k, g) && bpcore::up_swapped(bpcore::make_axis_geom(k, g, os)) ? 1 : 0;
   const int tile = (long)((pw + 31) / 32) * ((ph + 31) / 32) >= 296 ? 32 : 16;  // two 32 x 32 tiles per SM
@@ -568,7 +575,7 @@ cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, fl
   const auto kernel = tile == 32 ? k_crop_upsample<32> : k_crop_upsample<16>;
   kernel<<<grd, b, 0, st>>>(pw, ph, img, cut, dim, make_int2(p[0], p[1]), make_int2(p[2], p[3]),
                             make_int2(p[4], p[5]), make_int2(p[6], p[7]), os, bpcore::make_row_geom(k, os), swapped,
-                            up);
+                            up, odd);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -643,9 +650,9 @@ cudaError_t launch_square_to_image_many(const float* sq, size_t sq_stride, int c
   return cudaGetLastError();
 }
 
-cudaError_t launch_transpose(const float* in, int w, int h, size_t pitchE, float* out, cudaStream_t st) {
+cudaError_t launch_transpose(const float* in, int w, int h, size_t pitchE, float* out, cudaStream_t st, OddFlag odd) {
   dim3 b(32, 8), g((w + 31) / 32, (h + 31) / 32);
-  k_transpose<<<g, b, 0, st>>>(in, w, h, pitchE, out); ESB_COUNT_LAUNCH();
+  k_transpose<<<g, b, 0, st>>>(in, w, h, pitchE, out, odd); ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 

@@ -137,7 +137,8 @@ static_assert(sizeof(PatchInfo) == 32, "PatchInfo layout");
 // plain loads that k_subvol_grid is left with.
 __global__ void __launch_bounds__(256) k_patch_sample(const PatchInfo* __restrict__ info, int n_particles, int n_list,
                                                       int t, const float* __restrict__ imgs, size_t img_stride,
-                                                      int pw, int ph, float inv, float* __restrict__ patches) {
+                                                      int pw, int ph, float inv, float* __restrict__ patches,
+                                                      OddFlag odd) {
   const int lane = threadIdx.x & 31, warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int nwarps = gridDim.y * (blockDim.x >> 5);
   for (int p = blockIdx.x; p < n_particles; p += gridDim.x) {
@@ -148,8 +149,11 @@ __global__ void __launch_bounds__(256) k_patch_sample(const PatchInfo* __restric
       const float* img = imgs + (size_t)(pi.s0 + sl) * img_stride;
       const float px = ((float)(pi.ox + i) + 0.5f) * inv;
       float* dst = patches + pi.off + (long long)col * pi.ph;
-      for (int j = lane; j < pi.ph; j += 32)
-        dst[j] = sample_image(img, pw, ph, (size_t)pw, px, ((float)(pi.oy + j) + 0.5f) * inv, true, true);
+      for (int j = lane; j < pi.ph; j += 32) {
+        const float v = sample_image(img, pw, ph, (size_t)pw, px, ((float)(pi.oy + j) + 0.5f) * inv, true, true);
+        odd.see(v);
+        dst[j] = v;
+      }
     }
   }
 }
@@ -195,8 +199,9 @@ __global__ void __launch_bounds__(kQuadsPerItem, 6) k_subvol_grid(
     const SubvolWork* __restrict__ work, int n_work, const SubvolParticle* __restrict__ parts,
     const GridPair* __restrict__ pairs, const PatchInfo* __restrict__ info, const SlabTable* __restrict__ slabs,
     int n_list, int t0, int nt, const float* __restrict__ imgs, size_t img_stride, int pw, int ph, int os, int shift,
-    unsigned long long* __restrict__ misses) {
+    OddFlag odd, unsigned long long* __restrict__ misses) {
   const int lane = threadIdx.x & 31;
+  const bool any_odd = odd.set();
   for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
     const SubvolWork item = work[w];
     const SubvolParticle P = parts[item.particle];
@@ -217,6 +222,7 @@ __global__ void __launch_bounds__(kQuadsPerItem, 6) k_subvol_grid(
       const GridPair& pc = pairs[(size_t)item.particle * n_list + t];
       if (!pc.active) continue;
       const UpGeom& g = pc.g;
+      const bool plain = g.fits && !any_odd;
       int slab = -1, is = 0, js = 0, r0 = 0, r1 = 0, r2 = 0, r3 = 0;
       float s0 = 0.f, f0 = 0.f, ya = 0.f;
       PatchInfo pi{0, 0, 0, 0, 0, 0, 0};
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(kQuadsPerItem, 6) k_subvol_grid(
           base += (size_t)(t - t0) * img_stride;
         }
         float acc, dacc;
-        grid_sums<NC>(g, fmaf(cx, g.dsx, ss), fmaf(cx, g.dfx, sf), a0, a1, b0, b1, sl >= 0,
+        grid_sums<NC>(g, fmaf(cx, g.dsx, ss), fmaf(cx, g.dfx, sf), a0, a1, b0, b1, sl >= 0, plain,
                       [&](int ds, int dj, float fds, float fdj) {
                         GridSamples r;
                         r.base = base;
@@ -373,12 +379,14 @@ cudaError_t subvol_batch_build(SubvolBatch& b, int n_particles, float* const* bo
   b.first_work[n_particles] = (int)work.size();
   const size_t n_pairs = (size_t)n_particles * n_list;
   b.off_parts = align256(work.size() * sizeof(SubvolWork));
-  b.off_pairs = b.off_parts + align256(parts.size() * sizeof(SubvolParticle));
+  b.off_odd = b.off_parts + align256(parts.size() * sizeof(SubvolParticle));
+  b.off_pairs = b.off_odd + align256(sizeof(unsigned));
   const size_t most = b.off_pairs + n_pairs * std::max(sizeof(GridPair), sizeof(PairConst));
   cudaError_t e;
   if ((e = staging(b.host, b.host_cap, b.copied, most)) != cudaSuccess) return e;
   memcpy(b.host, work.data(), work.size() * sizeof(SubvolWork));
   memcpy(b.host + b.off_parts, parts.data(), parts.size() * sizeof(SubvolParticle));
+  memset(b.host + b.off_odd, 0, sizeof(unsigned));
   // per-pair constants on the host cores (the tables of 2000 particles x 61
   // tilts are 1.2e5 pairs)
   std::atomic<int> others{0};
@@ -419,6 +427,8 @@ cudaError_t subvol_batch_build(SubvolBatch& b, int n_particles, float* const* bo
   return cudaEventRecord(b.copied, st);
 }
 
+OddFlag subvol_odd(const SubvolBatch& b) { return OddFlag{(unsigned*)((char*)b.dev + b.off_odd), 1}; }
+
 // Blocks of a persistent grid: every resident block slot of every SM, at
 // most one per work item.
 static cudaError_t persistent_blocks(const void* kernel, int n_work, unsigned& blocks) {
@@ -446,7 +456,7 @@ cudaError_t subvol_batch_launch(const SubvolBatch& b, int t0, int nt, const floa
     kernel<<<blocks, kQuadsPerItem, 0, st>>>(
         (const SubvolWork*)base, b.n_work, (const SubvolParticle*)(base + b.off_parts),
         (const GridPair*)(base + b.off_pairs), nullptr, nullptr, b.n_list, t0, nt, imgs, img_stride, pw, ph, os, shift,
-        nullptr);
+        subvol_odd(b), nullptr);
   } else {
     if ((e = persistent_blocks((const void*)k_subvol_batch, b.n_work, blocks)) != cudaSuccess) return e;
     k_subvol_batch<<<blocks, kQuadsPerItem, 0, st>>>(
@@ -580,7 +590,7 @@ cudaError_t subvol_patch_sample(const SubvolBatch& b, int t, int p0, int p1, con
   const unsigned gx = (unsigned)std::min(p1 - p0, 148 * 8);
   const dim3 grd(gx, std::max(1u, std::min(16u, 2048u / gx)));
   k_patch_sample<<<grd, 256, 0, st>>>((const PatchInfo*)b.pdev + (size_t)p0 * b.n_list, p1 - p0, b.n_list, t, imgs,
-                                      img_stride, pw, ph, 1.0f / (float)os, b.patches);
+                                      img_stride, pw, ph, 1.0f / (float)os, b.patches, subvol_odd(b));
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -598,7 +608,8 @@ cudaError_t subvol_patch_launch(const SubvolBatch& b, int t0, int nt, int p0, in
   kernel<<<blocks, kQuadsPerItem, 0, st>>>(
       (const SubvolWork*)base + w0, n_work, (const SubvolParticle*)(base + b.off_parts),
       (const GridPair*)(base + b.off_pairs), (const PatchInfo*)pbase, (const SlabTable*)(pbase + b.off_slabs),
-      b.n_list, t0, nt, b.patches, 0, pw, ph, os, 0, (unsigned long long*)(pbase + b.off_miss));
+      b.n_list, t0, nt, b.patches, 0, pw, ph, os, 0, subvol_odd(b),
+      (unsigned long long*)(pbase + b.off_miss));
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }

@@ -41,7 +41,7 @@ struct SubvolBatch {
   unsigned char* host = nullptr;  // pinned staging copy of the tables
   size_t host_cap = 0;
   cudaEvent_t copied = nullptr;   // the last copy of the staging buffer to the device
-  size_t off_parts = 0, off_pairs = 0;
+  size_t off_parts = 0, off_odd = 0, off_pairs = 0;
   int n_work = 0;
   int n_list = 0;
   int n_particles = 0;
@@ -71,6 +71,10 @@ bool subvol_batchable(int n_particles, float* const* boxes, const KConst* consts
 // active may be NULL (all pairs active).
 cudaError_t subvol_batch_build(SubvolBatch& b, int n_particles, float* const* boxes, const KConst* consts,
                                const unsigned char* active, int n_list, int pw, int ph, int os, cudaStream_t st);
+
+// Flag of the call's images, set by the kernels that write them
+// (launch_transpose, subvol_patch_sample); cleared by subvol_batch_build.
+OddFlag subvol_odd(const SubvolBatch& b);
 
 // Adds list positions [t0, t0 + nt) to every box. Without slabs
 // (slabs.count == 0) position t reads image imgs + (t - t0) * img_stride;

@@ -370,3 +370,72 @@ def test_sart_graph_replay_equals_eager(ctf):
         rec.close()
     assert np.abs(vols[0]).max() > 0
     np.testing.assert_array_equal(vols[1], vols[0])
+
+
+@pytest.mark.parametrize("os_,psi", [(1, 0.0), (2, 0.0), (2, 0.3), (1, 90.0), (2, 25.0)])
+def test_back_projection_of_images_with_nan_and_infinity(os_, psi):
+    """A NaN or infinite pixel reaches the voxels whose shadow holds it and no
+    others, as in the faithful back-projector, and in particle boxes as one
+    launch per particle. The shifts keep the shadows' ends off the sample grid;
+    a voxel whose shadow ends at the pixel to rounding may differ. The faithful
+    kernel places a ray to 1e-3 pixels (float at |t| = 1e4), the shadow has two
+    ends per axis: 4e-3 of the voxels on average, whole runs of them along a
+    ray, so 3 % are allowed (6 % to 100 % more voxels come out of reads beyond
+    the shadow)."""
+    import artiatomi_b200 as E
+    from artiatomi_b200 import _lib as L
+
+    dims, W, H, tilt = (96, 80, 24), 96, 88, np.array([0.0, 33.0, -55.0], np.float32)
+    n = len(tilt)
+    xs, ys = np.array([0.17, -0.31, 0.43], np.float32), np.array([-0.13, 0.37, 0.21], np.float32)
+    pg = E.projection_geometry(E.Markers(tilt, xs, ys, None, np.full(n, psi, np.float32)), W, H)
+    vg = E.volume_geometry(dims)
+    imgs = np.ones((n, H, W), np.float32)
+    for i, bad in enumerate((np.nan, np.inf, -np.inf)):
+        imgs[i, H // 2, W // 2] = imgs[i, H // 3, W // 4] = bad
+    masks = []
+    for variant in (E.VARIANT_FAITHFUL, E.VARIANT_FAST):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=variant, oversampling=os_), pg, tilt)
+        for i in range(n):
+            v = cuda(np.zeros(dims[::-1], np.float32))
+            rec.views()[0].copy_(cuda(imgs[i]))
+            rec.back_projection(vg, v, i)
+            masks.append(~np.isfinite(host(v)))
+        rec.close()
+    boxes = []
+    for batched in (False, True):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, oversampling=os_), pg, tilt)
+        sub = [E.subvolume_geometry(s, 1.0, vg, p) for s, p in ((24, (48, 40, 12)), (16, (30, 28, 12)))]
+        pair = (L.ProjGeom * (2 * n))(*[pg[i % n] for i in range(2 * n)])
+        b = [cuda(np.zeros((s, s, s), np.float32)) for s in (24, 16)]
+        rec.subvolume_wbp(vg, sub, pair, b, cuda(imgs), np.arange(n, dtype=np.int32), batched=batched)
+        boxes.append([~np.isfinite(host(x)) for x in b])
+        rec.close()
+    assert boxes[0][0].any() and all(m.any() for m in masks)
+    for want, got in list(zip(masks[:n], masks[n:])) + list(zip(*boxes)):
+        assert (want != got).sum() <= max(2, 0.03 * want.sum()), (want.sum(), got.sum())
+
+
+def test_subset_with_nan_in_one_projection():
+    """The ordered subset of a 16-bit volume: a NaN pixel of one projection
+    reaches the voxels that it reaches alone."""
+    import torch
+
+    import artiatomi_b200 as E
+
+    dims, W, H, tilt = (96, 80, 24), 96, 88, np.array([-40.0, -10.0, 20.0, 50.0], np.float32)
+    n = len(tilt)
+    pg = E.projection_geometry(E.Markers(tilt), W, H)
+    vg = E.volume_geometry(dims)
+    imgs = np.random.default_rng(3).normal(size=(n, H, W)).astype(np.float32)
+    imgs[2, H // 2, W // 2] = np.nan
+    masks = []
+    for fuse in (False, True):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, oversampling=2), pg, tilt)
+        rec.fuse_subsets(fuse)
+        v = torch.zeros(dims[::-1], device="cuda", dtype=torch.float16)
+        rec.sart(vg, v, cuda(imgs), np.arange(n, dtype=np.int32), iterations=1, sirt_count=n)
+        masks.append(~np.isfinite(host(v)))
+        rec.close()
+    assert masks[0].any() and not masks[0].all()
+    np.testing.assert_array_equal(masks[1], masks[0])
