@@ -684,20 +684,24 @@ __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C,
   const long step1 = SN > 0 ? (long)sN : -(long)sN;
   Raw va = Raw(0), vb, vc, vd = Raw(0), wa = Raw(0), wb, wc, wd = Raw(0);
   float nMs = 0.f, nNs = 0.f;
-  bool X = false;
-  // row im with its window, clamped
+  bool X = false, Xp = false;  // a minor crossing in this layer, in the one before
+  // row im with its window, clamped; the outer positions where they have a
+  // weight (0 times an infinite voxel or NaN is NaN)
   auto fetch = [&]() {
+    nMs = __fmaf_rn(k, A.isM, nM0);
+    nNs = __fmaf_rn(kn, A.isN, nN0);
+    X = nNs <= nMs;
     const char* p = clamped(im, in0 - SN);
-    va = ldraw<VT>(p), wa = ldraw<VT>(p + dy);
+    va = wa = vd = wd = Raw(0);
+    ldraw_if<VT>(va, p, Xp);
+    ldraw_if<VT>(wa, p + dy, Xp);
     p = clamped(im, in0);
     vb = ldraw<VT>(p), wb = ldraw<VT>(p + dy);
     p = clamped(im, in0 + SN);
     vc = ldraw<VT>(p), wc = ldraw<VT>(p + dy);
     p = clamped(im, in0 + 2 * SN);
-    vd = ldraw<VT>(p), wd = ldraw<VT>(p + dy);
-    nMs = __fmaf_rn(k, A.isM, nM0);
-    nNs = __fmaf_rn(kn, A.isN, nN0);
-    X = nNs <= nMs;
+    ldraw_if<VT>(vd, p, X);
+    ldraw_if<VT>(wd, p + dy, X);
   };
   // the layer of the row at hand, which may be the ray's last
   auto edge_layer = [&]() {
@@ -705,6 +709,7 @@ __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C,
     layer(X, fminf(nNs, tL), tL, va, vb, vc, vd, wa, wb, wc, wd);
     im += SM;
     k += 1.f;
+    Xp = X;
     if (X) {
       in0 += SN;
       kn += 1.f;
@@ -760,13 +765,16 @@ __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C,
     fetch();
   }
   {  // the far row of the last layer
-    const char *p0 = clamped(im, in0 - SN), *p1 = clamped(im, in0), *p2 = clamped(im, in0 + SN);
+    const char *p1 = clamped(im, in0), *p2 = clamped(im, in0 + SN);
     S0 = fmaf(cvt<VT>(ldraw<VT>(p1)), g1, S0);
     S1 = fmaf(cvt<VT>(ldraw<VT>(p1 + dy)), g1, S1);
     T0 = fmaf(cvt<VT>(ldraw<VT>(p2)), g2, T0);
     T1 = fmaf(cvt<VT>(ldraw<VT>(p2 + dy)), g2, T1);
-    S0 = fmaf(cvt<VT>(ldraw<VT>(p0)), g0, S0);
-    S1 = fmaf(cvt<VT>(ldraw<VT>(p0 + dy)), g0, S1);
+    if (Xp) {
+      const char* p0 = clamped(im, in0 - SN);
+      S0 = fmaf(cvt<VT>(ldraw<VT>(p0)), g0, S0);
+      S1 = fmaf(cvt<VT>(ldraw<VT>(p0 + dy)), g0, S1);
+    }
   }
   return fmaf(b, S1 + T1, (1.0f - b) * (S0 + T0));
 }
