@@ -478,7 +478,8 @@ struct esb_reconstructor {
   bool r2c_many_ok[ESB_CTF_SLAB_BATCH + 1] = {};
   bool graphs = false;                   // replay SART iterations from a captured graph
   int fuse_subsets = -1;                 // subset back-projection in one volume pass: 1 on, 0 off, -1 half volumes
-  bool subvol_patches = false;           // sub-volume WBP with CTF: all tilts in one launch from gathered patches
+  bool subvol_patches = false;           // sub-volume WBP with CTF: all tilts in one launch from sampled patches
+  size_t subvol_patch_bytes = 0;         // bound on their memory, 0: the default
   cudaGraphExec_t sart_exec = nullptr;   // the last captured iteration
   // inputs the captured iteration was recorded with (it replays only for the
   // same ones) and the library kernels it launches
@@ -693,6 +694,12 @@ int esb_reconstructor_fuse_subsets(esb_reconstructor* rec, int enable) {
 int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable) {
   if (!rec) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_reconstructor_subvolume_patches: NULL reconstructor");
   rec->subvol_patches = enable != 0;
+  return ok();
+}
+
+int esb_reconstructor_subvolume_patch_bytes(esb_reconstructor* rec, size_t bytes) {
+  if (!rec) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_reconstructor_subvolume_patch_bytes: NULL reconstructor");
+  rec->subvol_patch_bytes = bytes;
   return ok();
 }
 
@@ -1114,6 +1121,24 @@ static int rec_subvol_slab_images(esb_reconstructor* r, const esb_vol_geom* full
     if ((rc = rec_fft_many(r, cnt, false))) return rc;
     ESB_CK(launch_square_to_image_batch(r->sq_batch, cnt, N, r->squareShift, 1.0f / ((float)N * (float)N), W, H, W,
                                         r->slab_imgs + (size_t)c0 * img, img, 1, r->stream), "CTF slab images");
+  }
+  return ESB_OK;
+}
+
+// Back-projects the slab images of projection `index` (rec_subvol_slab_images)
+// into the boxes of particles [p0, p1), one launch per particle.
+static int rec_subvol_slab_launches(esb_reconstructor* r, const esb_proj_geom* pair_geoms,
+                                    const esb_vol_geom* sub_geoms, const unsigned char* active, float* const* boxes,
+                                    int p0, int p1, int index, const SlabTable& T) {
+  const esb_recon_config& cf = r->cfg;
+  const int W = cf.proj_x, H = cf.proj_y;
+  for (int p = p0; p < p1; ++p) {
+    const size_t pair = (size_t)p * cf.n_proj + index;
+    if (active && !active[pair]) continue;
+    PhaseScope ps(r, 1);
+    ESB_CK(launch_bp_fast_slabs(rec_const(r, pair_geoms[pair], sub_geoms[p], 1), boxes[p], ESB_VOXEL_F32, r->slab_imgs,
+                                (size_t)W * H, T, W, H, W, 1.0f, cf.oversampling, 0.f, 0.f, 1, r->stream, 1),
+           "esb_subvolume_wbp");
   }
   return ESB_OK;
 }
@@ -1878,11 +1903,13 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
       // tilts (3 particles, 9 tilts: 534 us with one launch per tilt, 497
       // before there were patches)
       const bool few = n_particles <= 4;
+      auto bound = [&](size_t def) { return r->subvol_patch_bytes ? r->subvol_patch_bytes : def; };
       if (r->subvol_patches || few) {
         // every tilt's slab images filtered and the patches its pairs read
         // evaluated (up to 16 GiB), then all tilts in one persistent launch
-        const size_t bound = r->subvol_patches ? (size_t)16 << 30 : (size_t)64 << 20;
-        ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, true, bound, r->stream, planned),
+        const size_t most = r->subvol_patches ? bound((size_t)16 << 30)
+                                              : std::min(bound((size_t)4 << 30), (size_t)64 << 20);
+        ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, true, most, r->stream, planned),
                "esb_subvolume_wbp");
         if (planned) {
           for (int ii = 0; ii < proj_count; ++ii) {
@@ -1908,9 +1935,10 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
         }
       }
       // one tilt's patches (up to 4 GiB, else its particles in chunks), one
-      // launch per tilt
-      ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, false, (size_t)4 << 30, r->stream, planned),
-             "esb_subvolume_wbp");
+      // launch per tilt; a particle whose patches do not fit alone reads the
+      // slab images, as below
+      ESB_CK(subvol_patch_plan(r->batch, Ts.data(), W, H, cf.oversampling, false, bound((size_t)4 << 30), r->stream,
+                               planned), "esb_subvolume_wbp");
       if (planned) {
         size_t c = 0;
         for (int ii = 0; ii < proj_count; ++ii) {
@@ -1919,6 +1947,11 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
           if ((rc = rec_subvol_slab_images(r, full_vol, projections + (size_t)index * img, index, T))) return rc;
           for (; c < r->batch.chunks.size() && r->batch.chunks[c].t == ii; ++c) {
             const SubvolBatch::Chunk& ch = r->batch.chunks[c];
+            if (!ch.patches) {
+              if ((rc = rec_subvol_slab_launches(r, pair_geoms, sub_geoms, active, boxes, ch.p0, ch.p1, index, T)))
+                return rc;
+              continue;
+            }
             {
               PhaseScope ps(r, 3);
               ESB_CK(subvol_patch_sample(r->batch, ii, ch.p0, ch.p1, r->slab_imgs, img, W, H, cf.oversampling,
@@ -1931,15 +1964,18 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
         }
         return ok();
       }
-      for (int ii = 0; ii < proj_count; ++ii) {
-        const int index = index_list[ii];
-        SlabTable T;
-        if ((rc = rec_subvol_slab_images(r, full_vol, projections + (size_t)index * img, index, T))) return rc;
-        PhaseScope ps(r, 1);
-        ESB_CK(subvol_batch_launch(r->batch, ii, 1, r->slab_imgs, img, T, W, H, cf.oversampling, 1, r->stream),
-               "esb_subvolume_wbp");
+      if (!r->batch.all_axis) {  // the general chords on the slab images
+        for (int ii = 0; ii < proj_count; ++ii) {
+          const int index = index_list[ii];
+          SlabTable T;
+          if ((rc = rec_subvol_slab_images(r, full_vol, projections + (size_t)index * img, index, T))) return rc;
+          PhaseScope ps(r, 1);
+          ESB_CK(subvol_batch_launch(r->batch, ii, 1, r->slab_imgs, img, T, W, H, cf.oversampling, 1, r->stream),
+                 "esb_subvolume_wbp");
+        }
+        return ok();
       }
-      return ok();
+      // no memory for a plan: one launch per particle
     }
   }
   // EmSartSubVolumes.cpp:626-683 with Reconstructor.cpp:893-914 / 975-1033
@@ -1978,13 +2014,8 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
       // per particle that picks each quad's slab image by its depth
       SlabTable T;
       if ((rc = rec_subvol_slab_images(r, full_vol, proj, index, T))) return rc;
-      for (int p = 0; p < n_particles; ++p) {
-        if (active && !active[(size_t)p * np + index]) continue;
-        KConst c = rec_const(r, pair_geoms[(size_t)p * np + index], sub_geoms[p], 1);
-        PhaseScope ps(r, 1);
-        ESB_CK(launch_bp_fast_slabs(c, boxes[p], ESB_VOXEL_F32, r->slab_imgs, img, T, W, H, W, 1.0f, cf.oversampling,
-                                    0.f, 0.f, 1, r->stream, 1), "esb_subvolume_wbp");
-      }
+      if ((rc = rec_subvol_slab_launches(r, pair_geoms, sub_geoms, active, boxes, 0, n_particles, index, T)))
+        return rc;
       continue;
     }
     for (float ray = t_in; ray < t_out; ray += step) {

@@ -355,6 +355,13 @@ static cudaError_t device_buffer(void*& dev, size_t& cap, size_t bytes, cudaStre
   return cudaSuccess;
 }
 
+// Whether an allocation failed for want of memory; clears the error.
+static bool out_of_memory(cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation) return false;
+  cudaGetLastError();
+  return true;
+}
+
 constexpr long kPairsPerThread = 512;  // host threads are worth starting beyond this many pairs
 
 cudaError_t subvol_batch_build(SubvolBatch& b, int n_particles, float* const* boxes, const KConst* consts,
@@ -477,7 +484,8 @@ cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, in
   b.off_miss = b.off_slabs + align256((size_t)nl * sizeof(SlabTable));
   const size_t bytes = b.off_miss + sizeof(unsigned long long);
   cudaError_t e;
-  if ((e = staging(b.phost, b.phost_cap, b.pcopied, bytes)) != cudaSuccess) return e;
+  if ((e = staging(b.phost, b.phost_cap, b.pcopied, bytes)) != cudaSuccess) return out_of_memory(e) ? cudaSuccess : e;
+  if ((e = device_buffer(b.pdev, b.pcap, bytes, st)) != cudaSuccess) return out_of_memory(e) ? cudaSuccess : e;
   const SubvolParticle* parts = (const SubvolParticle*)(b.host + b.off_parts);
   const GridPair* pcs = (const GridPair*)(b.host + b.off_pairs);
   PatchInfo* info = (PatchInfo*)b.phost;
@@ -539,42 +547,48 @@ cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, in
     pi.ns = s1 - s0 + 1;
   }, kPairsPerThread);
   // offsets: over all pairs, or per list position, the particles in chunks
-  // that fit the buffer
-  const size_t max_floats = max_bytes / sizeof(float);
-  size_t most = 0;
-  b.chunks.clear();
-  if (all_tilts) {
-    for (long i = 0; i < (long)np * nl; ++i) {
-      info[i].off = (long long)most;
-      most += (size_t)info[i].ns * info[i].pw * info[i].ph;
-    }
-    if (most > max_floats) return cudaSuccess;
-  } else {
-    for (int t = 0; t < nl; ++t) {
-      size_t used = 0;
-      int first = 0;
-      for (int p = 0; p < np; ++p) {
-        PatchInfo& pi = info[(size_t)p * nl + t];
-        const size_t n = (size_t)pi.ns * pi.pw * pi.ph;
-        if (used > 0 && used + n > max_floats) {
-          b.chunks.push_back({t, first, p});
+  // that fit the buffer; the bound is halved until the device has room
+  for (size_t max_floats = max_bytes / sizeof(float);;) {
+    size_t most = 0;
+    b.chunks.clear();
+    if (all_tilts) {
+      for (long i = 0; i < (long)np * nl; ++i) {
+        info[i].off = (long long)most;
+        most += (size_t)info[i].ns * info[i].pw * info[i].ph;
+      }
+      if (most > max_floats) return cudaSuccess;
+    } else {
+      for (int t = 0; t < nl; ++t) {
+        size_t used = 0;
+        int first = 0;
+        auto cut = [&](int p, bool patches) {  // a chunk up to particle p
+          if (p > first) b.chunks.push_back({t, first, p, patches});
           first = p;
           used = 0;
+        };
+        for (int p = 0; p < np; ++p) {
+          PatchInfo& pi = info[(size_t)p * nl + t];
+          const size_t n = (size_t)pi.ns * pi.pw * pi.ph;
+          if (used + n > max_floats) cut(p, true);
+          pi.off = (long long)used;
+          if (n > max_floats) {
+            cut(p + 1, false);
+          } else {
+            used += n;
+            most = std::max(most, used);
+          }
         }
-        pi.off = (long long)used;
-        used += n;
-        most = std::max(most, used);
+        cut(np, true);
       }
-      b.chunks.push_back({t, first, np});
     }
-  }
-  void* buf = b.patches;
-  if ((e = device_buffer(buf, b.patches_cap, std::max<size_t>(most, 1) * sizeof(float), st)) != cudaSuccess) {
+    void* buf = b.patches;
+    e = device_buffer(buf, b.patches_cap, std::max<size_t>(most, 1) * sizeof(float), st);
     b.patches = (float*)buf;
-    return e;
+    if (e == cudaSuccess) break;
+    if (!out_of_memory(e)) return e;
+    if (all_tilts || most <= 1) return cudaSuccess;
+    max_floats = most / 2;
   }
-  b.patches = (float*)buf;
-  if ((e = device_buffer(b.pdev, b.pcap, bytes, st)) != cudaSuccess) return e;
   memcpy(b.phost + b.off_slabs, slabs, (size_t)nl * sizeof(SlabTable));
   memset(b.phost + b.off_miss, 0, sizeof(unsigned long long));
   if ((e = cudaMemcpyAsync(b.pdev, b.phost, bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;

@@ -58,6 +58,7 @@ struct SubvolBatch {
   size_t patches_cap = 0;  // bytes
   struct Chunk {
     int t, p0, p1;  // list position, particles [p0, p1)
+    bool patches;   // they fit the buffer; else the caller reads the slab images
   };
   std::vector<Chunk> chunks;     // of a plan per list position
   std::vector<int> first_work;   // first work item of every particle, and their number
@@ -88,9 +89,12 @@ cudaError_t subvol_batch_launch(const SubvolBatch& b, int t0, int nt, const floa
 // particle's quads read: the slabs its depth range meets, and the detector
 // rectangle of its box's shadow with a margin, at every sub-pixel grid point.
 // all_tilts: the patches of all positions in one buffer; else a buffer for
-// one position, its particles in chunks (b.chunks) that fit max_bytes. ok is
-// false (nothing planned) when some pair does not take the single-axis sums
-// or, with all_tilts, the patches exceed max_bytes.
+// one position, its particles in chunks (b.chunks) that fit max_bytes, a
+// particle whose patches alone exceed them in a chunk without patches. Where
+// the device has no room for max_bytes, as much as there is is taken. ok is
+// false (nothing planned) when some pair does not take the single-axis sums,
+// with all_tilts when the patches do not fit, and when there is no memory for
+// the tables.
 cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, int ph, int os, bool all_tilts,
                               size_t max_bytes, cudaStream_t st, bool& ok);
 

@@ -464,6 +464,11 @@ class Reconstructor:
         same boxes bit for bit."""
         check(lib.esb_reconstructor_subvolume_patches(self._h, int(on)))
 
+    def subvolume_patch_bytes(self, n: int = 0):
+        """Bound on the memory of subvolume_wbp's patches (0: the default);
+        particles beyond it take further launches."""
+        check(lib.esb_reconstructor_subvolume_patch_bytes(self._h, int(n)))
+
     def timing(self):
         """{phase: (ms, launches)} since the previous call; phases fp, bp, ctf, compare."""
         ms = np.zeros(4, np.float64)

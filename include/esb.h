@@ -395,6 +395,13 @@ int esb_reconstructor_fuse_subsets(esb_reconstructor* rec, int enable);
  * patches fit 64 MiB. Both give the same boxes bit for bit. */
 int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable);
 
+/* Bound on the memory of those patches in bytes (0: the default, 4 GiB for
+ * one tilt's, 16 GiB with esb_reconstructor_subvolume_patches on). Particles
+ * beyond it are added in further launches, particles whose patches do not fit
+ * alone, and all of them where the device has no memory for any, from the
+ * slab images by one launch each. */
+int esb_reconstructor_subvolume_patch_bytes(esb_reconstructor* rec, size_t bytes);
+
 /* ResetProjectionsDevice (Reconstructor.cpp:1678-1682). */
 int esb_rec_reset_projections(esb_reconstructor* rec);
 /* ForwardProjection (Reconstructor.cpp:1411-1421), CTF or not. */

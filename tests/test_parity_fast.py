@@ -242,7 +242,7 @@ def _subvolume_case(ctf, sizes, n=7, seed=31, psi_deg=0.0):
                 pair_o=pair_o, defocus=defocus if ctf else None, cfgd=cfgd, shifts=shifts, sizes=sizes)
 
 
-def _subvolume_gpu(c, batched, index_list, active=None, patches=None):
+def _subvolume_gpu(c, batched, index_list, active=None, patches=None, patch_bytes=None):
     import artiatomi_b200 as E
 
     W, H, n = c["W"], c["H"], c["n"]
@@ -250,6 +250,8 @@ def _subvolume_gpu(c, batched, index_list, active=None, patches=None):
     rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, **c["cfgd"]), pg, c["tilt"], c["defocus"])
     if patches is not None:
         rec.subvolume_patches(patches)
+    if patch_bytes is not None:
+        rec.subvolume_patch_bytes(patch_bytes)
     boxes = [cuda(np.zeros((s, s, s), np.float32)) for s in c["sizes"]]
     rec.subvolume_wbp(c["full"], c["sub"], c["pair"], boxes, cuda(c["projs"]), index_list, active=active,
                       batched=batched)
@@ -321,6 +323,63 @@ def test_subvolume_ctf_patches_match_per_tilt(psi_deg):
     for a, b in zip(per_tilt, one):
         assert np.abs(a).sum() > 0
         np.testing.assert_array_equal(b, a)
+
+
+@pytest.mark.parametrize("patches", [False, True])
+def test_subvolume_patch_bound(patches):
+    """Patches beyond the bound: in chunks of particles (bit for bit the boxes
+    of one chunk), and from the slab images where a particle's patches do not
+    fit alone (the launches per particle, to rounding). 200 kB hold two or
+    three of the smaller boxes' patches of a tilt, 1 byte none."""
+    c = _subvolume_case(True, [16, 24, 32, 48, 16, 24], n=9, seed=5, psi_deg=0.7)
+    il = np.random.default_rng(1).permutation(c["n"]).astype(np.int32)
+    active = (np.linalg.norm(c["shifts"], axis=2) < 1.5).astype(np.uint8)
+    free = _subvolume_gpu(c, True, il, active)
+    plain = _subvolume_gpu(c, False, il, active)
+    few = _subvolume_gpu(dict(c, sizes=c["sizes"][:3], sub=c["sub"][:3]), True, il, active[:3], patch_bytes=1)
+    chunks = _subvolume_gpu(c, True, il, active, patches, 200 << 10)
+    none = _subvolume_gpu(c, True, il, active, patches, 1)
+    for a, b in zip(free[:2], chunks[:2]):
+        np.testing.assert_array_equal(b, a)
+    for got in (chunks, none, few):
+        for a, b in zip(plain, got):
+            assert np.abs(a).sum() > 0
+            assert rel_l2(b, a) <= 1e-5
+    for a, b in zip(plain, none):
+        np.testing.assert_array_equal(b, a)
+
+
+def test_subvolume_patches_without_memory():
+    """Little free device memory: the call takes the patches that fit."""
+    import torch
+
+    import artiatomi_b200 as E
+
+    c = _subvolume_case(True, [48] * 400, n=3, seed=5)
+    il = np.arange(c["n"], dtype=np.int32)
+    W, H, n = c["W"], c["H"], c["n"]
+    pg = E.projection_geometry(E.Markers(c["tilt"], rotation_psi=c["psi"]), W, H)
+    boxes = [[torch.zeros((s, s, s), device="cuda") for s in c["sizes"]] for _ in range(2)]
+    projs = cuda(c["projs"])
+    for k, b in enumerate(boxes):
+        rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, **c["cfgd"]), pg, c["tilt"], c["defocus"])
+        small = [torch.zeros((48, 48, 48), device="cuda")]
+        rec.subvolume_wbp(c["full"], c["sub"][:1], c["pair"], small, projs, il, batched=False)  # plans, slab images
+        torch.cuda.synchronize()
+        ballast = []
+        try:
+            if k:
+                free = torch.cuda.mem_get_info()[0]
+                ballast.append(torch.empty(max(free - (64 << 20), 0), dtype=torch.uint8, device="cuda"))
+            rec.subvolume_wbp(c["full"], c["sub"], c["pair"], b, projs, il)
+            torch.cuda.synchronize()
+        finally:
+            del ballast
+            torch.cuda.empty_cache()
+        rec.close()
+    assert float(boxes[0][7].abs().sum()) > 0
+    for a, b in zip(*boxes):
+        assert rel_l2(host(b), host(a)) <= 1e-5
 
 
 @pytest.mark.parametrize("os_", [1, 2])
