@@ -22,9 +22,9 @@
 //
 // The per-voxel sums are those of the single-volume back-projector on
 // pre-sampled images (grid_sums in esb_bp_core.cuh) for projections without
-// a y component of the beam. Other geometry (and patches beyond the buffer
-// cap) takes k_subvol_batch: the general chords, or the single-axis sums on
-// the slab images read directly.
+// a y component of the beam. Other geometry takes k_subvol_batch, the general
+// chords on the images; particles whose patches do not fit the buffer take the
+// single-volume back-projector on the slab images, one launch each.
 #include <string.h>
 
 #include <atomic>
@@ -452,6 +452,7 @@ static cudaError_t persistent_blocks(const void* kernel, int n_work, unsigned& b
 cudaError_t subvol_batch_launch(const SubvolBatch& b, int t0, int nt, const float* imgs, size_t img_stride,
                                 const SlabTable& slabs, int pw, int ph, int os, int linear, cudaStream_t st) {
   if (b.n_work <= 0 || nt <= 0) return cudaSuccess;
+  if (b.all_axis && (slabs.count > 0 || linear)) return cudaErrorInvalidValue;  // patches, or a launch per particle
   unsigned blocks = 0;
   cudaError_t e;
   const char* base = (const char*)b.dev;

@@ -80,7 +80,8 @@ OddFlag subvol_odd(const SubvolBatch& b);
 // Adds list positions [t0, t0 + nt) to every box. Without slabs
 // (slabs.count == 0) position t reads image imgs + (t - t0) * img_stride;
 // with slabs each quad reads the image of its slab. Images are transposed
-// ([x][y]).
+// ([x][y]). Where every pair takes the single-axis sums (b.all_axis), slabs
+// and the linear filter are refused: those calls read patches.
 cudaError_t subvol_batch_launch(const SubvolBatch& b, int t0, int nt, const float* imgs, size_t img_stride,
                                 const SlabTable& slabs, int pw, int ph, int os, int linear, cudaStream_t st);
 
