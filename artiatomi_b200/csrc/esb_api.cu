@@ -697,6 +697,23 @@ int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable) {
   return ok();
 }
 
+// Fails when a finished sub-volume call has left out samples.
+static int rec_subvol_misses(esb_reconstructor* r, const char* what) {
+  unsigned long long misses = 0;
+  ESB_CK(subvol_patch_misses(r->batch, r->stream, misses), what);
+  if (misses)
+    return fail(ESB_ERR_UNSUPPORTED, std::string(what) + ": " + std::to_string(misses) +
+                                         " quads' samples fell outside the planned CTF patches");
+  return ESB_OK;
+}
+
+int esb_reconstructor_subvolume_check(esb_reconstructor* rec) {
+  if (!rec) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_reconstructor_subvolume_check: NULL reconstructor");
+  ESB_CK(cudaStreamSynchronize(rec->stream), "esb_reconstructor_subvolume_check");
+  const int rc = rec_subvol_misses(rec, "esb_subvolume_wbp");
+  return rc ? rc : ok();
+}
+
 int esb_reconstructor_subvolume_patch_bytes(esb_reconstructor* rec, size_t bytes) {
   if (!rec) return fail(ESB_ERR_INVALID_ARGUMENT, "esb_reconstructor_subvolume_patch_bytes: NULL reconstructor");
   rec->subvol_patch_bytes = bytes;
@@ -1865,6 +1882,7 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
   for (int ii = 0; ii < proj_count; ++ii)
     if (index_list[ii] < 0 || index_list[ii] >= np)
       return fail(ESB_ERR_INVALID_ARGUMENT, "esb_subvolume_wbp: index out of range");
+  if ((rc = rec_subvol_misses(r, "an earlier esb_subvolume_wbp"))) return rc;
   if (batched && cf.variant == ESB_VARIANT_FAST && n_particles > 0 && proj_count > 0) {
     std::vector<KConst> consts((size_t)n_particles * proj_count);
     std::vector<unsigned char> act((size_t)n_particles * proj_count);
@@ -1925,13 +1943,8 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
             ESB_CK(subvol_patch_launch(r->batch, 0, proj_count, 0, n_particles, W, H, cf.oversampling, r->stream),
                    "esb_subvolume_wbp");
           }
-          if (!r->subvol_patches) return ok();
-          unsigned long long misses = 0;
-          ESB_CK(subvol_patch_misses(r->batch, r->stream, misses), "esb_subvolume_wbp");
-          if (misses)
-            return fail(ESB_ERR_UNSUPPORTED, "esb_subvolume_wbp: " + std::to_string(misses) +
-                                                 " quad samples fell outside the planned CTF patches");
-          return ok();
+          ESB_CK(subvol_patch_count(r->batch, r->stream), "esb_subvolume_wbp");
+          return r->subvol_patches ? esb_reconstructor_subvolume_check(r) : ok();
         }
       }
       // one tilt's patches (up to 4 GiB, else its particles in chunks), one
@@ -1962,6 +1975,7 @@ int esb_subvolume_wbp(esb_reconstructor* r, const esb_vol_geom* full_vol, int n_
                    "esb_subvolume_wbp");
           }
         }
+        ESB_CK(subvol_patch_count(r->batch, r->stream), "esb_subvolume_wbp");
         return ok();
       }
       if (!r->batch.all_axis) {  // the general chords on the slab images

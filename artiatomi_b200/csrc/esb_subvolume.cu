@@ -482,9 +482,18 @@ cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, in
   if (!b.all_axis || b.n_work <= 0 || b.n_list <= 0) return cudaSuccess;
   const int np = b.n_particles, nl = b.n_list;
   b.off_slabs = align256((size_t)np * nl * sizeof(PatchInfo));
-  b.off_miss = b.off_slabs + align256((size_t)nl * sizeof(SlabTable));
-  const size_t bytes = b.off_miss + sizeof(unsigned long long);
+  const size_t bytes = b.off_slabs + (size_t)nl * sizeof(SlabTable);
   cudaError_t e;
+  if (!b.miss_host) {
+    if ((e = cudaHostAlloc((void**)&b.miss_host, sizeof(*b.miss_host), cudaHostAllocDefault)) != cudaSuccess)
+      return out_of_memory(e) ? cudaSuccess : e;
+    *b.miss_host = 0;
+  }
+  if (!b.miss_dev) {
+    if ((e = cudaMalloc((void**)&b.miss_dev, sizeof(*b.miss_dev))) != cudaSuccess)
+      return out_of_memory(e) ? cudaSuccess : e;
+    if ((e = cudaMemsetAsync(b.miss_dev, 0, sizeof(*b.miss_dev), st)) != cudaSuccess) return e;
+  }
   if ((e = staging(b.phost, b.phost_cap, b.pcopied, bytes)) != cudaSuccess) return out_of_memory(e) ? cudaSuccess : e;
   if ((e = device_buffer(b.pdev, b.pcap, bytes, st)) != cudaSuccess) return out_of_memory(e) ? cudaSuccess : e;
   const SubvolParticle* parts = (const SubvolParticle*)(b.host + b.off_parts);
@@ -591,7 +600,6 @@ cudaError_t subvol_patch_plan(SubvolBatch& b, const SlabTable* slabs, int pw, in
     max_floats = most / 2;
   }
   memcpy(b.phost + b.off_slabs, slabs, (size_t)nl * sizeof(SlabTable));
-  memset(b.phost + b.off_miss, 0, sizeof(unsigned long long));
   if ((e = cudaMemcpyAsync(b.pdev, b.phost, bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
   if ((e = cudaEventRecord(b.pcopied, st)) != cudaSuccess) return e;
   ok = true;
@@ -623,22 +631,25 @@ cudaError_t subvol_patch_launch(const SubvolBatch& b, int t0, int nt, int p0, in
   kernel<<<blocks, kQuadsPerItem, 0, st>>>(
       (const SubvolWork*)base + w0, n_work, (const SubvolParticle*)(base + b.off_parts),
       (const GridPair*)(base + b.off_pairs), (const PatchInfo*)pbase, (const SlabTable*)(pbase + b.off_slabs),
-      b.n_list, t0, nt, b.patches, 0, pw, ph, os, 0, subvol_odd(b),
-      (unsigned long long*)(pbase + b.off_miss));
+      b.n_list, t0, nt, b.patches, 0, pw, ph, os, 0, subvol_odd(b), b.miss_dev);
   ESB_COUNT_LAUNCH();
   return cudaGetLastError();
 }
 
-cudaError_t subvol_patch_misses(const SubvolBatch& b, cudaStream_t st, unsigned long long& misses) {
-  misses = 0;
-  if (!b.pdev) return cudaSuccess;
-  cudaError_t e = cudaMemcpyAsync(&misses, (const char*)b.pdev + b.off_miss, sizeof(misses), cudaMemcpyDeviceToHost,
-                                  st);
-  if (e != cudaSuccess) return e;
-  return cudaStreamSynchronize(st);
+cudaError_t subvol_patch_count(const SubvolBatch& b, cudaStream_t st) {
+  return cudaMemcpyAsync(b.miss_host, b.miss_dev, sizeof(*b.miss_host), cudaMemcpyDeviceToHost, st);
+}
+
+cudaError_t subvol_patch_misses(SubvolBatch& b, cudaStream_t st, unsigned long long& misses) {
+  misses = b.miss_host ? *(volatile unsigned long long*)b.miss_host : 0;
+  if (!misses) return cudaSuccess;
+  *b.miss_host = 0;
+  return cudaMemsetAsync(b.miss_dev, 0, sizeof(*b.miss_dev), st);
 }
 
 void subvol_batch_free(SubvolBatch& b) {
+  cudaFree(b.miss_dev);
+  b.miss_dev = nullptr;
   cudaFree(b.pdev);
   b.pdev = nullptr;
   b.pcap = 0;
@@ -655,6 +666,8 @@ void subvol_batch_free(SubvolBatch& b) {
   if (b.copied) cudaEventDestroy(b.copied);
   b.copied = nullptr;
   if (b.pcopied) cudaEventSynchronize(b.pcopied);
+  cudaFreeHost(b.miss_host);  // (the frees above waited for the last copy to it)
+  b.miss_host = nullptr;
   cudaFreeHost(b.phost);
   b.phost = nullptr;
   b.phost_cap = 0;

@@ -48,12 +48,13 @@ struct SubvolBatch {
   int all_axis = 0;  // every pair takes the single-axis sums
   // CTF patches (subvol_patch_plan): per pair the part of its tilt's slab
   // images that the box's quads read, gathered into one buffer
-  void* pdev = nullptr;  // patch table, slab tables, miss counter
+  void* pdev = nullptr;  // patch table, slab tables
   size_t pcap = 0;
   unsigned char* phost = nullptr;  // pinned staging copy of them
   size_t phost_cap = 0;
   cudaEvent_t pcopied = nullptr;
-  size_t off_slabs = 0, off_miss = 0;
+  size_t off_slabs = 0;
+  unsigned long long *miss_dev = nullptr, *miss_host = nullptr;  // miss counter, and its pinned copy
   float* patches = nullptr;
   size_t patches_cap = 0;  // bytes
   struct Chunk {
@@ -109,9 +110,12 @@ cudaError_t subvol_patch_sample(const SubvolBatch& b, int t, int p0, int p1, con
 cudaError_t subvol_patch_launch(const SubvolBatch& b, int t0, int nt, int p0, int p1, int pw, int ph, int os,
                                 cudaStream_t st);
 
-// Number of (quad, position) pairs whose samples the plan did not cover
-// (skipped, so nothing was read outside the patches); synchronises.
-cudaError_t subvol_patch_misses(const SubvolBatch& b, cudaStream_t st, unsigned long long& misses);
+// The quads (per position) whose samples a plan did not cover: they are left
+// out, so that nothing is read outside the patches, and counted on the device.
+// subvol_patch_count copies the count to pinned memory when the stream gets
+// there, subvol_patch_misses returns what has arrived and starts again from 0.
+cudaError_t subvol_patch_count(const SubvolBatch& b, cudaStream_t st);
+cudaError_t subvol_patch_misses(SubvolBatch& b, cudaStream_t st, unsigned long long& misses);
 
 void subvol_batch_free(SubvolBatch& b);
 

@@ -469,6 +469,11 @@ class Reconstructor:
         particles beyond it take further launches."""
         check(lib.esb_reconstructor_subvolume_patch_bytes(self._h, int(n)))
 
+    def subvolume_check(self):
+        """Waits for subvolume_wbp's launches and raises if one of them left
+        out samples that its planned patches did not hold."""
+        check(lib.esb_reconstructor_subvolume_check(self._h))
+
     def timing(self):
         """{phase: (ms, launches)} since the previous call; phases fp, bp, ctf, compare."""
         ms = np.zeros(4, np.float64)

@@ -221,6 +221,7 @@ def reconstruct_subvolumes(cfg: EmSartConfig, write: bool = True, batched: bool 
     for b in subvolume_batches(cfg, R.markers, R.tc, vg, R.W, R.H, rank, world):
         boxes = [torch.zeros((S, S, S), dtype=torch.float32, device=dev) for _ in b.parts]
         rec.subvolume_wbp(vg, b.sub, b.pair, boxes, R.prepared, index_list, active=b.active, batched=batched)
+        rec.subvolume_check()
         torch.cuda.synchronize()
         for k, p in enumerate(b.parts):
             name = cfg.SubVolPath + F.index_coding(motl[p], cfg.NamingConvention == 1) + ".em"

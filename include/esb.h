@@ -402,6 +402,12 @@ int esb_reconstructor_subvolume_patches(esb_reconstructor* rec, int enable);
  * slab images by one launch each. */
 int esb_reconstructor_subvolume_patch_bytes(esb_reconstructor* rec, size_t bytes);
 
+/* Waits for the reconstructor's stream and fails if an esb_subvolume_wbp call
+ * left out samples that its planned patches did not hold (none, by the
+ * plan's margins; esb_subvolume_wbp itself does not wait, and fails for the
+ * calls before it that have finished). */
+int esb_reconstructor_subvolume_check(esb_reconstructor* rec);
+
 /* ResetProjectionsDevice (Reconstructor.cpp:1678-1682). */
 int esb_rec_reset_projections(esb_reconstructor* rec);
 /* ForwardProjection (Reconstructor.cpp:1411-1421), CTF or not. */

@@ -255,6 +255,7 @@ def _subvolume_gpu(c, batched, index_list, active=None, patches=None, patch_byte
     boxes = [cuda(np.zeros((s, s, s), np.float32)) for s in c["sizes"]]
     rec.subvolume_wbp(c["full"], c["sub"], c["pair"], boxes, cuda(c["projs"]), index_list, active=active,
                       batched=batched)
+    rec.subvolume_check()  # no sample outside the planned patches
     return [host(b) for b in boxes]
 
 
@@ -309,20 +310,23 @@ def test_batched_subvolume_matches_per_particle(ctf):
 
 @pytest.mark.parametrize("psi_deg", [0.0, 0.7])
 def test_subvolume_ctf_patches_match_per_tilt(psi_deg):
-    """With CTF the batched call gathers, after each tilt's CTF chain, the
-    patch of the slab images each box reads, and adds all tilts in one
-    launch (esb_reconstructor_subvolume_patches). One launch per tilt over
-    the whole slab images gives the same boxes bit for bit: the same sums in
-    the same order, patch texels equal to the clamped image texels (boxes
-    here reach past the detector edge). 4 nm slabs: boxes span several."""
+    """With CTF the batched call evaluates, after each tilt's CTF chain, the
+    patch of the slab images each box reads. All tilts in one launch
+    (esb_reconstructor_subvolume_patches) and one launch per tilt from that
+    tilt's patches give the same boxes bit for bit: the same sums in the same
+    order. Both against the launches per particle, which read the whole slab
+    images, to rounding (boxes here reach past the detector's edge; 4 nm slabs:
+    boxes span several)."""
     c = _subvolume_case(True, [16, 24, 32, 48, 16, 24], n=9, seed=5, psi_deg=psi_deg)
     il = np.random.default_rng(1).permutation(c["n"]).astype(np.int32)
     active = (np.linalg.norm(c["shifts"], axis=2) < 1.5).astype(np.uint8)
     one = _subvolume_gpu(c, True, il, active, patches=True)
     per_tilt = _subvolume_gpu(c, True, il, active, patches=False)
-    for a, b in zip(per_tilt, one):
+    images = _subvolume_gpu(c, False, il, active)
+    for a, b, d in zip(per_tilt, one, images):
         assert np.abs(a).sum() > 0
         np.testing.assert_array_equal(b, a)
+        assert rel_l2(b, d) <= 1e-5
 
 
 @pytest.mark.parametrize("patches", [False, True])
