@@ -962,18 +962,30 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
 // the G + 2 y planes that the rays interpolate between,
 //   S + e Se + f Sf + e f Sef,
 // formed once per line; only the blend of two planes and the offset are a
-// ray's own. A sample that the offset carries across a cell's face (offsets
-// are kept below 1/64 voxel) is evaluated on the face's other side: the
-// interpolant is continuous there, and the difference, a kink times less than
-// 1/64 in one sample of a hundred, is a tenth of what the rounding of the
-// ray's float start point (5e-4 voxels, all samples) makes.
+// ray's own.
+//
+// A sample that the offset carries across a cell's face is evaluated on the
+// face's other side, off by the distance past the face times the kink there.
+// The sum of those errors grows with the offset's power 3/2, the walk's own
+// error, from the rounding of a ray's float start point, with the beam's
+// inclination. So offsets are bounded by kMaxShear and by a quarter of the
+// minor step; beams next to a volume axis, where whole rays would lie on the
+// far side of a face, thereby take the walk per ray. Against sums in 64 bits,
+// 389 x 421 x 96, lines / walk per ray, beams of 0 to 60 degrees, rotations
+// of 0.03 to 0.38: a smooth density with a tenth of noise, ratio at most
+// 1.004; white noise, the worst case, at most 1.18 (1.38e-4 / 1.17e-4 at 11
+// degrees). Offsets of up to 1/64 at any inclination gave 1.12 and 2.5, and
+// 17 and 45 at 0 degrees. Correcting those samples one by one makes lines and
+// walk agree to 1e-6, but every lane reads the volume at another layer: 93 ms
+// where the walk per ray takes 61.
 //
 // Per ray and layer that leaves a 2 G-th of the weights, control and loads
 // of each plane in place of all of them for two planes. What bounds it: the
 // latency of a layer's loads at 12 to 16 warps per SM (issue 52 % busy, FMA
 // pipe 35 %); caps of 96 and 80 registers (20 and 24 warps) spill and took
 // 33.5 and 44.3 ms where 128 take 33.3. 1024 x 1024 x 256, 16 tilts with 0.3
-// degrees jitter, CTF slabs: 61.1 ms with k_slicer_axis -> 33.3; 256 x 256 x
+// degrees jitter, CTF slabs: 61.1 ms with k_slicer_axis -> 39.5 (33.3 where
+// offsets may reach 1/64); 256 x 256 x
 // 128, 41 tilts: 7.3 ms with k_project_axis -> 3.2 (4 runs). A warp holds 16
 // detector rows x 2 sub-rows, so that its loads of a plane are contiguous.
 // `swap` exchanges u and v (a tilt axis across the image).
@@ -982,17 +994,17 @@ struct PlaneWalk {
   int nM, nN;          // voxels along the major and minor axis
   unsigned dM, dN;     // their strides in bytes
 };
-constexpr float kMaxShear = 1.0f / 64.0f;
+constexpr float kMaxShear = 1.0f / 144.0f;  // voxels
 
 // Plane sums over samples j0 .. J-1 of one ray: S[0] of the weights, and with
-// SH > 0 S[1], S[2] of their derivatives along the mirrored minor and major
-// axis, with SH > 1 S[3] of the mixed one; yoff: byte offsets of the planes
+// SHEAR S[1], S[2] of their derivatives along the mirrored minor and major
+// axis and S[3] of the mixed one; yoff: byte offsets of the planes
 // (32-bit: the volume is below 4 GiB).
-template <int VT, int NP, int SH>
+template <int VT, int NP, bool SHEAR>
 __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W, const void* __restrict__ vol,
                                            const unsigned (&yoff)[NP], float Mq, float Nq, int j0, int J,
-                                           float (&S)[SH == 0 ? 1 : SH + 2][NP]) {
-  constexpr int NS = SH == 0 ? 1 : SH + 2;
+                                           float (&S)[SHEAR ? 4 : 1][NP]) {
+  constexpr int NS = SHEAR ? 4 : 1;
   typedef typename RawVoxel<VT>::T Raw;
   const char* const base = (const char*)vol;
   const float fj0 = (float)j0, jb = fj0 - 0.5f;
@@ -1062,14 +1074,12 @@ __device__ __forceinline__ void plane_sums(const AxisStep& A, const PlaneWalk& W
     far[0][0] = uA;
     far[0][1] = tA + uB;
     far[0][2] = tB;
-    if constexpr (SH > 0) {
+    if constexpr (SHEAR) {
       const float vA = MA - McA, vB = MB - McB, wA = MA - MaA, wB = MB - MaB;
       n[1][0] = -vA, n[1][1] = vA - vB, n[1][2] = vB;
       far[1][0] = -McA, far[1][1] = McA - McB, far[1][2] = McB;
       n[2][0] = -wA, n[2][1] = -(MaA + wB), n[2][2] = -MaB;
       far[2][0] = wA, far[2][1] = MaA + wB, far[2][2] = MaB;
-    }
-    if constexpr (SH > 1) {
       n[3][0] = MA, n[3][1] = MB - MA, n[3][2] = -MB;
       far[3][0] = -MA, far[3][1] = MA - MB, far[3][2] = MB;
     }
@@ -1177,11 +1187,11 @@ struct PlaneRay {
 // Sums v[] of the line's sub-rays, each over its [tin, tout] cut to [lo, hi]
 // (0 for those outside). slab: the first sample is the one at the ray's
 // start; else run `seg` of `segs` of the samples (axis_ray_sum).
-template <int VT, int G, int SH>
+template <int VT, int G, bool SHEAR>
 __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, const PlaneWalk& W, int zmaj,
                                           const void* vol, const PlaneLine<G>& L, const unsigned (&yoff)[G + 2],
                                           bool slab, float lo, float hi, int seg, int segs, float* v) {
-  constexpr int N = 2 * G, NP = G + 2, NS = SH == 0 ? 1 : SH + 2;
+  constexpr int N = 2 * G, NP = G + 2, NS = SHEAR ? 4 : 1;
   float S[NS][NP];
 #pragma unroll
   for (int q = 0; q < NS; ++q)
@@ -1201,7 +1211,7 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
   }
   const int j0 = slab ? 1 : run_start(Jm, seg, segs), j1 = slab ? Jm : run_start(Jm, seg + 1, segs);
   if (mid && j0 < j1)
-    plane_sums<VT, NP, SH>(A, W, vol, yoff, W.sM > 0 ? bm : -bm, W.sN > 0 ? bn : -bn, j0, j1, S);
+    plane_sums<VT, NP, SHEAR>(A, W, vol, yoff, W.sM > 0 ? bm : -bm, W.sN > 0 ? bn : -bn, j0, j1, S);
   float P[NS][NP];  // (indexed by a ray's planes: local memory)
 #pragma unroll
   for (int q = 0; q < NS; ++q)
@@ -1216,7 +1226,7 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
     const PlaneRay R(c, A, L.s[g], t0, t1, L.b[g]);
     const float f = ((zmaj ? R.q.z : R.q.x) - bm) * (float)W.sM, e = ((zmaj ? R.q.x : R.q.z) - bn) * (float)W.sN;
     const bool joins = mid && R.ok && L.cell[g] <= G && abs(R.J - Jm) <= 1 &&
-                       (SH == 0 ? e == 0.f && f == 0.f : fabsf(e) <= kMaxShear && fabsf(f) <= kMaxShear);
+                       (SHEAR ? fabsf(e) <= kMaxShear && fabsf(f) <= kMaxShear : e == 0.f && f == 0.f);
     if (!joins) {
       if (seg == 0) v[g] = other_ray_sum<VT>(&c, vol, L.s[g], t0, t1, slab);
       continue;
@@ -1226,8 +1236,7 @@ __device__ __forceinline__ void line_sums(const KConst& c, const AxisStep& A, co
     for (int h = 0; h < 2; ++h) {
       const int p = L.cell[g] + h;
       sum[h] = P[0][p];
-      if constexpr (SH > 0) sum[h] = fmaf(e, P[1][p], fmaf(f, P[2][p], sum[h]));
-      if constexpr (SH > 1) sum[h] = fmaf(e * f, P[3][p], sum[h]);
+      if constexpr (SHEAR) sum[h] = fmaf(e * f, P[3][p], fmaf(e, P[1][p], fmaf(f, P[2][p], sum[h])));
     }
     float r = fmaf(L.b[g], sum[1], (1.0f - L.b[g]) * sum[0]);
     if (R.J != Jm && seg == segs - 1) {  // one sample more or less than the middle ray
@@ -1272,7 +1281,7 @@ __device__ __forceinline__ float pixel_sum(const float* v, int i, int swap) {
   return swap ? __fadd_rn(__fadd_rn(__fadd_rn(a, b), c), d) : __fadd_rn(__fadd_rn(__fadd_rn(a, c), b), d);
 }
 
-template <int VT, int G, int SH>
+template <int VT, int G, bool SHEAR>
 __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ KConst c,
                                                         const __grid_constant__ AxisStep A,
                                                         const __grid_constant__ PlaneWalk W, int zmaj, int swap, int segs,
@@ -1286,7 +1295,7 @@ __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ 
   L.in = 0;
   if (P.active) {
     L.template init<VT>(c, vol, P.x, P.y, swap, false, yoff);
-    line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, false, -FLT_MAX, FLT_MAX, P.seg, segs, v);
+    line_sums<VT, G, SHEAR>(c, A, W, zmaj, vol, L, yoff, false, -FLT_MAX, FLT_MAX, P.seg, segs, v);
   } else {
 #pragma unroll
     for (int g = 0; g < 2 * G; ++g) v[g] = 0.0f;
@@ -1313,7 +1322,7 @@ __global__ void __launch_bounds__(128) k_project_planes(const __grid_constant__ 
   }
 }
 
-template <int VT, int G, int SH>
+template <int VT, int G, bool SHEAR>
 __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ KConst c,
                                                        const __grid_constant__ AxisStep A,
                                                        const __grid_constant__ PlaneWalk W, int zmaj, int swap,
@@ -1358,7 +1367,7 @@ __global__ void __launch_bounds__(128) k_slicer_planes(const __grid_constant__ K
   for (int k = ka; k < kb; ++k) {
     float v[2 * G];
     if (L.in) {
-      line_sums<VT, G, SH>(c, A, W, zmaj, vol, L, yoff, true, slabs.bound[k], slabs.bound[k + 1], 0, 1, v);
+      line_sums<VT, G, SHEAR>(c, A, W, zmaj, vol, L, yoff, true, slabs.bound[k], slabs.bound[k + 1], 0, 1, v);
     } else {
 #pragma unroll
       for (int g = 0; g < 2 * G; ++g) v[g] = 0.f;
@@ -1427,8 +1436,10 @@ struct PlaneLaunch {
     shear = ex > 0.f || ez > 0.f ? 1 : 0;
     for (int g = 4; g >= 2 && !G; g -= 2) {
       // the offset of the line's outermost ray, taken at its start or along
-      // the ray to the volume's face, and its planes
-      const bool small = (float)g * (ex + ez) <= kMaxShear;
+      // the ray to the volume's face, against its bounds (above), and the
+      // line's planes
+      const float offset = (float)g * (ex + ez);
+      const bool small = !shear || (offset <= kMaxShear && 4.0f * offset <= A.dN);
       const bool planes = (float)(2 * g - 1) * ey < (float)g - 0.05f;
       // 2 pixels per thread from 2 warps per scheduler on, 4 from 4, runs
       // counted. Measured without runs: 128 warps of 2 pixels 25 us against
@@ -1478,8 +1489,8 @@ bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 
 // A launch of a plane kernel (ESB_PLANES), 4 warps per block.
 #define ESB_PLANES_SH(VT, GG)              \
   do {                                     \
-    if (L.shear) ESB_PLANES(VT, GG, 1);    \
-    else ESB_PLANES(VT, GG, 0);            \
+    if (L.shear) ESB_PLANES(VT, GG, true); \
+    else ESB_PLANES(VT, GG, false);        \
   } while (0)
 #define ESB_PLANES_VT(VT)                  \
   do {                                     \
@@ -1523,7 +1534,7 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
   if (L.G) {
     const int segs = 1, slab_parts = L.parts(x1 - x0, y1 - y0, slabs.count);
 #define ESB_PLANES(VT, GG, SH)                                                                                        \
-  k_slicer_planes<VT, GG, SH ? 2 : 0><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, imgs, img_stride, pitchE, \
+  k_slicer_planes<VT, GG, SH><<<grd, blk, 0, st>>>(c, L.A, L.W, L.zmaj, L.swap, vol, imgs, img_stride, pitchE, \
                                                            slabs, clear, x0, y0, x1, y1)
     ESB_PLANES_LAUNCH();
 #undef ESB_PLANES
