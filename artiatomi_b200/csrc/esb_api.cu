@@ -43,6 +43,8 @@ cudaError_t launch_bp_fast_slabs(const KConst& k, void* vol, int vt, const float
                                  const BpShape* shape = nullptr);
 cudaError_t launch_upsample(const KConst& k, const float* imgs, size_t img_stride, int count, int pw, int ph, int os,
                             int linear, float2* up, size_t up_stride, OddFlag odd, cudaStream_t st);
+bool slicer_takes_nw(const KConst& c, int vt, int pw, int ph);
+bool project_takes_nw(const KConst& c, int vt, int pw, int ph);
 bool bp_can_upsample(const KConst& k, int os);
 bool bp_reads_at_samples(const KConst& k, int os);
 bool bp_uses_axis(const KConst& k, int os, bool up);
@@ -762,7 +764,8 @@ int esb_rec_reset_projections(esb_reconstructor* r) {
 namespace {
 struct TuneKey {
   int kernel, dev, sms, vt, w, h, dx, dy, dz, os, ctf;
-  auto tie() const { return std::tie(kernel, dev, sms, vt, w, h, dx, dy, dz, os, ctf); }
+  int one;  // 1: launches that no candidate changes
+  auto tie() const { return std::tie(kernel, dev, sms, vt, w, h, dx, dy, dz, os, ctf, one); }
   bool operator<(const TuneKey& o) const { return tie() < o.tie(); }
 };
 std::mutex g_tune_mu;
@@ -775,12 +778,12 @@ const int kNBpShapes = 5;
 const char* kTuneNames[] = {"fp_slicer_fused", "fp_march", "bp_axis"};
 }  // namespace
 
-static TuneKey tune_key(esb_reconstructor* r, int kernel, int vt, const KConst& c, int ctf) {
+static TuneKey tune_key(esb_reconstructor* r, int kernel, int vt, const KConst& c, int ctf, bool choice = true) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return TuneKey{kernel, dev, sms, vt, r->cfg.proj_x, r->cfg.proj_y, (int)c.dim.x, (int)c.dim.y, (int)c.dim.z,
-                 r->cfg.oversampling, ctf};
+                 r->cfg.oversampling, ctf, choice ? 0 : 1};
 }
 
 static void* rec_tune_scratch(esb_reconstructor* r, size_t bytes) {
@@ -809,6 +812,10 @@ static int rec_tuned(esb_reconstructor* r, const TuneKey& key, int n, int def, R
     if (it != g_tune.end()) return it->second;
   }
   if (!g_tune_on.load()) return def;
+  if (n == 1) {  // nothing to try
+    std::lock_guard<std::mutex> lock(g_tune_mu);
+    return g_tune[key] = def;
+  }
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(r->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -897,7 +904,8 @@ extern "C" int esb_autotune_report(char* buf, size_t len, size_t* needed) {
 static int rec_slicer_nw(esb_reconstructor* r, const KConst& c, const void* vol, int vt, size_t img,
                          const SlabTable& T) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y;
-  const int i = rec_tuned(r, tune_key(r, 0, vt, c, 1), 3, 0, [&](int k) {
+  const bool choice = slicer_takes_nw(c, vt, W, H);
+  const int i = rec_tuned(r, tune_key(r, 0, vt, c, 1, choice), choice ? 3 : 1, 0, [&](int k) {
     return launch_slicer_fused(c, vol, vt, r->slab_imgs, img, W, T, 1, W, H, 0, 0, W, H, r->stream, kNw[k]);
   });
   return kNw[i];
@@ -908,7 +916,8 @@ static int rec_slicer_nw(esb_reconstructor* r, const KConst& c, const void* vol,
 static int rec_march_nw(esb_reconstructor* r, const KConst& c, const void* vol, int vt) {
   const int W = r->cfg.proj_x, H = r->cfg.proj_y;
   const size_t img = (size_t)W * H;
-  const int i = rec_tuned(r, tune_key(r, 1, vt, c, 0), 3, 0, [&](int k) {
+  const bool choice = project_takes_nw(c, vt, W, H);
+  const int i = rec_tuned(r, tune_key(r, 1, vt, c, 0, choice), choice ? 3 : 1, 0, [&](int k) {
     float* s = (float*)rec_tune_scratch(r, 2 * img * sizeof(float));
     if (!s) return cudaErrorMemoryAllocation;
     return launch_project_fast(c, vol, vt, 0, s, s + img, W, 0.f, 0.f, W, H, 0, 0, W, H, r->stream, kNw[k]);

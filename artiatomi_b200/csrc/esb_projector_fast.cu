@@ -1460,10 +1460,32 @@ struct PlaneLaunch {
   }
 };
 
+// Runs of a ray's samples in k_project_axis, by the whole detector's warps of
+// one pixel across: they, and with them the order of a ray's sum, depend
+// neither on the block shape nor on the region.
+int axis_runs(const KConst& c, bool zmaj, int pw, int ph) {
+  const dim3 warps = axis_grid(axis_swap(c), 1, pw, ph);
+  return max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 148.0 * 32, 8));
+}
+
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.
 bool big_volume(const KConst& c) { return (double)c.dim.x * c.dim.y * c.dim.z > 4294967295.0; }
 
 }  // namespace
+
+// Whether nw (warps per block) makes a difference to launch_slicer_fused and
+// launch_project_fast (mode 0): not to lines of rays, rays cut into runs and
+// volumes with 64-bit offsets.
+bool slicer_takes_nw(const KConst& c, int vt, int pw, int ph) {
+  return axis_projection(c) ? PlaneLaunch(c, vt, pw, ph, 1).G == 0 : !big_volume(c);
+}
+bool project_takes_nw(const KConst& c, int vt, int pw, int ph) {
+  if (!axis_projection(c)) return !big_volume(c);
+  bool zmaj;
+  int sm, sn;
+  axis_step(c, zmaj, sm, sn);
+  return PlaneLaunch(c, vt, pw, ph, max_runs(c, zmaj, 4)).G == 0 && axis_runs(c, zmaj, pw, ph) == 1;
+}
 
 // nw: warps per block (2, 4 or 8; 64-bit-offset volumes always take 4).
 
@@ -1588,11 +1610,7 @@ cudaError_t launch_project_fast(const KConst& c, const void* vol, int vt, int mo
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
     dim3 grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    // (the whole detector's warps of one pixel across: the runs, and with them
-    // the order of a ray's sum, depend neither on the block shape nor on the
-    // region)
-    const dim3 warps = axis_grid(swap, 1, pw, ph);
-    const int segs = max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 148.0 * 32, 8));
+    const int segs = axis_runs(c, zmaj, pw, ph);
     if (segs > 1) {
       nw = 8;
       grd = axis_grid(swap, nw / segs, x1 - x0, y1 - y0);

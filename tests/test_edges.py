@@ -364,3 +364,26 @@ def test_autotuned_projector_shapes_cut_rays_alike(size):
     assert np.abs(out[0]).max() > 0
     for j in range(2, 6):
         np.testing.assert_array_equal(out[j], out[j % 2])
+
+
+@pytest.mark.gpu
+def test_nothing_is_tried_where_candidates_are_one_launch():
+    """Lines of rays take no warps per block: the first projection of a shape
+    is one launch, as every later one."""
+    import artiatomi_b200 as E
+
+    dims, W, H = (256, 256, 16), 256, 256
+    tilt = np.array([20.0, 35.0], np.float32)
+    rec = E.Reconstructor(E.ReconConfig(W, H, 2, variant=E.VARIANT_FAST),
+                          E.projection_geometry(E.Markers(tilt), W, H), tilt)
+    vg, vol = E.volume_geometry(dims), cuda(np.ones(dims[::-1], np.float32))
+    E.autotune(-1)
+    counts = []
+    for i in range(2):
+        rec.reset_projections()
+        before = E.kernel_launches()
+        rec.forward_projection(vg, vol, i)
+        counts.append(E.kernel_launches() - before)
+    assert counts == [1, 1], counts
+    assert "fp_march" in E.autotune_report()
+    rec.close()
