@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) k_cc_peaks(const float* __restrict__
 
 inline int grid_for(long n) {
   long g = (n + kThreads - 1) / kThreads;
-  return (int)(g < 1 ? 1 : (g > 148 * 8 ? 148 * 8 : g));
+  return (int)(g < 1 ? 1 : (g > kSMs * 8 ? kSMs * 8 : g));
 }
 
 }  // namespace

@@ -45,6 +45,10 @@ inline KConst to_kconst(const esb_constants& c) {
   return k;
 }
 
+// Streaming multiprocessors of a B200. The rules that split work by it use the
+// constant, not the device's count: some of them choose the order of a sum.
+constexpr int kSMs = 148;
+
 // Defocus slabs of one projection (the reference's loop
 // for (ray = t_in; ray < t_out; ray += thickness), Reconstructor.cpp:515,
 // 935): slab k spans bound[k] <= t < bound[k+1] with the float recurrence

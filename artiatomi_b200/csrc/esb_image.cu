@@ -570,7 +570,7 @@ cudaError_t launch_crop_upsample(const KConst& k, int pw, int ph, float* img, fl
                                  int os, float2* up, OddFlag odd, cudaStream_t st) {
   const bpcore::BpGeom g = bpcore::make_geom(k, os);
   const int swapped = bpcore::axis_beam(k, g) && bpcore::up_swapped(bpcore::make_axis_geom(k, g, os)) ? 1 : 0;
-  const int tile = (long)((pw + 31) / 32) * ((ph + 31) / 32) >= 296 ? 32 : 16;  // two 32 x 32 tiles per SM
+  const int tile = (long)((pw + 31) / 32) * ((ph + 31) / 32) >= 2 * kSMs ? 32 : 16;  // two 32 x 32 tiles per SM
   const dim3 b(tile, 256 / tile), grd((pw + tile - 1) / tile, (ph + tile - 1) / tile);
   const auto kernel = tile == 32 ? k_crop_upsample<32> : k_crop_upsample<16>;
   kernel<<<grd, b, 0, st>>>(pw, ph, img, cut, dim, make_int2(p[0], p[1]), make_int2(p[2], p[3]),
@@ -658,7 +658,7 @@ cudaError_t launch_transpose(const float* in, int w, int h, size_t pitchE, float
 
 static inline int grid1(long n) {
   long b = (n + 255) / 256;
-  return (int)(b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16);
+  return (int)(b < kSMs * 16 ? (b < 1 ? 1 : b) : kSMs * 16);
 }
 
 cudaError_t launch_convert_input(const void* in, int type, long n, float* out, cudaStream_t st) {
@@ -706,7 +706,7 @@ cudaError_t launch_normalize(const float* in, float* out, long n, float mean, fl
 // Blocks of 256 columns, about 8 blocks per SM over the rows.
 static inline dim3 rows_grid(int w, int h) {
   const int gx = (w + 255) / 256;
-  return dim3(gx, std::max(1, std::min(h, 148 * 8 / gx)));
+  return dim3(gx, std::max(1, std::min(h, kSMs * 8 / gx)));
 }
 
 cudaError_t launch_prepare_square(const void* in, int type, int pw, int ph, int n, int bx, int by, int mirrorY,
@@ -765,7 +765,7 @@ cudaError_t launch_dose_weighting(float* spec, int n, float dose, float pixelsiz
 }
 
 cudaError_t launch_convert(const void* vol, int vt, long n, float* out, float sign, cudaStream_t st) {
-  int blocks = (int)((n + 255) / 256 < 148 * 32 ? (n + 255) / 256 : 148 * 32);
+  int blocks = (int)((n + 255) / 256 < kSMs * 32 ? (n + 255) / 256 : kSMs * 32);
   if (blocks < 1) blocks = 1;
   switch (vt) {
     case ESB_VOXEL_F32: k_convert<ESB_VOXEL_F32><<<blocks, 256, 0, st>>>(vol, n, out, sign); ESB_COUNT_LAUNCH(); break;
@@ -776,7 +776,7 @@ cudaError_t launch_convert(const void* vol, int vt, long n, float* out, float si
 }
 
 cudaError_t launch_store(const float* in, long n, void* vol, int vt, cudaStream_t st) {
-  int blocks = (int)((n + 255) / 256 < 148 * 32 ? (n + 255) / 256 : 148 * 32);
+  int blocks = (int)((n + 255) / 256 < kSMs * 32 ? (n + 255) / 256 : kSMs * 32);
   if (blocks < 1) blocks = 1;
   switch (vt) {
     case ESB_VOXEL_F32: k_store<ESB_VOXEL_F32><<<blocks, 256, 0, st>>>(in, n, vol); ESB_COUNT_LAUNCH(); break;

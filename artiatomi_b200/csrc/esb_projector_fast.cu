@@ -1419,7 +1419,7 @@ struct PlaneLaunch {
     return (double)((across + g - 1) / g) * ((along + 15) / 16);
   }
   // Parts, runs or slabs, for them to fill the GPU.
-  int parts(int w, int h, int max_parts) const { return parts_for(warps(w, h, G), 148.0 * 16, max_parts); }
+  int parts(int w, int h, int max_parts) const { return parts_for(warps(w, h, G), 16.0 * kSMs, max_parts); }
   // runs: how often a ray's samples may be cut into runs
   PlaneLaunch(const KConst& c, int vt, int w, int h, int runs) {
     bool z;
@@ -1447,7 +1447,7 @@ struct PlaneLaunch {
       // pixels 141, and with 4 runs 78. Slabs do not count: they are few
       // layers each, and 1024 warps of 4 pixels with their slabs spread took
       // 105 us where 2048 of 2 pixels take 72.
-      const bool enough = warps(w, h, g) * runs >= 148.0 * 4 * g;
+      const bool enough = warps(w, h, g) * runs >= 4.0 * kSMs * g;
       if (small && planes && enough) G = g;
     }
     const unsigned es = vt == ESB_VOXEL_F32 ? 4 : 2, sz = es * (unsigned)c.dim.x * (unsigned)c.dim.y;
@@ -1465,7 +1465,7 @@ struct PlaneLaunch {
 // neither on the block shape nor on the region.
 int axis_runs(const KConst& c, bool zmaj, int pw, int ph) {
   const dim3 warps = axis_grid(axis_swap(c), 1, pw, ph);
-  return max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 148.0 * 32, 8));
+  return max_runs(c, zmaj, parts_for((double)warps.x * warps.y, 32.0 * kSMs, 8));
 }
 
 // Volumes of 2^32 voxels or more take 64-bit element offsets in the walk.
@@ -1565,7 +1565,7 @@ cudaError_t launch_slicer_fused(const KConst& c, const void* vol, int vt, float*
     if (nw != 2 && nw != 8) nw = 4;
     const int swap = axis_swap(c);
     dim3 blk(32 * nw), grd = axis_grid(swap, nw, x1 - x0, y1 - y0);
-    grd.z = parts_for((double)grd.x * grd.y * nw, 148.0 * 32, slabs.count);
+    grd.z = parts_for((double)grd.x * grd.y * nw, 32.0 * kSMs, slabs.count);
     ESB_AXIS_LAUNCH(k_slicer_axis, grd, blk, st, vol, imgs, img_stride, pitchE, slabs, clear, swap, x0, y0, x1, y1);
     ESB_COUNT_LAUNCH();
     return cudaGetLastError();

@@ -610,7 +610,7 @@ cudaError_t subvol_patch_sample(const SubvolBatch& b, int t, int p0, int p1, con
                                 int pw, int ph, int os, cudaStream_t st) {
   if (p1 <= p0) return cudaSuccess;
   // about 2000 blocks, however few the particles
-  const unsigned gx = (unsigned)std::min(p1 - p0, 148 * 8);
+  const unsigned gx = (unsigned)std::min(p1 - p0, kSMs * 8);
   const dim3 grd(gx, std::max(1u, std::min(16u, 2048u / gx)));
   k_patch_sample<<<grd, 256, 0, st>>>((const PatchInfo*)b.pdev + (size_t)p0 * b.n_list, p1 - p0, b.n_list, t, imgs,
                                       img_stride, pw, ph, 1.0f / (float)os, b.patches, subvol_odd(b));
