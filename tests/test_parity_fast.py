@@ -118,8 +118,9 @@ def test_fast_back_projection_exact_chords(case, os_, linear, slab):
 @pytest.mark.parametrize("sirt,os_,aniso", [(1, 1, False), (3, 2, False), (2, 3, False), (3, 2, True)])
 def test_fast_sart_volume(sirt, os_, aniso):
     """FAST SART against the oracle (FP32 1e-3, FP64 2e-4). Oversampling 3
-    and magnification anisotropy take the back-projector that filters the
-    residual itself (no pre-sampled images)."""
+    takes the back-projector that filters the residual itself; the others read
+    pre-sampled images, with magnification anisotropy sampled through its
+    inverse."""
     import artiatomi_b200 as E
     from oracle.driver import OracleReconstructor
     from tests.test_parity_recon import _projections
@@ -210,6 +211,46 @@ def test_fast_sart_ctf():
         orc.sart(case["vo"], vo, 0, projs, il, 2, 2)
         e = rel_l2(got, vo)
         assert e <= tol, (prec, e)
+
+
+@pytest.mark.parametrize("psi,aniso", [(0.3, True), (87.0, False), (87.0, True)])
+def test_fast_ctf_back_projection_of_sampled_images(psi, aniso):
+    """The pre-sampled slab images of an odd detector: bilinear, through the
+    magnification anisotropy, and with the tilt axis across the image (the
+    image's fast axis along u), several slabs, against the FP64 oracle. As in
+    the tests of SART, a quad takes the slab and the macro cell of its first
+    corner in float here: 1e-3, or 1.5 times the deviation of the reference's
+    own float arithmetic."""
+    import artiatomi_b200 as E
+    from oracle import geometry as G
+    from oracle.driver import OracleReconstructor
+    from tests.test_parity_recon import _ctf_cfg
+
+    dims, W, H, tilt = (76, 66, 24), 81, 77, np.array([-50.0, -12.0, 31.0], np.float32)
+    n = len(tilt)
+    xs, ys, ps = np.array([0.7, -0.4, 0.2], np.float32), np.array([-0.3, 0.6, 0.1], np.float32), np.full(n, psi, np.float32)
+    pg = E.projection_geometry(E.Markers(tilt, xs, ys, None, ps), W, H)
+    og = G.projection_geometry(tilt, xs, ys, None, ps, W, H)
+    vg, vo = E.volume_geometry(dims), G.volume_geometry(dims)
+    defocus = _defocus(n, 5)
+    cfgd = dict(_ctf_cfg(W), oversampling=2)
+    m = mi = None
+    if aniso:
+        m, mi = E.mag_aniso_matrix(1.03, 25.0, W, H), E.mag_aniso_matrix(1.0 / 1.03, 25.0, W, H)
+    rec = E.Reconstructor(E.ReconConfig(W, H, n, variant=E.VARIANT_FAST, **cfgd), pg, tilt, defocus, m, mi)
+    imgs = np.random.default_rng(6).normal(size=(n, H, W)).astype(np.float32)
+    vol = cuda(np.zeros(dims[::-1], np.float32))
+    refs = [np.zeros(dims[::-1], np.float32) for _ in range(2)]
+    for i in range(n):
+        rec.views()[0].copy_(cuda(imgs[i]))
+        rec.back_projection(vg, vol, i, 2.0)
+    for precision in (0, 1):
+        orc = OracleReconstructor(cfgd, W, H, og, tilt, defocus, aniso=m, aniso_inv=mi, precision=precision)
+        for i in range(n):
+            orc.back_projection(vo, refs[precision], 0, i, 2.0, img=imgs[i].copy())
+    tol = max(1e-3, 1.5 * rel_l2(refs[0], refs[1]))
+    assert np.abs(refs[1]).max() > 0 and tol < 0.02
+    assert rel_l2(host(vol), refs[1]) <= tol, (rel_l2(host(vol), refs[1]), tol)
 
 
 def _subvolume_case(ctf, sizes, n=7, seed=31, psi_deg=0.0):
