@@ -685,23 +685,23 @@ __device__ __forceinline__ float axis_walk(const AxisStep& A, const Cell<VT>& C,
   Raw va = Raw(0), vb, vc, vd = Raw(0), wa = Raw(0), wb, wc, wd = Raw(0);
   float nMs = 0.f, nNs = 0.f;
   bool X = false, Xp = false;  // a minor crossing in this layer, in the one before
-  // row im with its window, clamped; the outer positions where they have a
-  // weight (0 times an infinite voxel or NaN is NaN)
+  // row im with its window, clamped; the outer positions 0 where they have no
+  // weight (0 times an infinite voxel or NaN is NaN; loads under predicates
+  // made small volumes 3 % slower)
   auto fetch = [&]() {
     nMs = __fmaf_rn(k, A.isM, nM0);
     nNs = __fmaf_rn(kn, A.isN, nN0);
     X = nNs <= nMs;
     const char* p = clamped(im, in0 - SN);
-    va = wa = vd = wd = Raw(0);
-    ldraw_if<VT>(va, p, Xp);
-    ldraw_if<VT>(wa, p + dy, Xp);
+    va = ldraw<VT>(p), wa = ldraw<VT>(p + dy);
     p = clamped(im, in0);
     vb = ldraw<VT>(p), wb = ldraw<VT>(p + dy);
     p = clamped(im, in0 + SN);
     vc = ldraw<VT>(p), wc = ldraw<VT>(p + dy);
     p = clamped(im, in0 + 2 * SN);
-    ldraw_if<VT>(vd, p, X);
-    ldraw_if<VT>(wd, p + dy, X);
+    vd = ldraw<VT>(p), wd = ldraw<VT>(p + dy);
+    if (!Xp) va = wa = Raw(0);
+    if (!X) vd = wd = Raw(0);
   };
   // the layer of the row at hand, which may be the ray's last
   auto edge_layer = [&]() {
@@ -981,14 +981,14 @@ __global__ void __launch_bounds__(256, 4) k_slicer_axis(const __grid_constant__ 
 //
 // Per ray and layer that leaves a 2 G-th of the weights, control and loads
 // of each plane in place of all of them for two planes. What bounds it: the
-// latency of a layer's loads at 12 to 16 warps per SM (issue 52 % busy, FMA
-// pipe 35 %); caps of 96 and 80 registers (20 and 24 warps) spill and took
+// latency of a layer's loads at 12 to 16 warps per SM (issue 65 % busy, FMA
+// pipe 41 %); caps of 96 and 80 registers (20 and 24 warps) spill and took
 // 33.5 and 44.3 ms where 128 take 33.3. 1024 x 1024 x 256, 16 tilts with 0.3
 // degrees jitter, CTF slabs: 61.1 ms with k_slicer_axis -> 39.5 (33.3 where
-// offsets may reach 1/64); 256 x 256 x
-// 128, 41 tilts: 7.3 ms with k_project_axis -> 3.2 (4 runs). A warp holds 16
-// detector rows x 2 sub-rows, so that its loads of a plane are contiguous.
-// `swap` exchanges u and v (a tilt axis across the image).
+// offsets may reach 1/64); 256 x 256 x 128, 41 tilts: 7.3 ms with
+// k_project_axis -> 3.2 (4 runs). A warp holds 16 detector rows x 2 sub-rows,
+// so that its loads of a plane are contiguous. `swap` exchanges u and v (a
+// tilt axis across the image).
 struct PlaneWalk {
   int sM, sN;          // step signs
   int nM, nN;          // voxels along the major and minor axis
