@@ -71,13 +71,14 @@ UNIT = "voxel-updates/s"
 
 # DRAM bytes per launch measured by ncu (dram__bytes_read.sum,
 # dram__bytes_write.sum) on the 1024x1024x64 volume / 1024^2 detector case,
-# per unit of the roofline: forward projection = k_slicer_axis (volume read,
-# slab images written) + k_travlen (ray lengths written), back-projection =
-# k_bp_axis (volume read and written, pre-sampled slab images read). The
-# volume part scales with the voxels, the image part with the pixels.
+# per unit of the roofline: forward projection = k_slicer_planes with lines of
+# 4 pixels, the kernel of most projections (volume read, slab images and the
+# rays' local arrays written) + k_travlen (ray lengths written);
+# back-projection = k_bp_up (volume read and written, pre-sampled slab images
+# read). The volume part scales with the voxels, the rest with the pixels.
 DRAM_V, DRAM_P = 1024 * 1024 * 64, 1024 * 1024
-DRAM_FP_READ, DRAM_FP_IMG = 268.44e6, 8.47e6 + 4.20e6
-DRAM_BP_READ, DRAM_BP_WRITE, DRAM_BP_IMG = 268.44e6, 211.57e6, 292.94e6 - 268.44e6
+DRAM_FP_READ, DRAM_FP_IMG = 268.44e6, 291.32e6 - 268.44e6 + 109.92e6 + 4.20e6
+DRAM_BP_READ, DRAM_BP_WRITE, DRAM_BP_IMG = 268.44e6, 233.48e6, 345.26e6 - 268.44e6
 
 
 def _peaks():

@@ -33,7 +33,7 @@ def main(argv=None):
     import torch
 
     from artiatomi_b200 import emsart as E
-    from artiatomi_b200.refine import _cc_shift, _particle_roi, _remove_radius, _remove_subvolume
+    from artiatomi_b200.refine import _cc_shift, _remove_radius, _remove_subvolume, particle_roi
 
     ap = argparse.ArgumentParser()
     ap.add_argument("--particles", type=int, default=16)
@@ -84,7 +84,7 @@ def main(argv=None):
         _remove_subvolume(vol, m, _remove_radius(S, cfg), saved)
         done = 0
         for i in range(n):
-            roi = _particle_roi(E.set_constant_values(pg[i], vg), m, vg, vs, safe, W, W)
+            roi = particle_roi(pg[i], m, vg, vs, safe, np.eye(3, dtype=np.float32))
             _cc_shift(R, vg, i, vol, [(sub, rot, roi)], roi, bufs, a.max_shift, a.multi_peak, (None, None))
             done += 1
         for region, keep in reversed(saved):

@@ -375,13 +375,21 @@ def test_subvolume_patch_bound(patches):
     """Patches beyond the bound: in chunks of particles (bit for bit the boxes
     of one chunk), and from the slab images where a particle's patches do not
     fit alone (the launches per particle, to rounding). 200 kB hold two or
-    three of the smaller boxes' patches of a tilt, 1 byte none."""
+    three of the smaller boxes' patches of a tilt, 1 byte none. Three particles
+    take one launch over all tilts where the patches fit, else those of a
+    tilt."""
     c = _subvolume_case(True, [16, 24, 32, 48, 16, 24], n=9, seed=5, psi_deg=0.7)
     il = np.random.default_rng(1).permutation(c["n"]).astype(np.int32)
     active = (np.linalg.norm(c["shifts"], axis=2) < 1.5).astype(np.uint8)
     free = _subvolume_gpu(c, True, il, active)
     plain = _subvolume_gpu(c, False, il, active)
-    few = _subvolume_gpu(dict(c, sizes=c["sizes"][:3], sub=c["sub"][:3]), True, il, active[:3], patch_bytes=1)
+    three = dict(c, sizes=c["sizes"][:3], sub=c["sub"][:3])
+    few = _subvolume_gpu(three, True, il, active[:3], patch_bytes=1)
+    for a, b, d in zip(free, _subvolume_gpu(three, True, il, active[:3]),
+                       _subvolume_gpu(three, True, il, active[:3], patch_bytes=200 << 10)):
+        np.testing.assert_array_equal(b, a)
+        if a.shape[0] < 32:
+            np.testing.assert_array_equal(d, a)
     chunks = _subvolume_gpu(c, True, il, active, patches, 200 << 10)
     none = _subvolume_gpu(c, True, il, active, patches, 1)
     for a, b in zip(free[:2], chunks[:2]):
