@@ -525,15 +525,14 @@ struct PhaseScope {
 static int rec_alloc(esb_reconstructor* r) {
   const size_t img = (size_t)r->cfg.proj_x * r->cfg.proj_y * sizeof(float);
   // the projection and the ray-length image are one buffer (projection
-  // first), so that a z-slab run sums both over ranks in one collective
-  ESB_CK(cudaMalloc(&r->proj_d, 2 * img), "esb_reconstructor_create");
+  // first), so that a z-slab run sums both over ranks in one collective; the
+  // flags of the pre-sampled projections follow
+  const size_t both = 2 * img + ESB_BP_SET_MAX * sizeof(unsigned);
+  ESB_CK(cudaMalloc(&r->proj_d, both), "esb_reconstructor_create");
   r->dist_d = r->proj_d + (size_t)r->cfg.proj_x * r->cfg.proj_y;
+  r->odd_d = (unsigned*)(r->dist_d + (size_t)r->cfg.proj_x * r->cfg.proj_y);
   ESB_CK(cudaMalloc(&r->real_d, img), "esb_reconstructor_create");
-  ESB_CK(cudaMemset(r->proj_d, 0, img), "esb_reconstructor_create");
-  ESB_CK(cudaMemset(r->dist_d, 0, img), "esb_reconstructor_create");
-  const size_t flags = ESB_BP_SET_MAX * sizeof(unsigned);
-  ESB_CK(cudaMalloc(&r->odd_d, flags), "esb_reconstructor_create");
-  ESB_CK(cudaMemset(r->odd_d, 0, flags), "esb_reconstructor_create");
+  ESB_CK(cudaMemset(r->proj_d, 0, both), "esb_reconstructor_create");
   if (r->cfg.ctf_mode) {
     const int N = r->N;
     ESB_CK(cudaMalloc(&r->square_d, (size_t)N * N * sizeof(float)), "esb_reconstructor_create");
@@ -546,7 +545,7 @@ static int rec_alloc(esb_reconstructor* r) {
 }
 
 static void rec_free(esb_reconstructor* r) {
-  cudaFree(r->proj_d);  // with dist_d
+  cudaFree(r->proj_d);  // with dist_d and odd_d
   cudaFree(r->real_d);
   cudaFree(r->square_d);
   cudaFree(r->fft_d);
@@ -561,7 +560,6 @@ static void rec_free(esb_reconstructor* r) {
   r->slab_imgs = nullptr;
   r->slab_cap = 0;
   cudaFree(r->up_imgs);
-  cudaFree(r->odd_d);
   cudaFree(r->tune_scratch);
   r->up_imgs = nullptr;
   r->up_cap = 0;
